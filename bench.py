@@ -280,10 +280,12 @@ class Ops:
         return bi, bo
 
     def launches_per_step(self):
-        """Kernel launches of one step: radon fwd 4 per 8-slice chunk, radon adj 3,
-        ptycho fwd 1, ptycho adj 1 plus the slab reduction when the angles are
-        split into parts (the operator's current split)."""
-        zc = -(-self.c["nz"] // 8)
+        """Kernel launches of one step: radon fwd 4 per 4 / streams chunks of 8
+        slices (2 streams by default), radon adj 3, ptycho fwd 1, ptycho adj 1
+        plus the slab reduction when the angles are split into parts (the
+        operator's current split)."""
+        batch = 4 // (self.tuned or {}).get("radon_fwd_streams", 2)
+        zc = -(-self.c["nz"] // (8 * batch))
         return 4 * zc + 3 + 1 + 1 + (self.ptycho.parts > 1)
 
 

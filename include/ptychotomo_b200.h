@@ -48,11 +48,14 @@ const char *pt_version(void);
 /* ---- USFFT Radon transform (tomography operator) ------------------------ */
 
 /* radonusfft::radonusfft(Ntheta, Nz, N)  — src/cuda/radonusfft.cu:5-39.
- * n is the object width; internal N = 3n/2, oversampled grid 2N, Gaussian
- * kernel half-width M and parameter mu as in radonusfft.cu:7-12. */
+ * n is the object width; internal N = 3n/2, oversampled grid 2N.  The
+ * reference's Gaussian half-width M and parameter mu (radonusfft.cu:7-12) are
+ * reported by pt_radon_get_params; the transform they approximate is gridded
+ * with a Kaiser-Bessel window of 8 cells, whose error is smaller. */
 int pt_radon_create(size_t ntheta, size_t nz, size_t n, pt_radon **out);
 /* Same, with the kernel half-width forced to m_override (0 = reference M).
- * A smaller M is a precision variant, not the reference operator. */
+ * A smaller M is a precision variant (its Gaussian as it stands), not the
+ * reference operator. */
 int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_override, pt_radon **out);
 /* radonusfft::~radonusfft — src/cuda/radonusfft.cu:41-52. NULL is accepted. */
 int pt_radon_destroy(pt_radon *h);
@@ -78,9 +81,9 @@ int pt_radon_adj_scaled(pt_radon *h, void *f, const void *g, float scale, void *
  * tomography CG, which needs the true gradient of its quadratic. */
 int pt_radon_adj_exact(pt_radon *h, void *f, const void *g, float scale, void *stream);
 /* Autotuner (no counterpart in the reference): times the forward with its
- * 8-slice chunks on the caller's stream alone and pipelined on two and on
- * four streams (one chunk's FFTs under another chunk's gather), each with the
- * Gaussian gather reading the grid through L1, from shared-memory tiles
+ * 8-slice chunks in one pipeline of four per launch on the caller's stream, two
+ * of two and four of one (one pipeline's FFTs under another's gather), each
+ * with the window gather reading the grid through L1, from shared-memory tiles
  * (16 x 16 window origins per tile) copied by the threads, and from the same
  * tiles loaded by the Tensor Memory Accelerator (one 3-D box per block,
  * completed on an mbarrier; offered when the tensor maps encode), `trials`

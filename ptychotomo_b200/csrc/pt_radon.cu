@@ -61,10 +61,8 @@ namespace {
 constexpr int ZC = 8;   // slices per chunk (slice-minor lanes)
 constexpr int RSETS = 4;   // forward chunk buffer sets (chunks in flight at most)
 constexpr int CK = 2;   // grid columns per block in the column kernels
+constexpr int ZH = 4;   // slices per block of the forward's column kernel
 constexpr double PI_REF = 3.1415926535;  // kernels.cuh:1
-
-template <int L>
-constexpr int fft_threads() { return L >= 1024 ? 64 : 32; }
 
 // circ, kernels.cuh:160-172 (r = 1.0f/N); evaluated without FMA contraction so
 // that it equals the float32 expression (4x*x + 4y*y) < 1 - r exactly.
@@ -83,9 +81,10 @@ __device__ __forceinline__ float deapod(int tx, int ty, int N, float mu)
     return __expf(-mu * (tx - N / 2) * (tx - N / 2) - mu * (ty - N / 2) * (ty - N / 2));
 }
 
-// fac[ty][tx] = circ / (the window's transform) on the N x N padded slice, the
-// factor that unpaddivphi / divphi and circ apply (kernels.cuh:5-37, 160-172),
-// evaluated once per handle; the row passes multiply by it.  inv1 (Kaiser-
+// fac[ty][tx] = (-1)^(tx + ty) circ / (the window's transform) on the N x N
+// padded slice: the factor that unpaddivphi / divphi and circ apply
+// (kernels.cuh:5-37, 160-172) with the centring sign of the 2N grid
+// (kernels.cuh:28-37), evaluated once per handle; the row passes multiply by it.  inv1 (Kaiser-
 // Bessel): 1 / transform per axis; null (Gaussian): circ / phi / (4 N^2) with
 // the expressions above.
 __global__ void k_deap_table(float *__restrict__ fac, int N, float mu, const double *__restrict__ inv1)
@@ -93,8 +92,9 @@ __global__ void k_deap_table(float *__restrict__ fac, int N, float mu, const dou
     const int tx = blockIdx.x * blockDim.x + threadIdx.x, ty = blockIdx.y;
     if (tx >= N) return;
     const float den = (float)(4 * N * N);
-    fac[(size_t)ty * N + tx] = inv1 ? circ_keep(tx, ty, N) * (float)(inv1[tx] * inv1[ty])
-                                    : circ_keep(tx, ty, N) / deapod(tx, ty, N, mu) / den;
+    const float f = inv1 ? circ_keep(tx, ty, N) * (float)(inv1[tx] * inv1[ty])
+                         : circ_keep(tx, ty, N) / deapod(tx, ty, N, mu) / den;
+    fac[(size_t)ty * N + tx] = ((tx + ty) & 1) ? -f : f;
 }
 
 // ---- gridding window -----------------------------------------------------------
@@ -128,8 +128,8 @@ __global__ void k_window(const float *__restrict__ xt, const float *__restrict__
 
 // The forward gather's record of a point, in visiting order (six float4):
 // floats 0..9 the x weights of the five column pairs that cover the window (0
-// for the columns outside it), 10..18 the y weights times the sign and scale
-// of the sample (fftshift1c and pre), 20 the point's index, 21 and 22 its
+// for the columns outside it), 10..18 the y weights times the sample's scale
+// pre, 20 the point's index, 21 and 22 its
 // window's first row and column pair on the haloed grid, 23 whether the window
 // needs all five pairs (an even-sized window that starts on a pair covers four).
 constexpr int REC4 = 6;
@@ -137,7 +137,7 @@ constexpr int NPAIR = 5;
 static_assert(WKB <= 9 && WGAUSS <= 9, "a window spans at most five column pairs and nine rows");
 template <int W>
 __global__ void k_point_records(const int *__restrict__ perm, const int *__restrict__ org,
-                                const float *__restrict__ wtab, float *__restrict__ rec, int npts, int N, float pre)
+                                const float *__restrict__ wtab, float *__restrict__ rec, int npts, float pre)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npts) return;
@@ -145,9 +145,8 @@ __global__ void k_point_records(const int *__restrict__ perm, const int *__restr
     const int ox = org[2 * p], oy = org[2 * p + 1], odd = ox & 1;
     const float *wx = wtab + (size_t)p * 2 * W, *wy = wx + W;
     float *r = rec + (size_t)i * REC4 * 4;
-    const float sc = ((p % N) & 1) ? pre : -pre;
     for (int j = 0; j < 2 * NPAIR; ++j) r[j] = (j >= odd && j - odd < W) ? wx[j - odd] : 0.f;
-    for (int j = 0; j < 9; ++j) r[10 + j] = j < W ? sc * wy[j] : 0.f;
+    for (int j = 0; j < 9; ++j) r[10 + j] = j < W ? pre * wy[j] : 0.f;
     r[19] = 0.f;
     r[20] = __int_as_float(p);
     r[21] = __int_as_float(oy);
@@ -169,37 +168,59 @@ __global__ void k_takexy(float *x, float *y, const float *theta, int N, int nthe
     y[tx + ty * N] = yv;
 }
 
+// The forward's four kernels work on up to RSETS chunks of ZC slices per
+// launch, one per buffer set: the chunk is the last grid dimension, `set` the
+// distance of two sets in float2.
+
 // ---- K1: pad2 + circ + divphi + fftshiftc + row FFT ------------------------
+// The block's ZC slices are interleaved transforms (lane q = slice), so the
+// output rows of the slice-minor buffer are contiguous.  The non-zero inputs
+// X = N/2 .. 3N/2 - 1 are the R1/2 middle rows i1 of the R1 x R2 split; the
+// table tw holds W^(i2 k1) i^k1: the shift of those rows by R1/4 gives
+// (-i)^k1, the centring sign of the outputs (-1)^k1.
+// The object is read and the transform written by the threads that compute it,
+// with one trip through shared memory between: 12.4 us for 8 slices at 256
+// wide (four Stockham passes and two staging copies: 21.7 us).
 template <int G>
-__global__ void __launch_bounds__(ZC *fft_threads<G>())
-    k_fwd_rows(const float2 *__restrict__ u, float2 *__restrict__ rbuf, int nz, int z0,
-               const float *__restrict__ fac, const float2 *__restrict__ tw)
+__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
+    k_fwd_rows(const float2 *__restrict__ u, float2 *__restrict__ rbuf, size_t set, int nz, int z0,
+               const float *__restrict__ fac, const float4 *__restrict__ tw)
 {
-    // the block's ZC slices are interleaved transforms: shared row X holds
-    // element X of every slice (ptfft::fft_iq), so the output is a straight
-    // copy into the slice-minor row buffer
-    constexpr int T = fft_threads<G>(), N = G / 2, n = G / 3;
+    using E = ptfft::Exchange<G, ZC>;
+    constexpr int N = G / 2, n = G / 3, R1 = E::R1, R2 = E::R2;
     constexpr int c0 = N / 6, c1 = 5 * N / 6 - 1;
     extern __shared__ float2 sm[];
     const int y = blockIdx.x;
     const int q = threadIdx.x % ZC, b = threadIdx.x / ZC;
-    const int z = z0 + q;
-    const int sr = min(max(y, c0), c1) - c0;
-    const int Y = y + N / 2;
-    for (int X = b; X < G; X += T) {
-        float2 v = czero();
-        const int tx = X - N / 2;
-        if (tx >= 0 && tx < N && z < nz) {
-            const int sc = min(max(tx, c0), c1) - c0;
-            v = __ldg(&fac[(size_t)y * N + tx]) * u[((size_t)z * n + sr) * n + sc];
-            if ((X + Y) & 1) v = -1.f * v;
+    if (b < R2) {
+        const int z = z0 + blockIdx.y * ZC + q;
+        float2 in[R1 / 2];
+        if (z < nz) {
+            const float2 *src = u + ((size_t)z * n + (min(max(y, c0), c1) - c0)) * n;
+            const float *f = fac + (size_t)y * N;
+#pragma unroll
+            for (int a = 0; a < R1 / 2; ++a) {
+                const int tx = a * R2 + b;
+                in[a] = __ldg(&f[tx]) * src[min(max(tx, c0), c1) - c0];
+            }
+        } else {
+#pragma unroll
+            for (int a = 0; a < R1 / 2; ++a) in[a] = czero();
         }
-        sm[X * ZC + q] = v;
+        float2 v[R1];
+        ptfft::dft_half<R1, -1>(in, v);
+        ptfft::twiddle_pairs<R1, R2>(v, b, tw);
+        E::put(sm, v, b, q);
     }
     __syncthreads();
-    ptfft::fft_iq<G, -1, T, ZC>(sm, q, b, tw);
-    float2 *dst = rbuf + (size_t)y * G * ZC;
-    for (int e = threadIdx.x; e < G * ZC; e += blockDim.x) dst[e] = sm[e];
+    if (b < R1) {
+        float2 w[R2];
+        E::get(sm, w, b, q);
+        ptfft::Dft<R2, -1, true>::run(w);
+        float2 *dst = rbuf + blockIdx.y * set + ((size_t)y * G + b) * ZC + q;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) dst[k2 * R1 * ZC] = w[k2];
+    }
 }
 
 // The forward's Fourier grid carries a halo, like the reference's (G+2M)^2
@@ -210,45 +231,53 @@ __global__ void __launch_bounds__(ZC *fft_threads<G>())
 constexpr int GH_ROWS = 8;    // the largest window (9 cells) minus one
 constexpr int GH_PAIRS = NPAIR - 1;
 
-// ---- K2: column FFT of the 2N grid, centring sign folded in ----------------
-// The block's CK columns x ZC slices are NF interleaved transforms: shared
-// row i holds element i of all NF (column c, slice z at c * ZC + z), so the
-// input rows (one 128-byte line of the row-FFT buffer per y) and the output
-// rows (one 128-byte line of the grid per ky) are straight copies, and the
-// passes (ptfft::fft_iq) are free of bank conflicts.
+// ---- K2: column FFT of the 2N grid ---------------------------------------------
+// The block's CK columns x ZH slices are NF interleaved transforms, ordered as
+// the grid's column pairs hold them (q = slice * CK + column), so both the
+// row-FFT buffer and the grid are touched in whole 32- or 64-byte runs.  Rows
+// outside N/2 .. 3N/2 - 1 are zero; the table is K1's.
+// 17.5 us for 8 slices at 256 wide (Stockham passes: 30.6 us).
 template <int G>
-__global__ void __launch_bounds__(CK *ZC *fft_threads<G>())
-    k_fwd_cols(const float2 *__restrict__ rbuf, float2 *__restrict__ fg, const float2 *__restrict__ tw)
+__global__ void __launch_bounds__(ptfft::Exchange<G, CK * ZH>::NT, G > 768 ? 1 : 2)
+    k_fwd_cols(const float2 *__restrict__ rbuf, float2 *__restrict__ fg, size_t set, const float4 *__restrict__ tw)
 {
-    constexpr int T = fft_threads<G>(), N = G / 2, NF = CK * ZC;
+    constexpr int NF = CK * ZH;
+    using E = ptfft::Exchange<G, NF>;
+    constexpr int R1 = E::R1, R2 = E::R2;
+    static_assert(CK == 2, "the grid layout pairs two columns");
     extern __shared__ float2 sm[];
-    const int kx0 = blockIdx.x * CK;
+    const int pr = blockIdx.x, zh = blockIdx.y * ZH;
     const int q = threadIdx.x % NF, b = threadIdx.x / NF;
-    for (int e = threadIdx.x; e < N * NF; e += blockDim.x) {
-        const int y = e / NF, r = e % NF;
-        sm[(N / 2 + y) * NF + r] = rbuf[((size_t)y * G + kx0) * ZC + r];
-    }
-    for (int e = threadIdx.x; e < N * NF; e += blockDim.x) {
-        const int i = e / NF, r = e % NF;
-        sm[(i < N / 2 ? i : i + N) * NF + r] = czero();
+    if (b < R2) {
+        const float2 *src = rbuf + blockIdx.z * set + ((size_t)b * G + pr * CK + q % CK) * ZC + zh + q / CK;
+        float2 in[R1 / 2];
+#pragma unroll
+        for (int a = 0; a < R1 / 2; ++a) in[a] = src[(size_t)a * R2 * G * ZC];
+        float2 v[R1];
+        ptfft::dft_half<R1, -1>(in, v);
+        ptfft::twiddle_pairs<R1, R2>(v, b, tw);
+        E::put(sm, v, b, q);
     }
     __syncthreads();
-    ptfft::fft_iq<G, -1, T, NF>(sm, q, b, tw);
-    // column-pair layout [ky][kx/2][z][kx&1]: one 128-byte line per (ky, pair),
-    // plus the halo copies (rows < GH_ROWS again at G + ky, pairs < GH_PAIRS
-    // again at G/2 + pair)
-    static_assert(CK == 2, "the grid layout pairs two columns");
-    constexpr int PS = G / 2 + GH_PAIRS;
-    const int pr = kx0 / 2;
-    for (int e = threadIdx.x; e < (G + GH_ROWS) * NF; e += blockDim.x) {
-        const int kyh = e / NF, r = e % NF;
-        const int ky = kyh < G ? kyh : kyh - G;
-        const int z = r >> 1, c = r & 1;
-        const int kx = kx0 + c;
-        float2 v = sm[ky * NF + c * ZC + z];
-        if ((kx + ky) & 1) v = -1.f * v;
-        fg[((size_t)kyh * PS + pr) * (2 * ZC) + r] = v;
-        if (pr < GH_PAIRS) fg[((size_t)kyh * PS + G / 2 + pr) * (2 * ZC) + r] = v;
+    if (b < R1) {
+        float2 w[R2];
+        E::get(sm, w, b, q);
+        ptfft::Dft<R2, -1, true>::run(w);
+        // column-pair layout [ky][kx/2][z][kx&1], plus the halo copies (rows <
+        // GH_ROWS again at G + ky, pairs < GH_PAIRS again at G/2 + pair)
+        constexpr size_t PS = G / 2 + GH_PAIRS;
+        float2 *dst = fg + blockIdx.z * set + (size_t)pr * (CK * ZC) + zh * CK + q;
+        const bool edge = pr < GH_PAIRS;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) {
+            const int ky = b + R1 * k2;
+            dst[ky * PS * (CK * ZC)] = w[k2];
+            if (edge) dst[(ky * PS + G / 2) * (CK * ZC)] = w[k2];
+            if (R1 * k2 < GH_ROWS && ky < GH_ROWS) {
+                dst[(ky + G) * PS * (CK * ZC)] = w[k2];
+                if (edge) dst[((ky + G) * PS + G / 2) * (CK * ZC)] = w[k2];
+            }
+        }
     }
 }
 
@@ -257,7 +286,7 @@ __global__ void __launch_bounds__(CK *ZC *fft_threads<G>())
 // a lane reads its slice's value at two neighbouring window columns with one
 // 16-byte load (the point's 8 lanes read one 128-byte line).  The window's
 // columns are covered by four or five column pairs; a covered column outside
-// the window has weight 0.  Writes the gathered, 1/N- and fftshift1c-scaled
+// the window has weight 0.  Writes the gathered, 1/N-scaled
 // samples to lines[(theta N + k) ZC + z].  Points are visited in the order of
 // `perm` (built at setobj): sorted by the 16 x 16-cell grid tile their window
 // starts in, then by the parity of its first column, so the points of a block
@@ -309,7 +338,8 @@ __device__ __forceinline__ float2 window_sum(const float4 *__restrict__ base, si
 
 template <int N, int W>
 __global__ void __launch_bounds__(GPB *ZC, 4)
-    k_fwd_gather_pts(const float2 *__restrict__ fg, float2 *__restrict__ lines, const float4 *__restrict__ rec, int npts)
+    k_fwd_gather_pts(const float2 *__restrict__ fg, size_t set, float2 *__restrict__ lines, const float4 *__restrict__ rec,
+                     int npts)
 {
     constexpr int G = 2 * N, PS = G / 2 + GH_PAIRS;
     static_assert(W - 1 <= GH_ROWS, "the grid halo must cover the window");
@@ -319,8 +349,8 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
     const float4 *r = rec + (size_t)pi * REC4;
     const float4 q = __ldg(&r[5]);
     const float4 *base =
-        reinterpret_cast<const float4 *>(fg) + ((size_t)__float_as_int(q.y) * PS + __float_as_int(q.z)) * ZC + lane;
-    lines[(size_t)__float_as_int(q.x) * ZC + lane] =
+        reinterpret_cast<const float4 *>(fg + blockIdx.y * set) + ((size_t)__float_as_int(q.y) * PS + __float_as_int(q.z)) * ZC + lane;
+    lines[((size_t)blockIdx.y * npts + __float_as_int(q.x)) * ZC + lane] =
         window_sum<W>(base, (size_t)PS * ZC, r, [](const float4 *p) { return __ldg(p); });
 }
 
@@ -359,8 +389,8 @@ __device__ __forceinline__ void tile_gather(const float4 *__restrict__ tsm, cons
 
 template <int N, int W>
 __global__ void __launch_bounds__(GPB *ZC, 4)
-    k_fwd_gather_tile(const float2 *__restrict__ fg, float2 *__restrict__ lines, const float4 *__restrict__ rec,
-                      const int4 *__restrict__ chunks)
+    k_fwd_gather_tile(const float2 *__restrict__ fg, size_t set, float2 *__restrict__ lines,
+                      const float4 *__restrict__ rec, const int4 *__restrict__ chunks, int npts)
 {
     constexpr int G = 2 * N;
     constexpr int PS = G / 2 + GH_PAIRS, NROWS = G + GH_ROWS;   // the haloed grid's pair pitch and rows
@@ -369,14 +399,14 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
     const int4 ch = chunks[blockIdx.x];   // (tile row, tile column, first, count)
     const int ty0 = ch.x * GTILE, px0 = ch.y * GTILE / 2;
     const int rows = min(tile_rows<W>(), NROWS - ty0), pairs = min(TILE_PAIRS, PS - px0);
-    const float4 *g4 = reinterpret_cast<const float4 *>(fg);
+    const float4 *g4 = reinterpret_cast<const float4 *>(fg + blockIdx.y * set);
     for (int e = threadIdx.x; e < rows * pairs * ZC; e += blockDim.x) {
         const int r = e / (pairs * ZC), rem = e % (pairs * ZC), pj = rem / ZC, q = rem % ZC;
         tsm[(r * TILE_PAIRS + pj) * ZC + q] = __ldg(&g4[((size_t)(ty0 + r) * PS + px0 + pj) * ZC + q]);
     }
     for (int e = threadIdx.x; e < ch.w * REC4; e += blockDim.x) rsm[e] = __ldg(&rec[(size_t)ch.z * REC4 + e]);
     __syncthreads();
-    tile_gather<W>(tsm, rsm, ch.w, ty0, px0, lines);
+    tile_gather<W>(tsm, rsm, ch.w, ty0, px0, lines + (size_t)blockIdx.y * npts * ZC);
 }
 
 // The same with the tile and the records staged by the Tensor Memory
@@ -394,10 +424,13 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
 constexpr int TMA_SPIN = 1 << 24;
 template <int W>
 constexpr size_t tma_smem() { return tile_smem<W>() + 16; }
+struct GridMaps {
+    CUtensorMap m[RSETS];   // one per buffer set
+};
 template <int N, int W>
 __global__ void __launch_bounds__(GPB *ZC, 4)
-    k_fwd_gather_tma(const __grid_constant__ CUtensorMap tmap, float2 *__restrict__ lines,
-                     const float4 *__restrict__ rec, const int4 *__restrict__ chunks, int *__restrict__ err,
+    k_fwd_gather_tma(const __grid_constant__ GridMaps maps, int set0, float2 *__restrict__ lines,
+                     const float4 *__restrict__ rec, const int4 *__restrict__ chunks, int npts, int *__restrict__ err,
                      int spin = TMA_SPIN, int check = 0)
 {
     // check != 0 (the status test only): the blocks first wait on a second
@@ -428,7 +461,7 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
         asm volatile(
             "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
             "%4}], [%5];" ::"r"(dst),
-            "l"(reinterpret_cast<unsigned long long>(&tmap)), "r"(0), "r"(px0), "r"(ty0), "r"(bar_a)
+            "l"(reinterpret_cast<unsigned long long>(&maps.m[set0 + blockIdx.y])), "r"(0), "r"(px0), "r"(ty0), "r"(bar_a)
             : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + TB),
                      "l"(rec + (size_t)ch.z * REC4), "r"(rbytes), "r"(bar_a)
@@ -449,28 +482,43 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
         wait(bar_a, TMA_SPIN);   // the copies land in this block's memory: let them finish first
         return;
     }
-    tile_gather<W>(tsm, rsm, ch.w, ty0, px0, lines);
+    tile_gather<W>(tsm, rsm, ch.w, ty0, px0, lines + (size_t)blockIdx.y * npts * ZC);
 }
 
 // ---- K3b: fftshift1c / 1-D inverse FFT / fftshift1c + crop + scale --------
+// tw: W^(i2 k1) (-1)^(i2 + k1), inverse: the two sign changes of the centred
+// transform.  Only the cropped outputs are formed.
 template <int N>
-__global__ void __launch_bounds__(ZC * 32)
+__global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
     k_fwd_lines(const float2 *__restrict__ lines, float2 *__restrict__ out, int nz, int z0, float scale,
-                const float2 *__restrict__ tw)
+                const float4 *__restrict__ tw)
 {
-    constexpr int n = 2 * N / 3, c0 = N / 6, T = 32;
+    using E = ptfft::Exchange<N, ZC>;
+    constexpr int n = 2 * N / 3, c0 = N / 6, R1 = E::R1, R2 = E::R2;
     extern __shared__ float2 sm[];
     const int th = blockIdx.x;
-    const float2 *src = lines + (size_t)th * N * ZC;   // [k][slice]: the interleaved layout already
-    for (int e = threadIdx.x; e < N * ZC; e += blockDim.x) sm[e] = src[e];
+    const int q = threadIdx.x % ZC, b = threadIdx.x / ZC;
+    if (b < R2) {
+        const float2 *src = lines + (((size_t)blockIdx.y * gridDim.x + th) * N + b) * ZC + q;
+        float2 v[R1];
+#pragma unroll
+        for (int i1 = 0; i1 < R1; ++i1) v[i1] = src[i1 * R2 * ZC];
+        ptfft::Dft<R1, +1, true>::run(v);
+        ptfft::twiddle_pairs<R1, R2>(v, b, tw);
+        E::put(sm, v, b, q);
+    }
     __syncthreads();
-    ptfft::fft_iq<N, +1, T, ZC>(sm, threadIdx.x % ZC, threadIdx.x / ZC, tw);
-    for (int e = threadIdx.x; e < ZC * n; e += blockDim.x) {
-        const int q = e % ZC, j = e / ZC;
-        const int z = z0 + q;
-        if (z < nz) {
-            const int k = c0 + j;
-            out[((size_t)th * nz + z) * n + j] = ((k & 1) ? scale : -scale) * sm[k * ZC + q];
+    const int z = z0 + blockIdx.y * ZC + q;
+    if (b < R1 && z < nz) {
+        float2 w[R2];
+        E::get(sm, w, b, q);
+        ptfft::Dft<R2, +1, true>::run(w);
+        float2 *dst = out + ((size_t)th * nz + z) * n;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) {
+            if (R1 * k2 + R1 <= c0 || R1 * k2 >= c0 + n) continue;   // wholly cropped
+            const int j = b + R1 * k2 - c0;
+            if (j >= 0 && j < n) dst[j] = scale * w[k2];
         }
     }
 }
@@ -478,35 +526,44 @@ __global__ void __launch_bounds__(ZC * 32)
 // ---- A1: pad (kernels.cuh:189-206) + fftshift1c/FFT/fftshift1c -------------
 // grid (ntheta, nzp / ZC); writes lines[(theta*N + k) * nzp + z].  ZP: the
 // exact adjoint's zero padding (the adjoint of the forward's crop) instead
-// of the reference's edge replication.
+// of the reference's edge replication.  tw: W^(i2 k1) (-1)^(i2 + k1), forward.
 template <int N, bool ZP = false>
-__global__ void __launch_bounds__(ZC * 32)
+__global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
     k_adj_lines(const float2 *__restrict__ g, float2 *__restrict__ lines, int nz, int nzp, float pre,
-                const float2 *__restrict__ tw)
+                const float4 *__restrict__ tw)
 {
-    constexpr int n = 2 * N / 3, c0 = N / 6, c1 = 5 * N / 6 - 1, T = 32;
+    using E = ptfft::Exchange<N, ZC>;
+    constexpr int n = 2 * N / 3, c0 = N / 6, c1 = 5 * N / 6 - 1, R1 = E::R1, R2 = E::R2;
     extern __shared__ float2 sm[];
     const int th = blockIdx.x, z0 = blockIdx.y * ZC;
     const int q = threadIdx.x % ZC, b = threadIdx.x / ZC;
     const int z = z0 + q;
-    for (int k = b; k < N; k += T) {
-        float2 v = czero();
-        if (z < nz) {
-            if (!ZP) v = g[((size_t)th * nz + z) * n + (min(max(k, c0), c1) - c0)];
-            else if (k >= c0 && k <= c1) v = g[((size_t)th * nz + z) * n + (k - c0)];
+    if (b < R2) {
+        float2 v[R1];
+        const float2 *src = g + ((size_t)th * nz + z) * n;
+#pragma unroll
+        for (int i1 = 0; i1 < R1; ++i1) {
+            const int k = i1 * R2 + b;
+            v[i1] = czero();
+            if (z < nz && (!ZP || (k >= c0 && k <= c1))) v[i1] = src[min(max(k, c0), c1) - c0];
         }
-        sm[k * ZC + q] = (k & 1) ? v : -1.f * v;
+        ptfft::Dft<R1, -1, true>::run(v);
+        ptfft::twiddle_pairs<R1, R2>(v, b, tw);
+        E::put(sm, v, b, q);
     }
     __syncthreads();
-    ptfft::fft_iq<N, -1, T, ZC>(sm, q, b, tw);
-    for (int e = threadIdx.x; e < N * ZC; e += blockDim.x) {
-        const int k = e / ZC, qq = e % ZC;
-        lines[((size_t)th * N + k) * nzp + z0 + qq] = ((k & 1) ? pre : -pre) * sm[e];
+    if (b < R1) {
+        float2 w[R2];
+        E::get(sm, w, b, q);
+        ptfft::Dft<R2, -1, true>::run(w);
+        float2 *dst = lines + ((size_t)th * N + b) * nzp + z;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) dst[(size_t)k2 * R1 * nzp] = pre * w[k2];
     }
 }
 
 // ---- A2: column gather (transpose of the forward gather) + column IFFT ----
-// grid (nzp / 16, G); block = 16 FFTs x T threads.  A warp owns 4 consecutive
+// grid (nzp / 16, G); block of CT threads.  A warp owns 4 consecutive
 // cells (a "cell group") of the column at a time; the group's list holds every
 // polar point whose kernel window covers any of the 4 cells, with the 4
 // weights (0 where the window misses a cell), in increasing point order.
@@ -514,17 +571,23 @@ __global__ void __launch_bounds__(ZC * 32)
 // order -> deterministic.  Each loaded g value feeds 4 accumulators.  A point
 // of the 8-cell window has 22 entries (8 columns x 2.75 groups), of the 15-cell
 // Gaussian 67: at 256^3 and 384 angles 1.58 against 2.79 ms.
+// The list loop takes 0.98 of the kernel's 1.34 ms, the transforms 0.27.
+// Tried and slower: a list per stream (more weight lines per load), one masked
+// trip per list end with the indices loaded ahead, columns as the fast grid
+// dimension.
 // ALL: write all N rows of the padded slice (rows N/2 .. N/2 + N - 1 of the
 // grid, for the exact adjoint's fold) instead of the n rows of the crop.
 constexpr int ZQ = 16;
 constexpr int CG = 4;  // cells per group
+template <int G>
+constexpr int col_threads() { return G >= 1024 ? 1024 : G >= 384 ? 512 : 256; }
 template <int G, bool ALL = false>
-__global__ void __launch_bounds__(ZQ *fft_threads<G>(), (G >= 1024 ? 1 : 2))
+__global__ void __launch_bounds__(col_threads<G>(), (G >= 1024 ? 1 : G >= 384 ? 2 : 4))
     k_adj_colgather(const float2 *__restrict__ lines, float2 *__restrict__ rbuf, const int *__restrict__ goff,
                     const int *__restrict__ gpt, const float4 *__restrict__ gw, const int *__restrict__ col_order,
-                    int nzp, const float2 *__restrict__ tw)
+                    int nzp, const float2 *__restrict__ tw1, const float2 *__restrict__ tw2)
 {
-    constexpr int T = fft_threads<G>(), N = G / 2, n = G / 3, NG4 = G / CG;
+    constexpr int N = G / 2, n = G / 3, NG4 = G / CG;
     constexpr int Y0 = N / 2 + N / 6;
     constexpr int U = 4;  // entries in flight per lane
     extern __shared__ float2 sm[];
@@ -578,35 +641,45 @@ __global__ void __launch_bounds__(ZQ *fft_threads<G>(), (G >= 1024 ? 1 : 2))
                 acc[c].w = fmaf(wc[c], v.w, acc[c].w);
             }
         }
-        // streams 0+2 and 1+3, then 0+1: a fixed order
+        // streams 0+2 and 1+3, then those two sums: each exchange hands over the
+        // half that the partner keeps, so stream s ends with cell s (12 shuffles
+        // instead of 32, and a store by all lanes)
+        {
+            const bool up2 = s & 2, up1 = s & 1;
+            float4 k[2], g;
 #pragma unroll
-        for (int o = 16; o >= 8; o >>= 1) {
-#pragma unroll
-            for (int c = 0; c < CG; ++c) {
-                acc[c].x += __shfl_down_sync(0xffffffffu, acc[c].x, o);
-                acc[c].y += __shfl_down_sync(0xffffffffu, acc[c].y, o);
-                acc[c].z += __shfl_down_sync(0xffffffffu, acc[c].z, o);
-                acc[c].w += __shfl_down_sync(0xffffffffu, acc[c].w, o);
+            for (int j = 0; j < 2; ++j) {
+                k[j] = up2 ? acc[2 + j] : acc[j];
+                g = up2 ? acc[j] : acc[2 + j];
+                k[j].x += __shfl_xor_sync(0xffffffffu, g.x, 16);
+                k[j].y += __shfl_xor_sync(0xffffffffu, g.y, 16);
+                k[j].z += __shfl_xor_sync(0xffffffffu, g.z, 16);
+                k[j].w += __shfl_xor_sync(0xffffffffu, g.w, 16);
             }
-        }
-        if (s == 0) {
-#pragma unroll
-            for (int c = 0; c < CG; ++c) {
-                const int ky = gi * CG + c;
-                const float sg = ((kx + ky) & 1) ? -1.f : 1.f;  // fftshiftc
-                sm[ky * ZQ + 2 * zl] = make_float2(sg * acc[c].x, sg * acc[c].y);
-                sm[ky * ZQ + 2 * zl + 1] = make_float2(sg * acc[c].z, sg * acc[c].w);
-            }
+            float4 r = up1 ? k[1] : k[0];
+            g = up1 ? k[0] : k[1];
+            r.x += __shfl_xor_sync(0xffffffffu, g.x, 8);
+            r.y += __shfl_xor_sync(0xffffffffu, g.y, 8);
+            r.z += __shfl_xor_sync(0xffffffffu, g.z, 8);
+            r.w += __shfl_xor_sync(0xffffffffu, g.w, 8);
+            reinterpret_cast<float4 *>(sm)[(gi * CG + s) * (ZQ / 2) + zl] = r;
         }
     }
     __syncthreads();
-    // the 16 slices' column transforms interleaved (shared row ky = element ky of each)
-    ptfft::fft_iq<G, +1, T, ZQ>(sm, threadIdx.x % ZQ, threadIdx.x / ZQ, tw);
+    // the 16 slices' column transforms in place (shared row ky = element ky of
+    // each; the grid's centring sign (-1)^ky is in tw2, (-1)^kx in the row
+    // pass's table); the cropped rows go from the last round's registers to memory
     constexpr int ROWS = ALL ? N : n, YB = ALL ? N / 2 : Y0;
-    for (int e = threadIdx.x; e < ROWS * ZQ; e += blockDim.x) {
-        const int r = e / ZQ, q = e % ZQ;
-        rbuf[((size_t)r * G + kx) * nzp + z0 + q] = sm[(YB + r) * ZQ + q];
-    }
+    constexpr int C = ptfft::split3_c(G), AB = G / C;
+    float2 *dst = rbuf + (size_t)kx * nzp + z0;
+    ptfft::fft3<G, +1, col_threads<G>(), ZQ>(sm, tw1, tw2, [&](int kk, int q, const float2 (&w)[C]) {
+#pragma unroll
+        for (int k3 = 0; k3 < C; ++k3) {
+            if (AB * k3 + AB <= YB || AB * k3 >= YB + ROWS) continue;   // wholly cropped
+            const int r = kk + AB * k3 - YB;
+            if (r >= 0 && r < ROWS) dst[(size_t)r * G * nzp + q] = w[k3];
+        }
+    });
 }
 
 // setobj: the 4 weights of every (cell group, point) entry, wx * wy of the
@@ -633,31 +706,51 @@ __global__ void k_make_entries(const unsigned *__restrict__ keys, int *__restric
     gw[e] = make_float4(w[0], w[1], w[2], w[3]);
 }
 
-// ---- A4: row inverse FFT + fftshiftc + unpaddivphi + circ + crop -----------
-// grid (n, nzp / ZC); reads rbuf[(r * G + kx) * nzp + z]
+// Round 1 of the adjoint's row transforms: src is the row's first column for
+// this thread's slice, columns nzp apart.
 template <int G>
-__global__ void __launch_bounds__(ZC *fft_threads<G>())
-    k_adj_rows(const float2 *__restrict__ rbuf, float2 *__restrict__ out, int nz, int nzp,
-               const float *__restrict__ fac, float scale, const float2 *__restrict__ tw)
+__device__ __forceinline__ void adj_row_round1(const float2 *__restrict__ src, int nzp, float2 *sm, int b, int q,
+                                               const float4 *__restrict__ tw)
 {
-    constexpr int T = fft_threads<G>(), N = G / 2, n = G / 3, c0 = N / 6;
+    using E = ptfft::Exchange<G, ZC>;
+    constexpr int R1 = E::R1, R2 = E::R2;
+    if (b < R2) {
+        float2 v[R1];
+#pragma unroll
+        for (int i1 = 0; i1 < R1; ++i1) v[i1] = src[(size_t)(i1 * R2 + b) * nzp];
+        ptfft::Dft<R1, +1, true>::run(v);
+        ptfft::twiddle_pairs<R1, R2>(v, b, tw);
+        E::put(sm, v, b, q);
+    }
+}
+
+// ---- A4: row inverse FFT + fftshiftc + unpaddivphi + circ + crop -----------
+// grid (n, nzp / ZC); reads rbuf[(r * G + kx) * nzp + z].  tw: W^(i2 k1)
+// (-1)^i2, inverse (the sign of the grid column; that of the output is in fac).
+template <int G>
+__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
+    k_adj_rows(const float2 *__restrict__ rbuf, float2 *__restrict__ out, int nz, int nzp,
+               const float *__restrict__ fac, float scale, const float4 *__restrict__ tw)
+{
+    using E = ptfft::Exchange<G, ZC>;
+    constexpr int N = G / 2, n = G / 3, c0 = N / 6, R1 = E::R1, R2 = E::R2;
     extern __shared__ float2 sm[];
     const int r = blockIdx.x, z0 = blockIdx.y * ZC;
-    for (int e = threadIdx.x; e < G * ZC; e += blockDim.x) {
-        const int kx = e / ZC, q = e % ZC;
-        sm[e] = rbuf[((size_t)r * G + kx) * nzp + z0 + q];
-    }
+    const int q = threadIdx.x % ZC, b = threadIdx.x / ZC;
+    adj_row_round1<G>(rbuf + (size_t)r * G * nzp + z0 + q, nzp, sm, b, q, tw);
     __syncthreads();
-    ptfft::fft_iq<G, +1, T, ZC>(sm, threadIdx.x % ZC, threadIdx.x / ZC, tw);
-    for (int e = threadIdx.x; e < ZC * n; e += blockDim.x) {
-        const int q = e % ZC, c = e / ZC;
-        const int z = z0 + q;
-        if (z < nz) {
-            const int tx = c0 + c, ty = c0 + r;
-            const int X = N / 2 + tx, Y = N / 2 + ty;
-            float2 v = sm[X * ZC + q];
-            if ((X + Y) & 1) v = -1.f * v;
-            out[((size_t)z * n + r) * n + c] = scale * (__ldg(&fac[(size_t)ty * N + tx]) * v);
+    const int z = z0 + q;
+    if (b < R1 && z < nz) {
+        float2 w[R2];
+        E::get(sm, w, b, q);
+        ptfft::Dft<R2, +1, true>::run(w);
+        const float *f = fac + (size_t)(c0 + r) * N + c0;
+        float2 *dst = out + ((size_t)z * n + r) * n;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) {
+            if (R1 * k2 + R1 <= N / 2 + c0 || R1 * k2 >= N / 2 + c0 + n) continue;   // wholly cropped
+            const int c = b + R1 * k2 - (N / 2 + c0);
+            if (c >= 0 && c < n) dst[c] = scale * (__ldg(&f[c]) * w[k2]);
         }
     }
 }
@@ -673,20 +766,28 @@ __global__ void __launch_bounds__(ZC *fft_threads<G>())
 // the crop goes to out, a margin row (ty <= c0 or ty >= c0 + n - 1) to its
 // slot of mbuf [n/2 + 2][nz][n] for the fold along y.
 template <int G>
-__global__ void __launch_bounds__(ZC *fft_threads<G>())
+__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
     k_adj_rows_exact(const float2 *__restrict__ rbuf, float2 *__restrict__ out, float2 *__restrict__ mbuf, int nz,
-                     int nzp, const float *__restrict__ fac, float scale, const float2 *__restrict__ tw)
+                     int nzp, const float *__restrict__ fac, float scale, const float4 *__restrict__ tw)
 {
-    constexpr int T = fft_threads<G>(), N = G / 2, n = G / 3, c0 = N / 6;
+    using E = ptfft::Exchange<G, ZC>;
+    constexpr int N = G / 2, n = G / 3, c0 = N / 6, R1 = E::R1, R2 = E::R2;
     extern __shared__ float2 sm[];
     const int ty = blockIdx.x, z0 = blockIdx.y * ZC;
-    for (int e = threadIdx.x; e < G * ZC; e += blockDim.x) {
-        const int kx = e / ZC, q = e % ZC;
-        sm[e] = rbuf[((size_t)ty * G + kx) * nzp + z0 + q];
+    {
+        const int q = threadIdx.x % ZC, b = threadIdx.x / ZC;
+        adj_row_round1<G>(rbuf + (size_t)ty * G * nzp + z0 + q, nzp, sm, b, q, tw);
+        __syncthreads();
+        float2 w[R2];
+        if (b < R1) E::get(sm, w, b, q);
+        __syncthreads();   // the exchange is read: the row goes back in natural order
+        if (b < R1) {
+            ptfft::Dft<R2, +1, true>::run(w);
+#pragma unroll
+            for (int k2 = 0; k2 < R2; ++k2) sm[(b + R1 * k2) * ZC + q] = w[k2];
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    ptfft::fft_iq<G, +1, T, ZC>(sm, threadIdx.x % ZC, threadIdx.x / ZC, tw);
-    const int Y = N / 2 + ty;
     const float *facr = fac + (size_t)ty * N;
     for (int e = threadIdx.x; e < ZC * n; e += blockDim.x) {
         const int q = e % ZC, c = e / ZC;
@@ -696,10 +797,7 @@ __global__ void __launch_bounds__(ZC *fft_threads<G>())
         const int lo = c == 0 ? 0 : c0 + c, hi = c == n - 1 ? N - 1 : c0 + c;
         float2 acc = czero();
         for (int tx = lo; tx <= hi; ++tx) {
-            const int X = N / 2 + tx;
-            float2 v = sm[X * ZC + q];
-            if ((X + Y) & 1) v = -1.f * v;
-            acc = acc + __ldg(&facr[tx]) * v;
+            acc = acc + __ldg(&facr[tx]) * sm[(N / 2 + tx) * ZC + q];
         }
         acc = scale * acc;
         if (ty > c0 && ty < c0 + n - 1) {
@@ -711,18 +809,20 @@ __global__ void __launch_bounds__(ZC *fft_threads<G>())
     }
 }
 
-// out row 0 = sum of margin slots 0..c0, row n-1 = the remaining slots (fixed order)
+// out row 0 = sum of margin slots 0..c0, row n-1 = the remaining slots (fixed
+// order; grid y: the row).  Unrolled: eight slots' loads are in flight.
 __global__ void k_adj_fold_rows(const float2 *__restrict__ mbuf, float2 *__restrict__ out, int nz, int n, int c0,
                                 int nslots)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)nz * n) return;
     const int z = (int)(i / n), c = (int)(i % n);
-    float2 a = czero(), b = czero();
-    for (int s = 0; s <= c0; ++s) a = a + mbuf[((size_t)s * nz + z) * n + c];
-    for (int s = c0 + 1; s < nslots; ++s) b = b + mbuf[((size_t)s * nz + z) * n + c];
-    out[((size_t)z * n) * n + c] = a;
-    out[((size_t)z * n + (n - 1)) * n + c] = b;
+    const bool last = blockIdx.y != 0;
+    const int s0 = last ? c0 + 1 : 0, s1 = last ? nslots : c0 + 1;
+    float2 a = czero();
+#pragma unroll 8
+    for (int s = s0; s < s1; ++s) a = a + mbuf[((size_t)s * nz + z) * n + c];
+    out[((size_t)z * n + (last ? n - 1 : 0)) * n + c] = a;
 }
 
 }  // namespace
@@ -735,10 +835,14 @@ struct pt_radon {
     float mu = 0.f;
     int device = -1;
     bool ready = false;
-    // two allocations cut into pieces: the geometry tables (tw_G .. tma_err,
-    // deap, inv1, goff, col_order) and the forward's buffer sets (rbuf, fgrid)
+    // two allocations cut into pieces: the tables (tw_fwd ..
+    // tma_err, deap, inv1, goff, col_order) and the forward's buffer sets (rbuf, fgrid)
     char *tables = nullptr, *sets = nullptr;
-    float2 *tw_G = nullptr, *tw_N = nullptr;
+    // twiddles with the centring signs: the forward's rows and columns, the
+    // adjoint's rows, the detector lines (twiddle_pairs layout), and the three
+    // rounds of the adjoint's columns
+    float4 *tw_fwd = nullptr, *tw_adj = nullptr, *tw_fwd_line = nullptr, *tw_inv_line = nullptr;
+    float2 *tw_col1 = nullptr, *tw_col2 = nullptr;
     float *theta = nullptr, *x = nullptr, *y = nullptr;
     int W = 0;                // cells of the gridding window per axis (WKB or WGAUSS)
     int *org = nullptr;       // first grid column and row of each point's window
@@ -750,14 +854,14 @@ struct pt_radon {
     int gather = 2;           // 0: gather through L1 (k_fwd_gather_pts), 1: shared-memory tiles, 2: TMA-staged tiles
     // gather 2: one 3-D tensor map per grid buffer set, and a device flag the
     // TMA kernel sets if a tile load did not complete
-    CUtensorMap tmap[RSETS];
+    GridMaps tmap;
     bool tma_ok = false;
     int *tma_err = nullptr;
-    // forward: per chunk of ZC slices, a row-FFT buffer and a Fourier grid.
-    // RSETS buffer sets and RSETS - 1 side streams: chunk c runs on set and
-    // stream c % streams (set 0 on the caller's stream), so up to `streams`
-    // chunks are in flight and one chunk's FFTs overlap another's gather
-    // (fork/join by events)
+    // forward: per chunk of ZC slices, a row-FFT buffer and a Fourier grid (a
+    // buffer set; RSETS of them, a constant distance apart).  `streams`
+    // pipelines of RSETS / streams chunks per launch: pipeline 0 on the
+    // caller's stream, the others on side streams (fork/join by events), so
+    // one pipeline's FFTs overlap another's gather
     float2 *rbuf[RSETS] = {}, *fgrid[RSETS] = {};
     int streams = 4;   // 1, 2 or 4 (pt_radon_autotune chooses)
     cudaStream_t side[RSETS - 1] = {};
@@ -838,7 +942,7 @@ bool encode_grid_maps(pt_radon *h)
     const cuuint32_t estr[3] = {1, 1, 1};
     for (int b = 0; b < RSETS; ++b) {
         if (((uintptr_t)h->fgrid[b] & 127) != 0) return false;
-        if (encode(&h->tmap[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, h->fgrid[b], dims, strides, box, estr,
+        if (encode(&h->tmap.m[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, h->fgrid[b], dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
@@ -846,75 +950,75 @@ bool encode_grid_maps(pt_radon *h)
     return true;
 }
 
+template <int L>
+constexpr int ex_smem() { return (int)ptfft::Exchange<L, ZC>::BYTES; }
+template <int G>
+constexpr int col_smem() { return ZQ * G * (int)sizeof(float2); }
+
 template <int G>
 int set_attrs()
 {
     constexpr int N = G / 2;
-    const int s1 = ZC * (G + 1) * sizeof(float2);
-    const int s2 = CK * ZC * (G + 1) * sizeof(float2);
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_rows<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_cols<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
-    const int s4 = ZQ * (G + 1) * sizeof(float2);
-    PT_CUDA(cudaFuncSetAttribute(k_adj_colgather<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, s4));
-    PT_CUDA(cudaFuncSetAttribute(k_adj_colgather<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s4));
-    PT_CUDA(cudaFuncSetAttribute(k_adj_rows<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
-    PT_CUDA(cudaFuncSetAttribute(k_adj_rows_exact<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
-    const int s3 = ZC * (N + 1) * sizeof(float2);
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_lines<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_gather_tile<N, WKB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_smem<WKB>()));
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_gather_tile<N, WGAUSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_smem<WGAUSS>()));
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_gather_tma<N, WKB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tma_smem<WKB>()));
-    PT_CUDA(cudaFuncSetAttribute(k_fwd_gather_tma<N, WGAUSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tma_smem<WGAUSS>()));
-    PT_CUDA(cudaFuncSetAttribute(k_adj_lines<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
-    PT_CUDA(cudaFuncSetAttribute(k_adj_lines<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
+    static_assert(CK * ZH == ZC, "ex_smem serves the column kernel too");
+#define PT_ATTR(K, S) PT_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(S)))
+    PT_ATTR(k_fwd_rows<G>, ex_smem<G>());
+    PT_ATTR(k_fwd_cols<G>, ex_smem<G>());
+    PT_ATTR(k_adj_colgather<G>, col_smem<G>());
+    PT_ATTR((k_adj_colgather<G, true>), col_smem<G>());
+    PT_ATTR(k_adj_rows<G>, ex_smem<G>());
+    PT_ATTR(k_adj_rows_exact<G>, ex_smem<G>());
+    PT_ATTR(k_fwd_lines<N>, ex_smem<N>());
+    PT_ATTR(k_adj_lines<N>, ex_smem<N>());
+    PT_ATTR((k_adj_lines<N, true>), ex_smem<N>());
+    PT_ATTR((k_fwd_gather_tile<N, WKB>), tile_smem<WKB>());
+    PT_ATTR((k_fwd_gather_tile<N, WGAUSS>), tile_smem<WGAUSS>());
+    PT_ATTR((k_fwd_gather_tma<N, WKB>), tma_smem<WKB>());
+    PT_ATTR((k_fwd_gather_tma<N, WGAUSS>), tma_smem<WGAUSS>());
+#undef PT_ATTR
     return PT_OK;
 }
 
 template <int G, int W>
 int run_fwd(pt_radon *h, float2 *g, const float2 *f, float scale, cudaStream_t st)
 {
-    constexpr int N = G / 2, T = fft_threads<G>();
-    const size_t s1 = ZC * (G + 1) * sizeof(float2);
-    const size_t s2 = CK * ZC * (G + 1) * sizeof(float2);
-    const size_t s3 = ZC * (N + 1) * sizeof(float2);
+    constexpr int N = G / 2;
+    using EG = ptfft::Exchange<G, ZC>;
+    using EN = ptfft::Exchange<N, ZC>;
     const int nchunks = (h->nz + ZC - 1) / ZC;
-    // buffer sets in use: at most `streams`, the chunk count, and the number
-    // of ZC-slice line blocks the lines buffer holds (nzp / ZC)
-    const int sets = std::max(1, std::min(std::min(h->streams, nchunks), h->nzp / ZC));
+    // `streams` pipelines, each with `batch` buffer sets: a launch of pipeline p
+    // works on up to `batch` chunks in sets p batch ..., gathered into the same
+    // blocks of the lines buffer (nzp / ZC blocks, at least the chunk count)
+    const int batch = RSETS / h->streams;
+    const int sets = std::min(h->streams, (nchunks + batch - 1) / batch);   // pipelines in use
+    const size_t stride = h->rbuf[1] - h->rbuf[0];
+    const int npts = h->ntheta * N;
     if (sets > 1) {   // fork: the side streams start after everything queued on st so far
         PT_CUDA(cudaEventRecord(h->ev_fork, st));
         for (int k = 1; k < sets; ++k) PT_CUDA(cudaStreamWaitEvent(h->side[k - 1], h->ev_fork, 0));
     }
-    for (int c = 0; c < nchunks; ++c) {
-        const int z0 = c * ZC;
-        // chunk buffers: set c % sets on stream c % sets (a set is reused only
-        // by its own stream, in order); gathered lines at block (c % sets) of
-        // the lines buffer
-        const int k = c % sets;
-        cudaStream_t s = k ? h->side[k - 1] : st;
+    for (int c = 0, it = 0; c < nchunks; c += batch, ++it) {
+        // pipeline it % sets reuses its buffer sets in order on its own stream
+        const int p = it % sets, k = p * batch, cnt = std::min(batch, nchunks - c), z0 = c * ZC;
+        cudaStream_t s = p ? h->side[p - 1] : st;
         float2 *rb = h->rbuf[k], *fg = h->fgrid[k];
-        float2 *ln = h->lines + (size_t)k * h->ntheta * N * ZC;
-        k_fwd_rows<G><<<N, ZC * T, s1, s>>>(f, rb, h->nz, z0, h->deap, h->tw_G);
+        float2 *ln = h->lines + (size_t)k * npts * ZC;
+        k_fwd_rows<G><<<dim3(N, cnt), EG::NT, EG::BYTES, s>>>(f, rb, stride, h->nz, z0, h->deap, h->tw_fwd);
         PT_LAUNCHED("k_fwd_rows");
-        k_fwd_cols<G><<<G / CK, CK * ZC * T, s2, s>>>(rb, fg, h->tw_G);
+        k_fwd_cols<G><<<dim3(G / CK, ZC / ZH, cnt), EG::NT, EG::BYTES, s>>>(rb, fg, stride, h->tw_fwd);
         PT_LAUNCHED("k_fwd_cols");
-        const int npts = h->ntheta * N;
         if (h->gather == 2) {
-            k_fwd_gather_tma<N, W><<<h->nchunks, GPB * ZC, tma_smem<W>(), s>>>(h->tmap[k], ln, h->rec, h->chunks,
-                                                                              h->tma_err);
+            k_fwd_gather_tma<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tma_smem<W>(), s>>>(
+                h->tmap, k, ln, h->rec, h->chunks, npts, h->tma_err);
             PT_LAUNCHED("k_fwd_gather_tma");
         } else if (h->gather == 1) {
-            k_fwd_gather_tile<N, W><<<h->nchunks, GPB * ZC, tile_smem<W>(), s>>>(fg, ln, h->rec, h->chunks);
+            k_fwd_gather_tile<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tile_smem<W>(), s>>>(fg, stride, ln, h->rec,
+                                                                                           h->chunks, npts);
             PT_LAUNCHED("k_fwd_gather_tile");
         } else {
-            k_fwd_gather_pts<N, W><<<(npts + GPB - 1) / GPB, GPB * ZC, 0, s>>>(fg, ln, h->rec, npts);
+            k_fwd_gather_pts<N, W><<<dim3((npts + GPB - 1) / GPB, cnt), GPB * ZC, 0, s>>>(fg, stride, ln, h->rec, npts);
             PT_LAUNCHED("k_fwd_gather_pts");
         }
-        k_fwd_lines<N><<<h->ntheta, ZC * 32, s3, s>>>(ln, g, h->nz, z0, scale, h->tw_N);
+        k_fwd_lines<N><<<dim3(h->ntheta, cnt), EN::NT, EN::BYTES, s>>>(ln, g, h->nz, z0, scale, h->tw_inv_line);
         PT_LAUNCHED("k_fwd_lines");
     }
     for (int k = 1; k < sets; ++k) {   // join: st continues after every side stream's chunks
@@ -927,32 +1031,32 @@ int run_fwd(pt_radon *h, float2 *g, const float2 *f, float scale, cudaStream_t s
 template <int G>
 int run_adj(pt_radon *h, float2 *f, const float2 *g, float scale, cudaStream_t st, bool exact)
 {
-    constexpr int N = G / 2, n = G / 3, T = fft_threads<G>();
-    const size_t s1 = ZC * (G + 1) * sizeof(float2);
-    const size_t s3 = ZC * (N + 1) * sizeof(float2);
-    const size_t s4 = ZQ * (G + 1) * sizeof(float2);
+    constexpr int N = G / 2, n = G / 3;
+    using EG = ptfft::Exchange<G, ZC>;
+    using EN = ptfft::Exchange<N, ZC>;
     const float pre = radon_pre(h);
     const int nzp = h->nzp;
+    const dim3 glines(h->ntheta, nzp / ZC), gcols(nzp / ZQ, G);
     if (exact) {
-        k_adj_lines<N, true><<<dim3(h->ntheta, nzp / ZC), ZC * 32, s3, st>>>(g, h->lines, h->nz, nzp, pre, h->tw_N);
+        k_adj_lines<N, true><<<glines, EN::NT, EN::BYTES, st>>>(g, h->lines, h->nz, nzp, pre, h->tw_fwd_line);
         PT_LAUNCHED("k_adj_lines");
-        k_adj_colgather<G, true><<<dim3(nzp / ZQ, G), ZQ * T, s4, st>>>(h->lines, h->rbuf_adj, h->goff, h->gpt,
-                                                                       h->gw, h->col_order, nzp, h->tw_G);
+        k_adj_colgather<G, true><<<gcols, col_threads<G>(), col_smem<G>(), st>>>(
+            h->lines, h->rbuf_adj, h->goff, h->gpt, h->gw, h->col_order, nzp, h->tw_col1, h->tw_col2);
         PT_LAUNCHED("k_adj_colgather");
-        k_adj_rows_exact<G><<<dim3(N, nzp / ZC), ZC * T, s1, st>>>(h->rbuf_adj, f, h->mbuf, h->nz, nzp, h->deap,
-                                                                   scale, h->tw_G);
+        k_adj_rows_exact<G><<<dim3(N, nzp / ZC), EG::NT, EG::BYTES, st>>>(h->rbuf_adj, f, h->mbuf, h->nz, nzp, h->deap,
+                                                                         scale, h->tw_adj);
         PT_LAUNCHED("k_adj_rows_exact");
         const size_t cnt = (size_t)h->nz * n;
-        k_adj_fold_rows<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(h->mbuf, f, h->nz, n, N / 6, n / 2 + 2);
+        k_adj_fold_rows<<<dim3((unsigned)((cnt + 127) / 128), 2), 128, 0, st>>>(h->mbuf, f, h->nz, n, N / 6, n / 2 + 2);
         PT_LAUNCHED("k_adj_fold_rows");
         return PT_OK;
     }
-    k_adj_lines<N><<<dim3(h->ntheta, nzp / ZC), ZC * 32, s3, st>>>(g, h->lines, h->nz, nzp, pre, h->tw_N);
+    k_adj_lines<N><<<glines, EN::NT, EN::BYTES, st>>>(g, h->lines, h->nz, nzp, pre, h->tw_fwd_line);
     PT_LAUNCHED("k_adj_lines");
-    k_adj_colgather<G><<<dim3(nzp / ZQ, G), ZQ * T, s4, st>>>(h->lines, h->rbuf_adj, h->goff, h->gpt, h->gw,
-                                                             h->col_order, nzp, h->tw_G);
+    k_adj_colgather<G><<<gcols, col_threads<G>(), col_smem<G>(), st>>>(
+        h->lines, h->rbuf_adj, h->goff, h->gpt, h->gw, h->col_order, nzp, h->tw_col1, h->tw_col2);
     PT_LAUNCHED("k_adj_colgather");
-    k_adj_rows<G><<<dim3(n, nzp / ZC), ZC * T, s1, st>>>(h->rbuf_adj, f, h->nz, nzp, h->deap, scale, h->tw_G);
+    k_adj_rows<G><<<dim3(n, nzp / ZC), EG::NT, EG::BYTES, st>>>(h->rbuf_adj, f, h->nz, nzp, h->deap, scale, h->tw_adj);
     PT_LAUNCHED("k_adj_rows");
     return PT_OK;
 }
@@ -1002,8 +1106,8 @@ template <int G, int W>
 int run_tma_wait_check(pt_radon *h, cudaStream_t st)
 {
     constexpr int N = G / 2;
-    k_fwd_gather_tma<N, W><<<h->nchunks, GPB * ZC, tma_smem<W>(), st>>>(h->tmap[0], h->lines, h->rec, h->chunks,
-                                                                        h->tma_err, 256, 1);
+    k_fwd_gather_tma<N, W><<<h->nchunks, GPB * ZC, tma_smem<W>(), st>>>(h->tmap, 0, h->lines, h->rec, h->chunks,
+                                                                        h->ntheta * N, h->tma_err, 256, 1);
     PT_LAUNCHED("k_fwd_gather_tma");
     return PT_OK;
 }
@@ -1031,6 +1135,57 @@ int dmalloc(T **p, size_t count)
         return PT_ERR_ALLOC;
     }
     return PT_OK;
+}
+
+// exp(dir 2 pi i m / L) times (-1)^neg, in double
+float2 unit_root(long long m, int L, int dir, int neg)
+{
+    const double a = dir * 2.0 * M_PI * (double)(m % L) / L, s = (neg & 1) ? -1.0 : 1.0;
+    return make_float2((float)(s * std::cos(a)), (float)(s * std::sin(a)));
+}
+
+// The twiddle tables of the handle's lengths (see ptfft::Exchange and fft3).
+cudaError_t upload_twiddles(pt_radon *h)
+{
+    // extra(i2, k1): quarter turns (times dir) the table adds to W^(i2 k1)
+    auto pairs = [](int L, int dir, auto &&extra) {
+        const int R1 = ptfft::split_r1(L), R2 = ptfft::split_r2(L);
+        std::vector<float4> t((size_t)L / 2);
+        for (int j = 0; j < R1 / 2; ++j)
+            for (int i2 = 0; i2 < R2; ++i2) {
+                float2 w[2];
+                for (int o = 0; o < 2; ++o) {
+                    const int k1 = 2 * j + o;
+                    w[o] = unit_root((long long)i2 * k1 + (long long)extra(i2, k1) * (L / 4), L, dir, 0);
+                }
+                t[(size_t)j * R2 + i2] = make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+            }
+        return t;
+    };
+    const int G = h->G, N = h->N;
+    // (-i)^k1 of the shifted rows times (-1)^k1, in quarter turns of exp(-2 pi i / 4): 3 k1
+    const auto fwd = pairs(G, -1, [](int, int k1) { return 3 * k1; });
+    const auto adj = pairs(G, +1, [](int i2, int) { return 2 * i2; });
+    const auto lf = pairs(N, -1, [](int i2, int k1) { return 2 * (i2 + k1); });
+    const auto li = pairs(N, +1, [](int i2, int k1) { return 2 * (i2 + k1); });
+    const int A = ptfft::split3_a(G), C = ptfft::split3_c(G), B = ptfft::split3_b(G), BC = B * C;
+    std::vector<float2> t1(G), t2(BC);
+    for (int k1 = 0; k1 < A; ++k1)
+        for (int i = 0; i < BC; ++i) t1[(size_t)k1 * BC + i] = unit_root((long long)i * k1, G, +1, 0);
+    for (int k2 = 0; k2 < B; ++k2)
+        for (int i3 = 0; i3 < C; ++i3) t2[(size_t)k2 * C + i3] = unit_root((long long)i3 * k2, BC, +1, i3);
+    struct {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    } up[] = {{h->tw_fwd, fwd.data(), fwd.size() * sizeof(float4)},    {h->tw_adj, adj.data(), adj.size() * sizeof(float4)},
+              {h->tw_fwd_line, lf.data(), lf.size() * sizeof(float4)}, {h->tw_inv_line, li.data(), li.size() * sizeof(float4)},
+              {h->tw_col1, t1.data(), t1.size() * sizeof(float2)},     {h->tw_col2, t2.data(), t2.size() * sizeof(float2)}};
+    for (const auto &u : up) {
+        const cudaError_t e = cudaMemcpy(u.dst, u.src, u.bytes, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 int check_device(const pt_radon *h)
@@ -1096,8 +1251,12 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
         if (rc == PT_OK) cuts(cut);
     };
     carve(h->tables, [&](auto &cut) {
-        cut(h->tw_G, (size_t)G);
-        cut(h->tw_N, N);
+        cut(h->tw_fwd, (size_t)G / 2);
+        cut(h->tw_adj, (size_t)G / 2);
+        cut(h->tw_fwd_line, N / 2);
+        cut(h->tw_inv_line, N / 2);
+        cut(h->tw_col1, (size_t)G);
+        cut(h->tw_col2, (size_t)G);
         cut(h->theta, ntheta);
         cut(h->x, npts);
         cut(h->y, npts);
@@ -1119,9 +1278,11 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
     });
     if (rc == PT_OK && cudaMemset(h->tma_err, 0, sizeof(int)) == cudaSuccess)
         h->tma_ok = encode_grid_maps(h);   // gather 2 is offered only if every map encodes
-    // default variant (the autotuner's usual choice from 128^3 up, within a
-    // few percent at 64^3): four chunk pipelines, TMA-staged tiles
-    h->streams = 4;
+    // default variant: two pipelines of two chunks per launch, TMA-staged tiles.
+    // Against four pipelines of one (us): 32 wide, 9 slices 25 and 42; 64^3 55
+    // and 123; 128 x 84 slices 140 and 144; 128^3 231 and 215; 256^3 1437 and
+    // 1443.  One pipeline of four is slower from 64^3 up (60, 148, 237, 1598)
+    h->streams = 2;
     h->gather = h->tma_ok ? 2 : 1;
     if (rc == PT_OK && cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess) rc = PT_ERR_CUDA;
     for (int k = 0; k < RSETS - 1 && rc == PT_OK; ++k)
@@ -1138,14 +1299,7 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
     if (rc == PT_OK) rc = dmalloc(&h->mbuf, (n / 2 + 2) * (size_t)nz * n);
     if (rc == PT_OK) rc = radon_set_attrs(G);
     if (rc == PT_OK) {
-        std::vector<float2> tw(G);
-        pt_make_twiddles(tw.data(), G);
-        if (cudaMemcpy(h->tw_G, tw.data(), G * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = PT_ERR_CUDA;
-        pt_make_twiddles(tw.data(), (int)N);
-        if (rc == PT_OK &&
-            cudaMemcpy(h->tw_N, tw.data(), N * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = PT_ERR_CUDA;
+        if (upload_twiddles(h) != cudaSuccess) rc = PT_ERR_CUDA;
         if (rc == PT_OK && h->inv1) {
             // transform of I0(beta sqrt(1 - (2 d / W)^2)) / I0(beta) (d in cells of
             // the G grid) at pixel t: W sinh(s) / s / I0(beta), s^2 = beta^2 - (pi W t / G)^2
@@ -1240,10 +1394,10 @@ extern "C" int pt_radon_setobj(pt_radon *h, const float *theta, void *stream)
         PT_CUDA(cudaMemcpyAsync(h->perm, perm.data(), npts * sizeof(int), cudaMemcpyHostToDevice, st));
         const unsigned blocks = (unsigned)((npts + 255) / 256);
         if (W == WKB)
-            k_point_records<WKB><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts, N,
+            k_point_records<WKB><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts,
                                                          radon_pre(h));
         else
-            k_point_records<WGAUSS><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts, N,
+            k_point_records<WGAUSS><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts,
                                                             radon_pre(h));
         PT_LAUNCHED("k_point_records");
         // the tiled gather's blocks: runs of one tile in perm order, at most TCH points each
@@ -1379,9 +1533,8 @@ extern "C" int pt_radon_adj_scaled(pt_radon *h, void *f, const void *g, float sc
     return radon_call(h, true, f, g, scale, stream);
 }
 
-// Autotuner: times the forward with its chunks on one stream and pipelined on
-// two, each with the gather through L1 and from shared-memory tiles, and
-// keeps the fastest (setup-time; blocks the host).
+// Autotuner: times the forward with one, two and four pipelines, each with the
+// three gathers, and keeps the fastest (setup-time; blocks the host).
 extern "C" int pt_radon_autotune(pt_radon *h, void *g, const void *f, int trials, int *streams_out, void *stream)
 {
     pt::clear_error();

@@ -56,11 +56,12 @@ class radonusfft:  # noqa: N801 - reference class name
               "radonusfft.adj_exact")
 
     def autotune(self, g, f, trials=3, stream=None):
-        """Time the forward with its slice chunks on one stream and pipelined
-        on two and on four, each with the gather through L1, from
-        shared-memory tiles and from TMA-staged tiles; keep the fastest for
-        this operator.  g, f: buffers of fwd's shapes (g is overwritten).
-        Returns (streams, gather), gather 0 (L1), 1 (tiles) or 2 (TMA tiles)."""
+        """Time the forward with its slice chunks in one pipeline of four per
+        launch, two of two and four of one (on as many streams), each with the
+        gather through L1, from shared-memory tiles and from TMA-staged tiles;
+        keep the fastest for this operator.  g, f: buffers of fwd's shapes (g is
+        overwritten).  Returns (streams, gather), gather 0 (L1), 1 (tiles) or 2
+        (TMA tiles)."""
         out = ctypes.c_int()
         check(lib().pt_radon_autotune(self._h, as_ptr(g), as_ptr(f), int(trials), ctypes.byref(out), _s(stream)),
               "radonusfft.autotune")
