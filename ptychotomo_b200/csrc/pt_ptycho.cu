@@ -3,14 +3,11 @@
 // Replaces class ptychofft of the reference (src/cuda/ptychofft.cu:1-93,
 // kernels mul/mula/takeshifts/shifts/shiftsa in src/include/kernels.cuh).
 //
-//  forward  g = F Q psi   (ptychofft.cu:58-76): one block per frame
-//    (angle, scan).  Each 1-D DFT of length det is a four-step factorisation
-//    det = N1 x N2: N1 points per thread in registers, N2 threads per line,
-//    one swizzled shared-memory exchange inside the group.  The probe-weighted
-//    patch (detector row = object column, kernels.cuh:257-263) is loaded
-//    straight into registers, transformed along the object row, transposed
-//    once through shared memory, transformed along the other axis and written
-//    with the per-scan phase (kernels.cuh:306-336) applied.
+//  forward  g = F Q psi   (ptychofft.cu:58-76): the probe-weighted patch
+//    (detector row = object column, kernels.cuh:257-263) is loaded straight
+//    into registers, transformed in three register rounds with two trips
+//    through shared memory, and written with the per-scan phase
+//    (kernels.cuh:306-336) applied.
 //  adjoint  psi = Q* F* g (ptychofft.cu:78-93): the same transform in reverse;
 //    block (part, angle) walks scans s = part, part + parts, ... in order and
 //    accumulates conj(probe) x frame into its own slab; with parts > 1 the
@@ -160,216 +157,303 @@ __global__ void __launch_bounds__(ptycho_block<DET>(), 1)
 }
 
 
-// ---- register four-step transforms (det >= 16) -----------------------------
+// ---- frames of det x det, det = 16 to 64, in three register rounds -----------
+// B[u][v] = f sum_{r,q} A[r][q] w^(DIR (u r + v q)), w = exp(2 pi i / det),
+// for a det x det array A whose q runs along memory.  r = rt + RT m and
+// u = k1 + 16 k2 split the r transform 16 x RT, q = qb + 16 qa and
+// v = v1 + QA v2 the q transform QA x 16:
+//   R1  thread (q, rt): 16-point DFT over m, times w^(rt k1)
+//   R2  (k1, qb): RT-point DFT over rt (gives k2), QA-point DFT over qa
+//       (gives v1), times w^(qb v1) f
+//   R3  thread (u, v1): 16-point DFT over qb (gives v2)
+// The forward takes A = probe x patch [y][x] and stores frame[kx = v][ky = u];
+// the adjoint takes A = frame[kx][ky] and adds pixel [y = v][x = u].  Both
+// touch memory in whole row segments.
+//
+// Between the rounds the frame sits in shared memory as rows (k1, j) of 16
+// values qb, j = qa RT + rt after R1 and v1 RT + k2 after R2: R2 reads and
+// writes the same slots, so it needs no barrier of its own.  The row's 16-byte
+// slots are XORed with k1 & 7, so R3's 16-byte reads of eight consecutive u
+// fall on eight different slots; every access takes the minimum number of
+// wavefronts.
+//
+// 16 values per thread keep the kernels at 80 registers, so several blocks
+// share an SM and one's loads and stores run under another's arithmetic; a
+// row / transpose / column form with 512-thread blocks ran one block per SM
+// with four barriers per frame.  A probe smaller than the detector leaves
+// most of A zero (forward) or most of B unused (adjoint): R1 (R3) then runs
+// on the probe's columns only, packed onto the first threads, and R2 skips
+// the slots outside it.
+// 192 angles x 225 scans, 64 x 64 detector, 16-pixel probe, forward: 1.04 ->
+// 0.38 ms; Poisson gradient of 128 x 49 scans of a 64-pixel probe: 0.31 ->
+// 0.13 ms.
 template <int DET>
-struct PF {
-    static constexpr int N2 = DET >= 64 ? 8 : 4;           // threads per line
-    static constexpr int N1 = DET / N2;                    // points per thread
-    static constexpr int KPT = N1 / N2;                    // k1 values per thread after the exchange
-    static constexpr int NT = DET * N2 < 512 ? DET * N2 : 512;  // threads per block
-    static constexpr int NG = NT / N2;                     // thread groups
-    static constexpr int CPG = DET / NG;                   // lines per group
-    static constexpr int P = DET + 8;                      // frame pitch (P = 8 mod 16)
-    static constexpr size_t SMEM = (size_t)(DET * P + DET) * sizeof(float2);
+struct FR {
+    static constexpr int QA = DET / 16, RT = DET / 16, J = QA * RT;
+    static constexpr int NT = DET * QA;                  // threads per frame
+    static constexpr int FPB = NT < 32 ? 32 / NT : 1;    // frames per block
+    static constexpr int BLOCK = NT * FPB;
+    static constexpr int R2C = 256 / NT;                 // (k1, qb) pairs per thread
+    static constexpr int BPS = 768 / BLOCK;              // resident blocks per SM at 80 registers a thread
+    static constexpr int BPSP = 512 / BLOCK;             // probe adjoint: 128 registers
+    static constexpr size_t SMEM = (size_t)FPB * DET * DET * sizeof(float2);
+    static_assert(DET * RT == NT, "R1 and R3 give every thread one line of 16");
 };
 
-// frame swizzle: row r, column c live at r * P + (c ^ fswz(r))
-template <int DET>
-__device__ __forceinline__ int fswz(int r)
-{
-    return ((r / PF<DET>::KPT) % PF<DET>::N2) * 2;
-}
+// Byte offset of row (0, j), value qb, before the XOR of k1; row (k1, j) is
+// k1 J rows of 128 bytes further on.  Written so that the compile-time index
+// of each round (k1 in R1, the row j in R2, the slot in R3) is an XOR or an
+// immediate offset on one register.
+__device__ __forceinline__ unsigned fr_off(int j, int qb) { return ((unsigned)j << 7) + ((unsigned)qb << 3); }
+__device__ __forceinline__ float2 *fr_ptr(float2 *ex, unsigned off) { return reinterpret_cast<float2 *>(reinterpret_cast<char *>(ex) + off); }
 
-// DFT of one line held as v[m] = x[t + N2 m] by the N2 threads t of a group.
-// On return v[j N2 + k2] = X[t KPT + j + N1 k2].  `sc` is the group's
-// scratch (DET + 1 complex), `tws` the table exp(-2 pi i m / DET).
+// R1 of a line v[m] = A[rt + RT m][q]; w holds exp(-2 pi i m / DET)
 template <int DET, int DIR>
-__device__ __forceinline__ void line_dft(float2 (&v)[PF<DET>::N1], int t, float2 *sc, const float2 *tws)
+__device__ __forceinline__ void fr_r1(float2 (&v)[16], float2 *ex, int q, int rt, const float2 *__restrict__ w)
 {
-    using F = PF<DET>;
-    ptfft::Dft<F::N1, DIR>::run(v);
+    constexpr int RT = FR<DET>::RT;
+    ptfft::Dft<16, DIR, true>::run(v);
+    if constexpr (RT > 1) {
 #pragma unroll
-    for (int k1 = 1; k1 < F::N1; ++k1) {
-        float2 w = tws[t * k1];
-        if (DIR > 0) w.y = -w.y;
-        v[k1] = cmul(v[k1], w);
+        for (int k1 = 1; k1 < 16; ++k1) {
+            float2 t = __ldg(&w[rt * k1]);
+            if (DIR > 0) t.y = -t.y;
+            v[k1] = cmul(v[k1], t);
+        }
     }
-    __syncwarp();
+    const unsigned o = fr_off((q >> 4) * RT + rt, q & 15);
 #pragma unroll
-    for (int k1 = 0; k1 < F::N1; ++k1) sc[t * F::N1 + ((k1 + t * F::KPT) % F::N1)] = v[k1];
-    __syncwarp();
+    for (int k1 = 0; k1 < 16; ++k1) *fr_ptr(ex, (o ^ ((k1 & 7) << 4)) + k1 * FR<DET>::J * 128) = v[k1];
+}
+
+// R2 in place.  in(q): whether R1 wrote column q (the others are zero);
+// out(u): whether R3 reads row u.
+template <int DET, int DIR, typename In, typename Out>
+__device__ __forceinline__ void fr_r2(float2 *ex, int t, float2 f, const float2 *__restrict__ w, In in, Out out)
+{
+    using F = FR<DET>;
 #pragma unroll
-    for (int j = 0; j < F::KPT; ++j) {
-        float2 u[F::N2];
-        const int k1 = t * F::KPT + j;
+    for (int c = 0; c < F::R2C; ++c) {
+        const int item = t + c * F::NT, k1 = item >> 4, qb = item & 15;
+        float2 *s = fr_ptr(ex, (fr_off(0, qb) ^ ((k1 & 7) << 4)) + k1 * F::J * 128);
+        float2 a[F::QA][F::RT];
 #pragma unroll
-        for (int n2 = 0; n2 < F::N2; ++n2) u[n2] = sc[n2 * F::N1 + ((k1 + n2 * F::KPT) % F::N1)];
-        ptfft::Dft<F::N2, DIR>::run(u);
+        for (int qa = 0; qa < F::QA; ++qa) {
+            const bool ok = in(qb + 16 * qa);
 #pragma unroll
-        for (int k2 = 0; k2 < F::N2; ++k2) v[j * F::N2 + k2] = u[k2];
+            for (int rt = 0; rt < F::RT; ++rt) a[qa][rt] = ok ? s[(qa * F::RT + rt) * 16] : czero();
+            ptfft::Dft<F::RT, DIR, true>::run(a[qa]);
+        }
+#pragma unroll
+        for (int k2 = 0; k2 < F::RT; ++k2) {
+            float2 b[F::QA];
+#pragma unroll
+            for (int qa = 0; qa < F::QA; ++qa) b[qa] = a[qa][k2];
+            ptfft::Dft<F::QA, DIR, true>::run(b);
+#pragma unroll
+            for (int v1 = 0; v1 < F::QA; ++v1) a[v1][k2] = b[v1];
+        }
+#pragma unroll
+        for (int v1 = 0; v1 < F::QA; ++v1) {
+            float2 t1 = f;
+            if (v1 > 0) {
+                t1 = __ldg(&w[qb * v1]);
+                if (DIR > 0) t1.y = -t1.y;
+                t1 = cmul(t1, f);
+            }
+#pragma unroll
+            for (int k2 = 0; k2 < F::RT; ++k2)
+                if (out(k1 + 16 * k2)) s[(v1 * F::RT + k2) * 16] = cmul(a[v1][k2], t1);
+        }
     }
 }
 
-template <int DET, bool SUB = false>
-__global__ void __launch_bounds__(PF<DET>::NT, 1)
+// R3's read of row (u, v1)
+template <int DET>
+__device__ __forceinline__ void fr_r3_read(float2 (&v)[16], const float2 *ex, int u, int v1)
+{
+    const int k1 = u & 15;
+    const unsigned o = ((k1 * FR<DET>::J + v1 * FR<DET>::RT + (u >> 4)) << 7) + ((k1 & 7) << 4);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const float4 x = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(ex) + (o ^ (s << 4)));
+        v[2 * s] = make_float2(x.x, x.y);
+        v[2 * s + 1] = make_float2(x.z, x.w);
+    }
+}
+
+// An opaque copy of a thread index: what is derived from it (slot and window
+// addresses, twiddles) is formed where it is used in each frame, instead of
+// being hoisted out of the frame loop into registers.
+__device__ __forceinline__ int fresh(int t)
+{
+    asm volatile("mov.b32 %0, %0;" : "+r"(t));
+    return t;
+}
+
+template <int DET, bool FULL, bool SUB = false>
+__global__ void __launch_bounds__(FR<DET>::BLOCK, FR<DET>::BPS)
     k_ptycho_fwd(const float2 *__restrict__ psi, float2 *__restrict__ g, const int *__restrict__ corner,
                  const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan,
-                 int nframes, int P, float scale, const float2 *__restrict__ tw, const int *__restrict__ sid = nullptr)
+                 int nframes, int P, float scale, const float2 *__restrict__ w, const int *__restrict__ sid = nullptr)
 {
-    using F = PF<DET>;
-    extern __shared__ float2 sm[];
-    float2 *fr = sm;
-    float2 *tws = sm + DET * F::P;
-    for (int i = threadIdx.x; i < DET; i += F::NT) tws[i] = tw[i];
-    const int t = threadIdx.x % F::N2, grp = threadIdx.x / F::N2;
-    float2 *sc = fr + grp * (DET + 1);
-    const int off = (DET - P) / 2;
-    __syncthreads();
-    for (int fid = blockIdx.x; fid < nframes; fid += gridDim.x) {
-        const int th = fid / nscan;
-        const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
-        float2 *out = g + (size_t)fid * DET * DET;
-        if (stx < 0 || sty < 0) {  // skipped scan: the reference leaves a zero frame
-            for (int e = threadIdx.x; e < DET * DET; e += F::NT) out[e] = czero();
-            continue;
-        }
-        const float2 *src = psi + ((size_t)th * nz + sty) * n + stx;
-        const float2 *pr = SUB ? prbT + (size_t)sid[fid] * P * P : prbT;  // sub-pixel: the frame's shifted probe
-        float2 v[F::CPG][F::N1];
-        // along the object row: line = detector column iy, points ix = t + N2 m
+    using F = FR<DET>;
+    extern __shared__ float4 sm4[];
+    const int t0 = threadIdx.x % F::NT, sub = threadIdx.x / F::NT;
+    float2 *ex = reinterpret_cast<float2 *>(sm4) + sub * DET * DET;
+    const int PW = FULL ? DET : P, off0 = FULL ? 0 : (DET - P) / 2;
+    // R1's line: column px of the window, rows rt + RT m
+    const int px0 = t0 % PW, rt0 = t0 / PW;
+    const bool line = rt0 < F::RT;
+    for (int f0 = blockIdx.x * F::FPB; f0 < nframes; f0 += gridDim.x * F::FPB) {
+        const int fid = f0 + sub;
+        const bool have = fid < nframes;
+        const int stx = have ? corner[2 * fid] : -1, sty = have ? corner[2 * fid + 1] : -1;
+        const bool act = stx >= 0 && sty >= 0;
+        const int t = fresh(t0), px = fresh(px0), rt = fresh(rt0), off = FULL ? 0 : fresh(off0);
+        if (act && line) {
+            const float2 *src = psi + ((size_t)(fid / nscan) * nz + sty) * n + stx + px;
+            const float2 *pr = (SUB ? prbT + (size_t)sid[fid] * P * P : prbT) + px;  // sub-pixel: the frame's shifted probe
+            float2 v[16];
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int py = grp + F::NG * c - off;
-#pragma unroll
-            for (int m = 0; m < F::N1; ++m) {
-                const int px = t + F::N2 * m - off;
-                float2 val = czero();
-                if (py >= 0 && py < P && px >= 0 && px < P)
-                    val = cmul(__ldg(&pr[py * P + px]), __ldg(&src[(size_t)py * n + px]));
-                v[c][m] = val;
+            for (int m = 0; m < 16; ++m) {
+                const int py = rt + F::RT * m - off;
+                v[m] = FULL || (py >= 0 && py < P) ? cmul(__ldg(&pr[py * PW]), __ldg(&src[(size_t)py * n])) : czero();
             }
-            line_dft<DET, -1>(v[c], t, sc, tws);
+            fr_r1<DET, -1>(v, ex, off + px, rt, w);
         }
         __syncthreads();
-#pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int iy = grp + F::NG * c;
-#pragma unroll
-            for (int j = 0; j < F::KPT; ++j)
-#pragma unroll
-                for (int k2 = 0; k2 < F::N2; ++k2) {
-                    const int kx = t * F::KPT + j + F::N1 * k2;
-                    fr[kx * F::P + (iy ^ fswz<DET>(kx))] = v[c][j * F::N2 + k2];
-                }
-        }
+        if (act)
+            fr_r2<DET, -1>(ex, t, scale * phase[fid], w, [&](int q) { return FULL || (q >= off && q < off + P); },
+                           [](int) { return true; });
         __syncthreads();
+        float2 v[16];
+        const int u = t % DET, v1 = t / DET;
+        if (act) fr_r3_read<DET>(v, ex, u, v1);
+        __syncthreads();  // read: the next frame's R1 may write
+        if (!have) continue;
+        float2 *out = g + (size_t)fid * DET * DET;
+        if (act) {
+            ptfft::Dft<16, -1, true>::run(v);
+        } else {   // skipped scan: the reference leaves a zero frame
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int kx = grp + F::NG * c;
-            const int sw = fswz<DET>(kx);
-#pragma unroll
-            for (int m = 0; m < F::N1; ++m) v[c][m] = fr[kx * F::P + ((t + F::N2 * m) ^ sw)];
+            for (int v2 = 0; v2 < 16; ++v2) v[v2] = czero();
         }
-        __syncthreads();
-        const float2 ph = scale * phase[fid];
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            line_dft<DET, -1>(v[c], t, sc, tws);
-            const int kx = grp + F::NG * c;
-#pragma unroll
-            for (int k2 = 0; k2 < F::N2; ++k2)
-#pragma unroll
-                for (int j = 0; j < F::KPT; ++j)
-                    out[kx * DET + t * F::KPT + j + F::N1 * k2] = cmul(v[c][j * F::N2 + k2], ph);
-        }
-        __syncthreads();
+        for (int v2 = 0; v2 < 16; ++v2) __stcs(&out[(v1 + F::QA * v2) * DET + u], v[v2]);  // frame[kx][ky = u]
     }
 }
 
-// grid (parts, ntheta): block (part, angle) owns slab dst[angle][part]
-template <int DET, int RESID, bool SUB = false>
-__global__ void __launch_bounds__(PF<DET>::NT, 1)
-    k_ptycho_adj(const float2 *__restrict__ g, float2 *__restrict__ dst, const int *__restrict__ corner,
-                 const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan,
-                 int P, float scale, const float2 *__restrict__ tw, const float *__restrict__ data, float dscale,
-                 const int *__restrict__ sid = nullptr)
+// Object adjoint: grid (parts, ntheta), block (part, angle) owns slab
+// dst[angle][part].  PROBE (the adjoint with respect to the probe): grid
+// (blocks, 1), block b walks frames b, b + gridDim.x, ... < nframes (FPB at a
+// time) and sums conj(psi patch) x frame into its P x P partial dst[b]; each
+// element belongs to one thread, which keeps it in registers (FPB = 1).
+template <int DET, bool FULL, int RESID, bool SUB = false, bool PROBE = false>
+__global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET>::BPS)
+    k_ptycho_adj(const float2 *__restrict__ g, float2 *dst, const int *__restrict__ corner,
+                 const float2 *__restrict__ phase, const float2 *prbT, int nz, int n, int nscan, int P, float scale,
+                 const float2 *__restrict__ w, const float *__restrict__ data, float dscale,
+                 const int *__restrict__ sid = nullptr, const float2 *psi = nullptr, int nframes = 0)
 {
-    using F = PF<DET>;
-    extern __shared__ float2 sm[];
-    float2 *fr = sm;
-    float2 *tws = sm + DET * F::P;
-    const int part = blockIdx.x, parts = gridDim.x, th = blockIdx.y;
-    float2 *slab = dst + ((size_t)th * parts + part) * nz * n;
-    for (int i = threadIdx.x; i < DET; i += F::NT) tws[i] = tw[i];
-    for (int e = threadIdx.x; e < nz * n; e += F::NT) slab[e] = czero();
-    const int t = threadIdx.x % F::N2, grp = threadIdx.x / F::N2;
-    float2 *sc = fr + grp * (DET + 1);
-    const int off = (DET - P) / 2;
-    __syncthreads();
-    for (int s = part; s < nscan; s += parts) {
-        const int fid = th * nscan + s;
-        const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
-        if (stx < 0 || sty < 0) continue;
-        const float2 ph = phase[fid];
-        const float2 *pr = SUB ? prbT + (size_t)sid[fid] * P * P : prbT;
-        const float2 *in = g + (size_t)fid * DET * DET;
-        float2 v[F::CPG][F::N1];
-        // along the detector row: line = kx, points ky = t + N2 m (contiguous)
+    using F = FR<DET>;
+    extern __shared__ float4 sm4[];
+    const int t0 = threadIdx.x % F::NT, sub = threadIdx.x / F::NT;
+    float2 *ex = reinterpret_cast<float2 *>(sm4) + sub * DET * DET;
+    const int part = blockIdx.x, parts = gridDim.x, th0 = blockIdx.y;
+    const int PW = FULL ? DET : P, off0 = FULL ? 0 : (DET - P) / 2;
+    // R3's line: window column px (= u - off), rows v1 + QA v2
+    const int px0 = t0 % PW, v10 = t0 / PW;
+    const bool line = v10 < F::QA;
+    float2 *slab = PROBE ? dst + (size_t)(part * F::FPB + sub) * P * P : dst + ((size_t)th0 * parts + part) * nz * n;
+    if (!PROBE)
+        for (int e = threadIdx.x; e < nz * n; e += F::BLOCK) slab[e] = czero();
+    float2 acc[PROBE ? 16 : 1];
+    if constexpr (PROBE) {
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int kx = grp + F::NG * c;
+        for (int v2 = 0; v2 < 16; ++v2) acc[v2] = czero();
+    }
+    const int count = PROBE ? nframes : nscan;
+    for (int s0 = part * F::FPB; s0 < count; s0 += parts * F::FPB) {
+        const int s = s0 + sub;
+        const int fid = PROBE ? s : th0 * nscan + s;
+        const bool have = s < count;
+        const int stx = have ? corner[2 * fid] : -1, sty = have ? corner[2 * fid + 1] : -1;
+        const bool act = stx >= 0 && sty >= 0;
+        if (F::FPB == 1 && !act) continue;
+        const int t = fresh(t0), px = fresh(px0), v1 = fresh(v10), off = FULL ? 0 : fresh(off0);
+        if (act) {
+            const int ky = t % DET, rt = t / DET;
+            const size_t e0 = (size_t)fid * DET * DET + rt * DET + ky;
+            float2 v[16];
 #pragma unroll
-            for (int m = 0; m < F::N1; ++m) {
-                const int e = kx * DET + t + F::N2 * m;
-                v[c][m] = scale * cmulc(ph, resid<RESID>(__ldg(&in[e]), data, (size_t)fid * DET * DET + e, dscale));
+            for (int m = 0; m < 16; ++m) v[m] = __ldcs(&g[e0 + m * F::RT * DET]);
+            if constexpr (RESID != 0) {
+                float d[16];
+#pragma unroll
+                for (int m = 0; m < 16; ++m) d[m] = __ldcs(&data[e0 + m * F::RT * DET]);
+#pragma unroll
+                for (int m = 0; m < 16; ++m) v[m] = resid_of<RESID>(v[m], d[m] * dscale);
             }
-            line_dft<DET, +1>(v[c], t, sc, tws);
+            fr_r1<DET, +1>(v, ex, ky, rt, w);
         }
         __syncthreads();
+        if (act) {
+            const float2 ph = phase[fid];
+            fr_r2<DET, +1>(ex, t, make_float2(scale * ph.x, -scale * ph.y), w, [](int) { return true; },
+                           [&](int u) { return FULL || (u >= off && u < off + P); });
+        }
+        __syncthreads();
+        float2 v[16];
+        if (act && line) fr_r3_read<DET>(v, ex, off + px, v1);
+        __syncthreads();  // read: the next frame's R1 may write
+        if (act && line) ptfft::Dft<16, +1, true>::run(v);
+        // object: slab += conj(probe) x value; probe: sum of conj(psi) x value
+        const float2 *mul = PROBE ? psi + ((size_t)(fid / nscan) * nz + sty) * n + stx + px
+                                  : (SUB ? prbT + (size_t)(act ? sid[fid] : 0) * P * P : prbT) + px;
+        const size_t ms = PROBE ? n : PW;
+        // frames of one block that share a slab add to it one after the other
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int kx = grp + F::NG * c;
+        for (int o = 0; o < (PROBE ? 1 : F::FPB); ++o) {
+            if (!PROBE && o > 0) __syncthreads();
+            if (!act || !line || (!PROBE && F::FPB > 1 && sub != o)) continue;
+            if constexpr (PROBE) {
 #pragma unroll
-            for (int j = 0; j < F::KPT; ++j)
-#pragma unroll
-                for (int k2 = 0; k2 < F::N2; ++k2) {
-                    const int iy = t * F::KPT + j + F::N1 * k2;
-                    fr[iy * F::P + (kx ^ fswz<DET>(iy))] = v[c][j * F::N2 + k2];
+                for (int v2 = 0; v2 < 16; ++v2) {
+                    const int py = v1 + F::QA * v2 - off;
+                    if (FULL || (py >= 0 && py < P)) acc[v2] = acc[v2] + cmulc(__ldg(&mul[py * ms]), v[v2]);
                 }
-        }
-        __syncthreads();
+            } else {
+                float2 *col = slab + (size_t)sty * n + stx + px;
+                // RB rows at a time: their loads are issued before the first store
+                constexpr int RB = FULL ? 8 : 4;
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int iy = grp + F::NG * c;
-            const int sw = fswz<DET>(iy);
+                for (int h = 0; h < 16; h += RB) {
+                    float2 cur[RB], pv[RB];
 #pragma unroll
-            for (int m = 0; m < F::N1; ++m) v[c][m] = fr[iy * F::P + ((t + F::N2 * m) ^ sw)];
-        }
-        __syncthreads();
+                    for (int j = 0; j < RB; ++j) {
+                        const int py = v1 + F::QA * (h + j) - off;
+                        const bool ok = FULL || (py >= 0 && py < P);
+                        pv[j] = ok ? __ldg(&mul[py * ms]) : czero();
+                        cur[j] = ok ? col[(size_t)py * n] : czero();
+                    }
 #pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            line_dft<DET, +1>(v[c], t, sc, tws);
-            const int py = grp + F::NG * c - off;
-            if (py < 0 || py >= P) continue;
-            float2 *row = slab + (size_t)(sty + py) * n + stx;
-            float2 cur[F::N1];
-#pragma unroll
-            for (int k2 = 0; k2 < F::N2; ++k2)
-#pragma unroll
-                for (int j = 0; j < F::KPT; ++j) {
-                    const int px = t * F::KPT + j + F::N1 * k2 - off;
-                    cur[j * F::N2 + k2] = (px >= 0 && px < P) ? row[px] : czero();
+                    for (int j = 0; j < RB; ++j) {
+                        const int py = v1 + F::QA * (h + j) - off;
+                        if (FULL || (py >= 0 && py < P)) col[(size_t)py * n] = cur[j] + cmulc(pv[j], v[h + j]);
+                    }
                 }
-#pragma unroll
-            for (int k2 = 0; k2 < F::N2; ++k2)
-#pragma unroll
-                for (int j = 0; j < F::KPT; ++j) {
-                    const int px = t * F::KPT + j + F::N1 * k2 - off;
-                    if (px >= 0 && px < P)
-                        row[px] = cur[j * F::N2 + k2] + cmulc(__ldg(&pr[py * P + px]), v[c][j * F::N2 + k2]);
-                }
+            }
         }
-        __syncthreads();
+    }
+    if constexpr (PROBE) {
+        if (line) {
+#pragma unroll
+            for (int v2 = 0; v2 < 16; ++v2) {
+                const int py = v10 + F::QA * v2 - off0;
+                if (FULL || (py >= 0 && py < P)) slab[(size_t)py * P + px0] = acc[v2];
+            }
+        }
     }
 }
 
@@ -502,7 +586,7 @@ __global__ void __launch_bounds__(512, 1)
         const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
         float2 *out = g + (size_t)fid * 128 * 128;
         if (stx < 0 || sty < 0) {
-            for (int e = threadIdx.x; e < 128 * 128 / 2; e += 512) reinterpret_cast<float4 *>(out)[e] = make_float4(0, 0, 0, 0);
+            for (int e = threadIdx.x; e < 128 * 128; e += 512) out[e] = czero();
             continue;
         }
         const float2 *src = psi + ((size_t)th * nz + sty) * n + stx;
@@ -573,7 +657,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
 // The adjoints with two exchanges (see k_ptycho_fwd128).  Object adjoint:
 // grid (parts, ntheta), block (part, angle) owns slab dst[angle][part] and
 // walks that angle's scans part, part + parts, ...  PROBE (the adjoint with
-// respect to the probe, as k_ptycho_adj_probe): grid (blocks, 1), block b
+// respect to the probe): grid (blocks, 1), block b
 // walks frames b, b + gridDim.x, ... < nframes and accumulates
 // conj(psi patch) x frame into its P x P partial dst[b].  RESID forms the
 // Poisson / Gaussian residual of each frame value on load.  R3's thread adds
@@ -605,7 +689,8 @@ __global__ void __launch_bounds__(512, 1)
         // 4.95 ms; the object adjoint with the residual went 5.89 -> 5.99 ms
         // (Poisson), so it goes without.
         constexpr bool PREFETCH = RESID == 0 || PROBE;
-        if (PREFETCH && threadIdx.x < 8 && s + parts < count) {
+        const bool aligned = (((uintptr_t)g | (RESID != 0 ? (uintptr_t)data : 0)) & 15) == 0;
+        if (PREFETCH && aligned && threadIdx.x < 8 && s + parts < count) {
             const size_t nf = (size_t)fid + parts;
             prefetch_l2(g + (nf * 128 * 128 + threadIdx.x * 2048), 16384);
             if (RESID != 0 && threadIdx.x < 4) prefetch_l2(data + (nf * 128 * 128 + threadIdx.x * 4096), 16384);
@@ -709,92 +794,36 @@ __global__ void k_probe_t(const float2 *__restrict__ prb, float2 *__restrict__ p
 // G = scale x inverse DFT of conj(phase) g (the same transform as the object
 // adjoint).  Block b walks frames b, b + gridDim.x, ... and accumulates into
 // its own P x P partial part[b] (prbT layout); every (py, px) of the window
-// belongs to one thread, so no atomics; k_probe_reduce sums the partials in
-// block order.  RESID: the frames are the data-term residual of g (as
-// k_ptycho_adj).
-template <int DET, int RESID>
-__global__ void __launch_bounds__(PF<DET>::NT, 1)
-    k_ptycho_adj_probe(const float2 *__restrict__ g, float2 *__restrict__ part, const float2 *__restrict__ psi,
-                       const int *__restrict__ corner, const float2 *__restrict__ phase, int nz, int n, int nscan,
-                       int nframes, int P, float scale, const float2 *__restrict__ tw, const float *__restrict__ data,
-                       float dscale)
-{
-    using F = PF<DET>;
-    extern __shared__ float2 sm[];
-    float2 *fr = sm;
-    float2 *tws = sm + DET * F::P;
-    float2 *acc = part + (size_t)blockIdx.x * P * P;
-    for (int i = threadIdx.x; i < DET; i += F::NT) tws[i] = tw[i];
-    for (int e = threadIdx.x; e < P * P; e += F::NT) acc[e] = czero();
-    const int t = threadIdx.x % F::N2, grp = threadIdx.x / F::N2;
-    float2 *sc = fr + grp * (DET + 1);
-    const int off = (DET - P) / 2;
-    __syncthreads();
-    for (int fid = blockIdx.x; fid < nframes; fid += gridDim.x) {
-        const int th = fid / nscan;
-        const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
-        if (stx < 0 || sty < 0) continue;
-        const float2 ph = phase[fid];
-        const float2 *in = g + (size_t)fid * DET * DET;
-        float2 v[F::CPG][F::N1];
-#pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int kx = grp + F::NG * c;
-#pragma unroll
-            for (int m = 0; m < F::N1; ++m) {
-                const int e = kx * DET + t + F::N2 * m;
-                v[c][m] = scale * cmulc(ph, resid<RESID>(__ldg(&in[e]), data, (size_t)fid * DET * DET + e, dscale));
-            }
-            line_dft<DET, +1>(v[c], t, sc, tws);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int kx = grp + F::NG * c;
-#pragma unroll
-            for (int j = 0; j < F::KPT; ++j)
-#pragma unroll
-                for (int k2 = 0; k2 < F::N2; ++k2) {
-                    const int iy = t * F::KPT + j + F::N1 * k2;
-                    fr[iy * F::P + (kx ^ fswz<DET>(iy))] = v[c][j * F::N2 + k2];
-                }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            const int iy = grp + F::NG * c;
-            const int sw = fswz<DET>(iy);
-#pragma unroll
-            for (int m = 0; m < F::N1; ++m) v[c][m] = fr[iy * F::P + ((t + F::N2 * m) ^ sw)];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < F::CPG; ++c) {
-            line_dft<DET, +1>(v[c], t, sc, tws);
-            const int py = grp + F::NG * c - off;
-            if (py < 0 || py >= P) continue;
-            const float2 *orow = psi + ((size_t)th * nz + sty + py) * n + stx;
-            float2 *arow = acc + (size_t)py * P;
-#pragma unroll
-            for (int k2 = 0; k2 < F::N2; ++k2)
-#pragma unroll
-                for (int j = 0; j < F::KPT; ++j) {
-                    const int px = t * F::KPT + j + F::N1 * k2 - off;
-                    if (px >= 0 && px < P) arow[px] = arow[px] + cmulc(__ldg(&orow[px]), v[c][j * F::N2 + k2]);
-                }
-        }
-    }
-}
+// belongs to one thread, so no atomics; k_probe_reduce sums the partials in a
+// fixed order.  The kernels are the object adjoints in their PROBE mode.
 
-// gprb[px P + py] = c sum_b part[b][py P + px], blocks in order
-__global__ void k_probe_reduce(const float2 *__restrict__ part, float2 *__restrict__ gprb, int nblk, int P, float c)
+// gprb[px P + py] = c sum_b part[b][py P + px].  A block takes 32 elements; its
+// eight warps sum the partials b = warp, warp + 8, ..., then the eight sums are
+// added in warp order, in FP64: the order (one rank's partials or two ranks')
+// then shows in the last bit at most.
+__global__ void __launch_bounds__(256)
+    k_probe_reduce(const float2 *__restrict__ part, float2 *__restrict__ gprb, int nblk, int P, float c)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P * P) return;
-    float2 s = part[i];
-    for (int b = 1; b < nblk; ++b) s = s + part[(size_t)b * P * P + i];
+    __shared__ double2 sums[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    double2 s = make_double2(0.0, 0.0);
+    if (i < P * P)
+#pragma unroll 4
+        for (int b = warp; b < nblk; b += 8) {
+            const float2 v = part[(size_t)b * P * P + i];
+            s.x += v.x;
+            s.y += v.y;
+        }
+    sums[warp][lane] = s;
+    __syncthreads();
+    if (warp || i >= P * P) return;
+    for (int k = 1; k < 8; ++k) {
+        s.x += sums[k][lane].x;
+        s.y += sums[k][lane].y;
+    }
     const int py = i / P, px = i % P;
-    gprb[px * P + py] = c * s;
+    gprb[px * P + py] = make_float2((float)(c * s.x), (float)(c * s.y));
 }
 
 }  // namespace
@@ -895,43 +924,37 @@ int ptycho_attrs()
         PT_ATTR((k_ptycho_adj_small<DET, 0>), s);
         PT_ATTR((k_ptycho_adj_small<DET, 1>), s);
         PT_ATTR((k_ptycho_adj_small<DET, 2>), s);
-    } else {
-        const int s = (int)PF<DET>::SMEM;
-        PT_ATTR(k_ptycho_fwd<DET>, s);
-        PT_ATTR((k_ptycho_adj<DET, 0>), s);
-        PT_ATTR((k_ptycho_adj<DET, 1>), s);
-        PT_ATTR((k_ptycho_adj<DET, 2>), s);
-        PT_ATTR((k_ptycho_adj_probe<DET, 0>), s);
-        PT_ATTR((k_ptycho_adj_probe<DET, 1>), s);
-        PT_ATTR((k_ptycho_adj_probe<DET, 2>), s);
-        PT_ATTR((k_ptycho_fwd<DET, true>), s);
-        PT_ATTR((k_ptycho_adj<DET, 0, true>), s);
-        PT_ATTR((k_ptycho_adj<DET, 1, true>), s);
-        PT_ATTR((k_ptycho_adj<DET, 2, true>), s);
-        if constexpr (DET == 128) {
-            PT_ATTR((k_ptycho_fwd128<true>), P128_SMEM);
-            PT_ATTR((k_ptycho_fwd128<false>), P128_SMEM);
-            PT_ATTR((k_ptycho_fwd128<true, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_fwd128<false, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 0>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<false, 0>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 0, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<false, 0, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 1>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<false, 1>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 1, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<false, 1, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 2>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<false, 2>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 2, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<false, 2, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 0, false, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 1, false, true>), P128_SMEM);
-            PT_ATTR((k_ptycho_adj128<true, 2, false, true>), P128_SMEM);
-        }
+    } else if constexpr (DET == 128) {
+        PT_ATTR((k_ptycho_fwd128<true>), P128_SMEM);
+        PT_ATTR((k_ptycho_fwd128<false>), P128_SMEM);
+        PT_ATTR((k_ptycho_fwd128<true, true>), P128_SMEM);
+        PT_ATTR((k_ptycho_fwd128<false, true>), P128_SMEM);
+#define PT_ATTR_ADJ(RESID)                                                  \
+    PT_ATTR((k_ptycho_adj128<true, RESID>), P128_SMEM);                     \
+    PT_ATTR((k_ptycho_adj128<false, RESID>), P128_SMEM);                    \
+    PT_ATTR((k_ptycho_adj128<true, RESID, true>), P128_SMEM);               \
+    PT_ATTR((k_ptycho_adj128<false, RESID, true>), P128_SMEM);              \
+    PT_ATTR((k_ptycho_adj128<true, RESID, false, true>), P128_SMEM);        \
+    PT_ATTR((k_ptycho_adj128<false, RESID, false, true>), P128_SMEM);
+        PT_ATTR_ADJ(0)
+        PT_ATTR_ADJ(1)
+        PT_ATTR_ADJ(2)
+#undef PT_ATTR_ADJ
     }
 #undef PT_ATTR
     return PT_OK;
+}
+
+// go(FULL, SUB) for the handle: whether the probe fills the detector, and
+// whether each frame has its own shifted probe
+template <typename Go>
+void by_kind(const pt_ptycho *h, Go go)
+{
+    const bool full = h->P == h->det;
+    if (h->quant)
+        full ? go(std::true_type{}, std::true_type{}) : go(std::false_type{}, std::true_type{});
+    else
+        full ? go(std::true_type{}, std::false_type{}) : go(std::false_type{}, std::false_type{});
 }
 
 template <int DET, int RESID>
@@ -945,32 +968,22 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
         PT_LAUNCHED("k_ptycho_adj_small");
         return PT_OK;
     } else {
-        using F = PF<DET>;
         float2 *dst = h->parts > 1 ? h->partial : out;
         const dim3 grid(h->parts, h->ntheta);
-        // the det = 128 adjoint (k_ptycho_adj128) for 16-byte aligned frames
-        const bool fast128 = DET == 128 && ((uintptr_t)in % 16) == 0 && (RESID == 0 || (uintptr_t)data % 16 == 0);
         // SUB: the sub-pixel model's per-frame probe tables (a separate
         // instantiation, so the reference model's kernels are unchanged)
-        auto go = [&](auto sub) {
-            constexpr bool S = decltype(sub)::value;
-            if (fast128 && h->P == DET)
-                k_ptycho_adj128<true, RESID, S><<<grid, 512, P128_SMEM, st>>>(
-                    in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
-                    h->tw, data, dscale, h->shift_ids());
-            else if (fast128)
-                k_ptycho_adj128<false, RESID, S><<<grid, 512, P128_SMEM, st>>>(
+        auto go = [&](auto full, auto sub) {
+            constexpr bool FU = decltype(full)::value, S = decltype(sub)::value;
+            if constexpr (DET == 128)
+                k_ptycho_adj128<FU, RESID, S><<<grid, 512, P128_SMEM, st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, h->shift_ids());
             else
-                k_ptycho_adj<DET, RESID, S><<<grid, F::NT, F::SMEM, st>>>(
+                k_ptycho_adj<DET, FU, RESID, S><<<grid, FR<DET>::BLOCK, FR<DET>::SMEM, st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw,
                     data, dscale, h->shift_ids());
         };
-        if (h->quant)
-            go(std::true_type{});
-        else
-            go(std::false_type{});
+        by_kind(h, go);
         PT_LAUNCHED("k_ptycho_adj");
         if (h->parts > 1) {
             const size_t slab = (size_t)h->nz * h->n, total = slab * h->ntheta;
@@ -997,31 +1010,22 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
         k_ptycho_fwd_small<DET><<<dim3(h->nscan, h->ntheta), ptycho_block<DET>(), s, st>>>(
             in, out, h->corner, h->phase, h->prb, h->nz, h->n, h->nscan, h->P, h->c, scale, h->tw);
     } else {
-        using F = PF<DET>;
-        // the det = 128 kernel writes frames with 16-byte stores; one resident
-        // block per SM walks the frames (grid-stride), so the grid is one
-        // block per SM (1.2 % faster than a block per frame at 256^3)
-        const bool fast128 = DET == 128 && ((uintptr_t)out % 16) == 0;
-        const int grid128 = std::min(nframes, h->nsm);
-        auto go = [&](auto sub) {
-            constexpr bool S = decltype(sub)::value;
-            if (fast128 && h->P == DET)
-                k_ptycho_fwd128<true, S><<<grid128, 512, P128_SMEM, st>>>(
+        // the resident blocks walk the frames (grid-stride)
+        auto go = [&](auto full, auto sub) {
+            constexpr bool FU = decltype(full)::value, S = decltype(sub)::value;
+            if constexpr (DET == 128) {
+                k_ptycho_fwd128<FU, S><<<std::min(nframes, h->nsm), 512, P128_SMEM, st>>>(
                     in, out, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, nframes, h->P, scale,
                     h->tw128, h->tw, h->shift_ids());
-            else if (fast128)
-                k_ptycho_fwd128<false, S><<<grid128, 512, P128_SMEM, st>>>(
-                    in, out, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, nframes, h->P, scale,
-                    h->tw128, h->tw, h->shift_ids());
-            else
-                k_ptycho_fwd<DET, S><<<nframes, F::NT, F::SMEM, st>>>(in, out, h->corner, h->phase_tab(),
-                                                                     h->probe_tab(), h->nz, h->n, h->nscan, nframes,
-                                                                     h->P, scale, h->tw, h->shift_ids());
+            } else {
+                using F = FR<DET>;
+                const int grid = std::min((nframes + F::FPB - 1) / F::FPB, h->nsm * F::BPS);
+                k_ptycho_fwd<DET, FU, S><<<grid, F::BLOCK, F::SMEM, st>>>(in, out, h->corner, h->phase_tab(),
+                                                                         h->probe_tab(), h->nz, h->n, h->nscan,
+                                                                         nframes, h->P, scale, h->tw, h->shift_ids());
+            }
         };
-        if (h->quant)
-            go(std::true_type{});
-        else
-            go(std::false_type{});
+        by_kind(h, go);
     }
     PT_LAUNCHED("k_ptycho_fwd");
     return PT_OK;
@@ -1064,22 +1068,25 @@ int probe_adj_launch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 
         pt::set_error("ptychofft.adj_probe: not compiled for detector %d (16 to 128)", DET);
         return PT_ERR_UNSUPPORTED;
     } else {
-        using F = PF<DET>;
         const int nframes = h->ntheta * h->nscan;
-        // det 128 with a 128 probe: the two-exchange adjoint in its probe mode;
-        // smaller probes keep the generic kernel
-        const bool fast128 = DET == 128 && h->P == DET && ((uintptr_t)in % 16) == 0 &&
-                             (RESID == 0 || (uintptr_t)data % 16 == 0);
-        if (fast128)
-            k_ptycho_adj128<true, RESID, false, true><<<h->prb_blocks, 512, P128_SMEM, st>>>(
-                in, h->prb_part, h->corner, h->phase, h->prbT, h->nz, h->n, h->nscan, h->P, scale, h->tw128, h->tw,
-                data, dscale, nullptr, psi, nframes);
+        auto go = [&](auto full) {
+            constexpr bool FU = decltype(full)::value;
+            if constexpr (DET == 128)
+                k_ptycho_adj128<FU, RESID, false, true><<<h->prb_blocks, 512, P128_SMEM, st>>>(
+                    in, h->prb_part, h->corner, h->phase, h->prbT, h->nz, h->n, h->nscan, h->P, scale, h->tw128,
+                    h->tw, data, dscale, nullptr, psi, nframes);
+            else
+                k_ptycho_adj<DET, FU, RESID, false, true>
+                    <<<h->prb_blocks / FR<DET>::FPB, FR<DET>::BLOCK, FR<DET>::SMEM, st>>>(
+                        in, h->prb_part, h->corner, h->phase, h->prbT, h->nz, h->n, h->nscan, h->P, scale, h->tw, data,
+                        dscale, nullptr, psi, nframes);
+        };
+        if (h->P == DET)
+            go(std::true_type{});
         else
-            k_ptycho_adj_probe<DET, RESID><<<h->prb_blocks, F::NT, F::SMEM, st>>>(
-                in, h->prb_part, psi, h->corner, h->phase, h->nz, h->n, h->nscan, nframes, h->P, scale, h->tw, data,
-                dscale);
+            go(std::false_type{});
         PT_LAUNCHED("k_ptycho_adj_probe");
-        k_probe_reduce<<<(h->P * h->P + 255) / 256, 256, 0, st>>>(h->prb_part, gprb, h->prb_blocks, h->P, h->c);
+        k_probe_reduce<<<(h->P * h->P + 31) / 32, 256, 0, st>>>(h->prb_part, gprb, h->prb_blocks, h->P, h->c);
         PT_LAUNCHED("k_probe_reduce");
         return PT_OK;
     }
@@ -1098,6 +1105,51 @@ int probe_adj_dispatch(pt_ptycho *h, float2 *gprb, const float2 *in, const float
 #undef PT_CASE
     pt::set_error("ptychofft: detector size %d not compiled", h->det);
     return PT_ERR_UNSUPPORTED;
+}
+
+// Blocks of the probe adjoint that an SM holds, and the frames a block works on at a time.
+struct Residency {
+    int probe_blocks, frames;
+};
+Residency residency(int det)
+{
+    switch (det) {
+    case 16: return {FR<16>::BPSP, FR<16>::FPB};
+    case 32: return {FR<32>::BPSP, FR<32>::FPB};
+    case 64: return {FR<64>::BPSP, FR<64>::FPB};
+    default: return {1, 1};
+    }
+}
+
+// The adjoint's split of an angle's scans over blocks.  Det 128 (one block per
+// SM): waves x scans per block, with a 3 % charge per extra part for the slab
+// traffic.  Smaller detectors (several blocks per SM), in units of one frame's
+// time on a full SM: a block alone needs about LONE units per frame, so few
+// blocks are bound by their own chain of frames and many by the SM's share;
+// every part also clears, and the reduction reads, its slab (nz n values
+// against a frame's det^2).
+int choose_parts(const pt_ptycho &h, int nsm)
+{
+    constexpr double LONE = 3.0;
+    const Residency res = residency(h.det);
+    int best_p = 1;
+    double best = 1e300;
+    for (int p = 1; p <= std::min(h.nscan, 16); ++p) {
+        const double blocks = std::ceil((double)h.ntheta * p / nsm);             // per SM
+        const double chain = std::ceil((double)h.nscan / (p * res.frames)) * res.frames;   // frames per block
+        double cost;
+        if (h.det == 128) {
+            cost = blocks * chain * (1.0 + 0.03 * (p - 1));
+        } else {
+            const double slab = (double)h.nz * h.n / ((double)h.det * h.det);
+            cost = std::max(chain * LONE, blocks * chain) + (p > 1 ? blocks * slab : 0.0);
+        }
+        if (cost < best - 1e-9) {
+            best = cost;
+            best_p = p;
+        }
+    }
+    return best_p;
 }
 
 void ptycho_free(pt_ptycho *h)
@@ -1261,27 +1313,16 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
         pt::set_error("ptychofft: no CUDA device");
         return PT_ERR_CUDA;
     }
-    // adjoint split: enough (part, angle) blocks to fill the GPU twice
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
     h->nsm = nsm;
-    // waves x scans-per-block, with a 3% charge per extra part for the slab traffic;
     // PT_PTYCHO_ADJ_PARTS=<k> overrides the choice (tuning)
     h->parts = 1;
     const char *env_parts = getenv("PT_PTYCHO_ADJ_PARTS");
-    if (env_parts && atoi(env_parts) >= 1) {
+    if (env_parts && atoi(env_parts) >= 1)
         h->parts = std::min<int>(atoi(env_parts), (int)nscan);
-    } else if (detx >= 16) {
-        double best = 1e300;
-        for (int p = 1; p <= (int)std::min<size_t>(nscan, 16); ++p) {
-            const double waves = std::ceil((double)ntheta * p / nsm);
-            const double cost = waves * std::ceil((double)nscan / p) * (1.0 + 0.03 * (p - 1));
-            if (cost < best - 1e-9) {
-                best = cost;
-                h->parts = p;
-            }
-        }
-    }
+    else if (detx >= 16)
+        h->parts = choose_parts(*h, nsm);
     bool ok = cudaMalloc((void **)&h->tw, detx * sizeof(float2)) == cudaSuccess &&
               cudaMalloc((void **)&h->tw128, 64 * sizeof(float4)) == cudaSuccess &&
               cudaMalloc((void **)&h->prb, nprb * nprb * sizeof(float2)) == cudaSuccess &&
@@ -1292,8 +1333,10 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
               cudaMalloc((void **)&h->corner, 2 * ntheta * nscan * sizeof(int)) == cudaSuccess &&
               cudaMalloc((void **)&h->frac, 2 * ntheta * nscan * sizeof(float)) == cudaSuccess &&
               cudaMalloc((void **)&h->prbT2, nprb * nprb * sizeof(float2)) == cudaSuccess;
-    // probe adjoint: one block per SM (two below 64x64 detectors), one partial each
-    h->prb_blocks = (int)std::min<size_t>((size_t)nsm * (detx >= 64 ? 1 : 2), ntheta * nscan);
+    // probe adjoint: one partial per frame in flight
+    const Residency res = residency((int)detx);
+    const size_t inflight = (size_t)nsm * res.probe_blocks;
+    h->prb_blocks = (int)(std::min(inflight, (ntheta * nscan + res.frames - 1) / res.frames) * res.frames);
     ok = ok && cudaMalloc((void **)&h->prb_part, (size_t)h->prb_blocks * nprb * nprb * sizeof(float2)) == cudaSuccess;
     if (!ok) {
         ptycho_free(h);
