@@ -13,11 +13,9 @@
 //    accumulates conj(probe) x frame into its own slab; with parts > 1 the
 //    slabs are summed in a fixed order by a second kernel.  Deterministic,
 //    no atomics.
-//  Detector 128x128 (k_ptycho_fwd128, k_ptycho_adj128) splits the 2-D
-//    transform 16 x 8 by 4 x 32 instead, so a frame passes through shared
-//    memory twice rather than three times, with coalesced 256-byte warp
-//    accesses on both sides; one 512-thread block per SM.  The adjoint also
-//    serves the residual-on-load and probe adjoints.
+//  Detector 128x128 has its own kernels (k_ptycho_fwd128, k_ptycho_adj128): 32
+//    values per thread, one 512-thread block per SM.
+//  The adjoints also serve the residual-on-load and probe adjoints.
 //  Detector 8x8 uses a plain shared-memory Stockham path.
 #include <algorithm>
 #include <cmath>
@@ -458,9 +456,35 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
 }
 
 // ---- det = 128 ---------------------------------------------------------
-// shared memory: the 128 KB exchange buffer alone.  The remaining ~100 KB of
-// L1 keeps most of the 128 KB probe table, reread for every frame, resident.
-constexpr int P128_SMEM = 128 * 128 * 8;
+// The same three rounds for a 128 x 128 frame, 32 values per thread and one
+// 512-thread block per SM (the frame's exchange buffer takes 128 KB):
+//   R1  thread (q = 32 g + lane, rt = w + 4 c, c = 0, 1): 16-point DFTs over m
+//       of r = rt + 8 m, times w128^(rt k1)
+//   R2  thread (k1 = warp, qb = lane): 8-point DFT over rt, u = k1 + 16 k2;
+//       4-point DFT over qa of q = qb + 32 qa, v1; times w128^(qb v1) f
+//   R3  thread (u = tid & 127, v1 = g): 32-point DFT over qb, v = v1 + 4 v2
+// with g = tid >> 7 the thread's group of four warps and w its warp there.
+// R1's lanes load 32 consecutive q (256 B of one row) and R3's lanes hold 32
+// consecutive u, so every global access of a warp covers 256 bytes.
+//
+// The exchange rows (k1, j) hold 32 values qb (256 B, 16-byte slots XORed with
+// k1 & 7), j = qa 8 + rt after R1 and v1 8 + k2 after R2, which works in place.
+// Group g writes the rows qa = g in R1 and reads the rows v1 = g in R3: the
+// same memory.  So a frame has two block-wide barriers, around R2; from R3 to
+// the next frame's R1 a group waits for its own four warps only, and one
+// group's loads and stores run under another's arithmetic.
+//
+// The probe table (128 KB) does not stay in the 100 KB of L1 that the exchange
+// buffer leaves: rereading it cyclically hit 10 % (forward).  Its first 96 KB
+// sit in shared memory instead, the rest is read through L2.
+// 256^3, 384 angles x 169 scans: forward 3.75 -> 3.42 ms (a table of 64 KB:
+// 3.47; without the early patch loads 3.59), adjoint 4.26 -> 3.70 ms.  The
+// adjoint keeps 32 KB only: with 96 KB in the table the L1 left for loads in
+// flight is too small (4.00 ms; 16 KB 3.83, 48 KB 3.75).  The arithmetic and
+// the exchange alone take 2.1 ms of the forward, the exchange 1.1 ms.
+constexpr int P128_EX = 128 * 128 * 8;          // exchange buffer
+constexpr int P128_FTAB = 96 * 1024, P128_ATAB = 32 * 1024;   // probe rows kept in shared memory: forward, adjoint
+constexpr int P128_FSMEM = P128_EX + P128_FTAB, P128_ASMEM = P128_EX + P128_ATAB;
 
 // The det-128 twiddles a thread needs, w(t k1) for k1 = 0..15, in pairs:
 // entry q * 8 + t of the 64-entry float4 table holds w(2q t) and w((2q+1) t)
@@ -477,163 +501,77 @@ __device__ __forceinline__ void twiddle16(float2 (&v)[16], float4 w, int q)
     v[2 * q + 1] = cmul(v[2 * q + 1], w1);
 }
 
-// ---- det-128 frames with two shared-memory exchanges --------------------
-// B[u][v] = f sum_{r,q} A[r][q] w128^(DIR (u r + v q)) for a 128 x 128 array
-// A whose q runs along memory, in three register rounds:
-//   R1  thread (q = tid & 127, rt = (tid >> 7) + 4 c, c = 0, 1): 16-point
-//       DFTs over m of r = rt + 8 m, times w128^(rt k1)   -> (k1, q, rt)
-//   R2  thread (k1 = warp, qb = lane): the 8-point DFT over rt gives
-//       u = k1 + 16 k2; the 4-point DFT over qa of q = qb + 32 qa gives v1;
-//       times w128^(qb v1) and the frame factor f        -> (v1, u, qb)
-//   R3  thread (u = tid & 127, v1 = tid >> 7): the 32-point DFT over qb
-//       gives v = v1 + 4 v2.
-// R1's lanes load 32 consecutive q (256 B of one row) and R3's lanes hold 32
-// consecutive u.  The forward takes A = probe x patch [y][x] and stores
-// frame[kx = v][ky = u]; the adjoint takes A = frame[kx][ky] and adds
-// pixel [y = v][x = u] into the slab, so both touch 256 consecutive bytes per
-// warp access.  Between the rounds the frame goes once through the 128 KB
-// buffer ex, as E1[k1][qa][rt][qb] and E2[v1][u][qb]; E2's rows of 32 values
-// (256 B) have their 16-byte slots permuted by an XOR with u & 7, so that
-// every exchange access of a warp takes the minimum number of shared
-// wavefronts (two for 8-byte, four for 16-byte accesses).
-__device__ __forceinline__ int e1_at(int k1, int qa, int rt, int qb) { return ((k1 * 4 + qa) * 8 + rt) * 32 + qb; }
-__device__ __forceinline__ int e2_at(int v1, int u, int qb)
+// R1 of one line: v[m] = A[rt + 8 m][q].  tw4 is twiddle16's pair table; rt is
+// the same across a warp, so its loads are broadcasts.
+template <int DIR, bool PK>
+__device__ __forceinline__ void f128_r1(float2 (&v)[16], float2 *ex, int q, int rt, const float4 *__restrict__ tw4)
 {
-    return (v1 * 128 + u) * 32 + 2 * ((qb >> 1) ^ (u & 7)) + (qb & 1);
+    ptfft::Dft<16, DIR, PK>::run(v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) twiddle16<DIR>(v, __ldg(&tw4[k * 8 + rt]), k);
+    const unsigned o = ((unsigned)((q >> 5) * 8 + rt) << 8) + ((unsigned)(q & 31) << 3);
+#pragma unroll
+    for (int k1 = 0; k1 < 16; ++k1) *fr_ptr(ex, (o ^ ((k1 & 7) << 4)) + k1 * 8192) = v[k1];
 }
 
-// R1 of one frame: v[c][m] holds A[rt + 8 m][q], rt = (tid >> 7) + 4 c;
-// transformed and written to E1.  The caller synchronises before and after.
-// tw4 is twiddle16's pair table; rt is the same across a warp, so its
-// loads are broadcasts.
-template <int DIR>
-__device__ __forceinline__ void frame_r1(float2 (&v)[2][16], float2 *ex, const float4 *__restrict__ tw4)
+// R2 in place for thread (k1 = warp, qb = lane).  The twiddles w128^(qb j)
+// (j = 1..3, in direction DIR; w128[m] = exp(-2 pi i m / 128)) are multiplied
+// by the frame factor f: the factor rides on them.
+template <int DIR, bool PK>
+__device__ __forceinline__ void f128_r2(float2 *ex, int t, float2 f, const float2 *__restrict__ w128)
 {
-    const int q = threadIdx.x & 127;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int rt = (threadIdx.x >> 7) + 4 * c;
-        ptfft::Dft<16, DIR>::run(v[c]);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) twiddle16<DIR>(v[c], __ldg(&tw4[k * 8 + rt]), k);
-#pragma unroll
-        for (int k1 = 0; k1 < 16; ++k1) ex[e1_at(k1, q >> 5, rt, q & 31)] = v[c][k1];
-    }
-}
-
-// R2 of one frame for thread (k1 = warp, qb = lane): reads E1, synchronises
-// (E1 fully read), transforms, and writes E2.  The twiddles w128^(qb j)
-// (j = 1..3, in direction DIR; w128[m] = exp(-2 pi i m / 128)) times the
-// frame factor f, and f itself for j = 0: the factor rides on the twiddles.
-template <int DIR>
-__device__ __forceinline__ void frame_r2(float2 *ex, float2 f, const float2 *__restrict__ w128)
-{
-    const int k1 = threadIdx.x >> 5, qb = threadIdx.x & 31;
+    const int k1 = t >> 5, qb = t & 31;
     float2 rw1 = __ldg(&w128[qb]), rw2 = __ldg(&w128[2 * qb]), rw3 = __ldg(&w128[3 * qb]);
     if (DIR > 0) {
         rw1.y = -rw1.y;
         rw2.y = -rw2.y;
         rw3.y = -rw3.y;
     }
+    float2 *s = fr_ptr(ex, (((unsigned)qb << 3) ^ ((k1 & 7) << 4)) + k1 * 8192);
     float2 a[4][8];
 #pragma unroll
     for (int qa = 0; qa < 4; ++qa)
 #pragma unroll
-        for (int rt = 0; rt < 8; ++rt) a[qa][rt] = ex[e1_at(k1, qa, rt, qb)];
-    __syncthreads();
+        for (int rt = 0; rt < 8; ++rt) a[qa][rt] = s[(qa * 8 + rt) * 32];
 #pragma unroll
-    for (int qa = 0; qa < 4; ++qa) ptfft::Dft<8, DIR>::run(a[qa]);
+    for (int qa = 0; qa < 4; ++qa) ptfft::Dft<8, DIR, PK>::run(a[qa]);
     const float2 r1 = cmul(rw1, f), r2 = cmul(rw2, f), r3 = cmul(rw3, f);
 #pragma unroll
     for (int k2 = 0; k2 < 8; ++k2) {
-        ptfft::dft4<DIR>(a[0][k2], a[1][k2], a[2][k2], a[3][k2]);
-        const int u = k1 + 16 * k2;
-        ex[e2_at(0, u, qb)] = cmul(a[0][k2], f);
-        ex[e2_at(1, u, qb)] = cmul(a[1][k2], r1);
-        ex[e2_at(2, u, qb)] = cmul(a[2][k2], r2);
-        ex[e2_at(3, u, qb)] = cmul(a[3][k2], r3);
+        ptfft::dft4<DIR, PK>(a[0][k2], a[1][k2], a[2][k2], a[3][k2]);
+        s[k2 * 32] = cmul(a[0][k2], f);
+        s[(8 + k2) * 32] = cmul(a[1][k2], r1);
+        s[(16 + k2) * 32] = cmul(a[2][k2], r2);
+        s[(24 + k2) * 32] = cmul(a[3][k2], r3);
     }
 }
 
-// R3's read of E2 for thread (u = tid & 127, v1 = tid >> 7): w[qb], qb = 0..31.
-__device__ __forceinline__ void frame_r3_read(float2 (&w)[32], const float2 *ex)
+// R3's read of row (u, v1): w[qb], qb = 0..31.
+__device__ __forceinline__ void f128_r3_read(float2 (&w)[32], const float2 *ex, int u, int v1)
 {
-    const int u = threadIdx.x & 127, v1 = threadIdx.x >> 7;
-    const float4 *e4 = reinterpret_cast<const float4 *>(ex) + (v1 * 128 + u) * 16;
+    const int k1 = u & 15;
+    const unsigned o = ((unsigned)(k1 * 32 + v1 * 8 + (u >> 4)) << 8) + ((k1 & 7) << 4);
 #pragma unroll
     for (int s = 0; s < 16; ++s) {
-        const float4 q = e4[s ^ (u & 7)];
+        const float4 q = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(ex) + (o ^ (s << 4)));
         w[2 * s] = make_float2(q.x, q.y);
         w[2 * s + 1] = make_float2(q.z, q.w);
     }
 }
 
-// The forward with two exchanges (see above); grid-stride over frames, one
-// resident block per SM.  w128[m] = exp(-2 pi i m / 128).
-template <bool FULL, bool SUB = false>
-__global__ void __launch_bounds__(512, 1)
-    k_ptycho_fwd128(const float2 *__restrict__ psi, float2 *__restrict__ g, const int *__restrict__ corner,
-                    const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan,
-                    int nframes, int P, float scale, const float4 *__restrict__ tw4,
-                    const float2 *__restrict__ w128, const int *__restrict__ sid = nullptr)
+// barrier of group g's 128 threads (named barriers 1..4; 0 is __syncthreads)
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
+
+// Copies the first probe rows into shared memory; the caller synchronises.
+__device__ __forceinline__ void f128_probe_rows(float2 *tab, const float2 *__restrict__ prbT, int rows, int P)
 {
-    extern __shared__ float4 sm4[];
-    float2 *ex = reinterpret_cast<float2 *>(sm4);
-    const int q = threadIdx.x & 127, r0 = threadIdx.x >> 7;  // R1: x = q, y = r0 + 4 c + 8 m; R3: ky = q
-    const int off = FULL ? 0 : (128 - P) / 2;
-    for (int fid = blockIdx.x; fid < nframes; fid += gridDim.x) {
-        const int th = fid / nscan;
-        const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
-        float2 *out = g + (size_t)fid * 128 * 128;
-        if (stx < 0 || sty < 0) {
-            for (int e = threadIdx.x; e < 128 * 128; e += 512) out[e] = czero();
-            continue;
-        }
-        const float2 *src = psi + ((size_t)th * nz + sty) * n + stx;
-        const float2 *pr = SUB ? prbT + (size_t)sid[fid] * P * P : prbT;  // sub-pixel: the frame's shifted probe
-        // an opaque per-frame copy of the probe pointer and window offset: the
-        // 32 probe addresses and window tests are formed here, not hoisted out
-        // of the frame loop into registers
-        int offf = off;
-        asm volatile("mov.b64 %0, %0;" : "+l"(pr));
-        asm volatile("mov.b32 %0, %0;" : "+r"(offf));
-        const int PS = FULL ? 128 : P;  // a constant row stride: the probe rows are immediate offsets
-        {
-            float2 v[2][16];
-            const int px = q - offf;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-#pragma unroll
-                for (int m = 0; m < 16; ++m) {
-                    const int py = r0 + 4 * c + 8 * m - offf;
-                    if (FULL) {
-                        v[c][m] = cmul(__ldg(&pr[py * PS + px]), __ldg(&src[(size_t)py * n + px]));
-                    } else {
-                        float2 val = czero();
-                        if (py >= 0 && py < P && px >= 0 && px < P)
-                            val = cmul(__ldg(&pr[py * PS + px]), __ldg(&src[(size_t)py * n + px]));
-                        v[c][m] = val;
-                    }
-                }
-            }
-            frame_r1<-1>(v, ex, tw4);
-        }
-        __syncthreads();
-        frame_r2<-1>(ex, scale * phase[fid], w128);
-        __syncthreads();
-        float2 w[32];
-        frame_r3_read(w, ex);
-        __syncthreads();  // E2 fully read: the next frame's R1 may write
-        ptfft::Dft<32, -1>::run(w);
-#pragma unroll
-        for (int v2 = 0; v2 < 32; ++v2) __stcs(&out[(r0 + 4 * v2) * 128 + q], w[v2]);  // frame[kx = r0 + 4 v2][ky = q]
-    }
+    for (int e = threadIdx.x; e < rows * P; e += 512) tab[e] = __ldg(&prbT[e]);
 }
 
-// Loads of data read once (frames, counts) that do not allocate in L1, so
-// that the probe table, reread for every frame, keeps its L1 lines (at
-// 256^3 / 384 angles: plain adjoint 4.39 -> 4.24 ms, Poisson residual 5.85
-// -> 5.52 ms, Gaussian 6.32 -> 5.99 ms).
+// Loads of data read once (frames, counts, patches) that do not allocate in
+// L1, so that what is reread keeps its L1 lines (at 256^3 / 384 angles: plain
+// adjoint 4.39 -> 4.24 ms, Poisson residual 5.85 -> 5.52 ms, Gaussian 6.32 ->
+// 5.99 ms, before the probe rows moved to shared memory).
 __device__ __forceinline__ float2 ld_once(const float2 *p)
 {
     float2 r;
@@ -654,16 +592,113 @@ __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// The adjoints with two exchanges (see k_ptycho_fwd128).  Object adjoint:
-// grid (parts, ntheta), block (part, angle) owns slab dst[angle][part] and
-// walks that angle's scans part, part + parts, ...  PROBE (the adjoint with
-// respect to the probe): grid (blocks, 1), block b
-// walks frames b, b + gridDim.x, ... < nframes and accumulates
-// conj(psi patch) x frame into its P x P partial dst[b].  RESID forms the
-// Poisson / Gaussian residual of each frame value on load.  R3's thread adds
-// pixel column x = u, rows y = v1 + 4 v2, so the 32 lanes of a warp touch
-// 256 consecutive bytes of one slab (or partial) row whatever the frame's
-// column parity.  w128[m] = exp(-2 pi i m / 128).
+// Forward, grid-stride over frames, one resident block per SM.  The first half
+// of the next frame's patch values (line c = 0) is requested before R3's
+// arithmetic and stores, so its latency runs under them.
+template <bool FULL, bool SUB = false>
+__global__ void __launch_bounds__(512, 1)
+    k_ptycho_fwd128(const float2 *__restrict__ psi, float2 *__restrict__ g, const int *__restrict__ corner,
+                    const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan,
+                    int nframes, int P, float scale, const float4 *__restrict__ tw4,
+                    const float2 *__restrict__ w128, const int *__restrict__ sid = nullptr)
+{
+    extern __shared__ float4 sm4[];
+    float2 *ex = reinterpret_cast<float2 *>(sm4);
+    float2 *tab = ex + 128 * 128;
+    const int grp = threadIdx.x >> 7, q0 = threadIdx.x >> 7 << 5 | (threadIdx.x & 31), rt0 = (threadIdx.x >> 5) & 3;
+    const int PS = FULL ? 128 : P;  // a constant row stride: the probe rows are immediate offsets
+    const int off0 = FULL ? 0 : (128 - P) / 2;
+    const int rows = SUB ? 0 : FULL ? P128_FTAB / 1024 : min(P, P128_FTAB / (P * (int)sizeof(float2)));
+    f128_probe_rows(tab, prbT, rows, P);
+    __syncthreads();
+    // patch value (row rt + 8 m, column q) of frame f; 0 outside the window
+    auto patch = [&](const float2 *src, int px, int py, int off) {
+        return FULL || (px >= 0 && px < P && py >= 0 && py < P) ? ld_once(&src[(ptrdiff_t)py * n]) : czero();
+    };
+    auto source = [&](int fid, int sx, int sy, int px) {
+        return psi + ((size_t)(fid / nscan) * nz + sy) * n + sx + px;
+    };
+    int fid = blockIdx.x;
+    int stx = corner[2 * fid], sty = corner[2 * fid + 1];
+    float2 pre[16];
+    {
+        const bool ok = stx >= 0 && sty >= 0;
+        const int px = q0 - off0;
+        const float2 *src = source(fid, max(stx, 0), max(sty, 0), px);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) pre[m] = ok ? patch(src, px, rt0 + 8 * m - off0, off0) : czero();
+    }
+    while (true) {
+        const int nxt = fid + gridDim.x;
+        const bool more = nxt < nframes;
+        const int nsx = more ? corner[2 * nxt] : -1, nsy = more ? corner[2 * nxt + 1] : -1;
+        const bool act = stx >= 0 && sty >= 0, nact = nsx >= 0 && nsy >= 0;
+        const int q = fresh(q0), rt = fresh(rt0), off = FULL ? 0 : fresh(off0), px = q - off;
+        float2 *out = g + (size_t)fid * 128 * 128;
+        float2 w[32];
+        if (act) {
+            const float2 *src = source(fid, stx, sty, px);
+            const float2 *pr = (SUB ? prbT + (size_t)sid[fid] * P * P : prbT) + px;  // sub-pixel: the frame's shifted probe
+            const float2 *ps = tab + px;
+            auto probe = [&](int m, int py) {
+                if (!FULL && !(px >= 0 && px < P && py >= 0 && py < P)) return czero();
+                if (!SUB && (FULL ? m < P128_FTAB / 8192 : py < rows)) return ps[py * PS];
+                return __ldg(&pr[py * PS]);
+            };
+            float2 v[16];
+#pragma unroll
+            for (int m = 0; m < 16; ++m) v[m] = patch(src, px, rt + 4 + 8 * m - off, off);
+#pragma unroll
+            for (int m = 0; m < 16; ++m) pre[m] = cmul(probe(m, rt + 8 * m - off), pre[m]);
+            f128_r1<-1, false>(pre, ex, q, rt, tw4);
+#pragma unroll
+            for (int m = 0; m < 16; ++m) v[m] = cmul(probe(m, rt + 4 + 8 * m - off), v[m]);
+            f128_r1<-1, false>(v, ex, q, rt + 4, tw4);
+            __syncthreads();
+            f128_r2<-1, false>(ex, fresh(threadIdx.x), scale * phase[fid], w128);
+            __syncthreads();
+            f128_r3_read(w, ex, fresh(threadIdx.x & 127), grp);
+            group_sync(grp);  // the group's rows are read: its next R1 may write
+        }
+        {
+            const float2 *src = source(more ? nxt : fid, max(nsx, 0), max(nsy, 0), px);
+#pragma unroll
+            for (int m = 0; m < 16; ++m) pre[m] = nact ? patch(src, px, rt + 8 * m - off, off) : czero();
+        }
+        float2 *o = out + grp * 128 + fresh(threadIdx.x & 127);   // frame[kx = grp + 4 v2][ky = u]
+        if (act) {
+            ptfft::Dft<32, -1, false>::run(w);
+#pragma unroll
+            for (int v2 = 0; v2 < 32; ++v2) __stcs(&o[4 * v2 * 128], w[v2]);
+        } else {   // skipped scan: the reference leaves a zero frame
+#pragma unroll
+            for (int v2 = 0; v2 < 32; ++v2) __stcs(&o[4 * v2 * 128], czero());
+        }
+        if (!more) break;
+        fid = nxt;
+        stx = nsx;
+        sty = nsy;
+    }
+}
+
+// *p += v in L2, without waiting for the sum (one FP32 addition per component,
+// as a load, an add and a store round it).  Each frame adds to a pixel at most
+// once and the frames of a block are separated by its barriers, so the order of
+// the sums, and the result, is that of the frames.
+__device__ __forceinline__ void add_l2(float2 *p, float2 v)
+{
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
+}
+
+// The adjoints (see k_ptycho_fwd128).  Object adjoint: grid (parts, ntheta),
+// block (part, angle) owns slab dst[angle][part] and walks that angle's scans
+// part, part + parts, ...  PROBE (the adjoint with respect to the probe): grid
+// (blocks, 1), block b walks frames b, b + gridDim.x, ... < nframes and
+// accumulates conj(psi patch) x frame into its P x P partial dst[b].  RESID
+// forms the Poisson / Gaussian residual of each frame value on load.  R3's
+// thread adds pixel column x = u, rows y = v1 + 4 v2, so the 32 lanes of a
+// warp touch 256 consecutive bytes of one slab (or partial) row whatever the
+// frame's column parity.  w128[m] = exp(-2 pi i m / 128).
 template <bool FULL, int RESID, bool SUB = false, bool PROBE = false>
 __global__ void __launch_bounds__(512, 1)
     k_ptycho_adj128(const float2 *__restrict__ g, float2 *dst, const int *__restrict__ corner,
@@ -674,20 +709,24 @@ __global__ void __launch_bounds__(512, 1)
 {
     extern __shared__ float4 sm4[];
     float2 *ex = reinterpret_cast<float2 *>(sm4);
+    float2 *tab = ex + 128 * 128;
     const int part = blockIdx.x, parts = gridDim.x, th0 = blockIdx.y;
     float2 *slab = PROBE ? dst + (size_t)part * P * P : dst + ((size_t)th0 * parts + part) * nz * n;
     for (int e = threadIdx.x; e < (PROBE ? P * P : nz * n); e += 512) slab[e] = czero();
-    const int q = threadIdx.x & 127, r0 = threadIdx.x >> 7;  // R1: ky = q, kx = r0 + 4 c + 8 m; R3: x = q
-    const int off = FULL ? 0 : (128 - P) / 2;
+    const int grp = threadIdx.x >> 7, q0 = threadIdx.x >> 7 << 5 | (threadIdx.x & 31), rt0 = (threadIdx.x >> 5) & 3;
+    const int off0 = FULL ? 0 : (128 - P) / 2;
+    constexpr bool TAB = !SUB && !PROBE;
+    const int rows = !TAB ? 0 : FULL ? P128_ATAB / 1024 : min(P, P128_ATAB / (P * (int)sizeof(float2)));
+    f128_probe_rows(tab, prbT, rows, P);
+    __syncthreads();
     const int count = PROBE ? nframes : nscan;
     for (int s = part; s < count; s += parts) {
         const int fid = PROBE ? s : th0 * nscan + s;
         const int th = PROBE ? fid / nscan : th0;
         // the block's next frame (and its counts) into L2 one frame ahead, in
-        // 16 KB pieces: its loads then wait on L2 rather than on HBM.  At
-        // 256^3 / 384 angles: plain 4.64 -> 4.42 ms, probe adjoint 5.04 ->
-        // 4.95 ms; the object adjoint with the residual went 5.89 -> 5.99 ms
-        // (Poisson), so it goes without.
+        // 16 KB pieces: its loads then wait on L2 rather than on HBM
+        // (plain adjoint 4.64 -> 4.42 ms with the earlier kernel).  Not with the
+        // residual: 45 angles of 100 to 400 scans, Poisson 0.90 -> 1.00 ms.
         constexpr bool PREFETCH = RESID == 0 || PROBE;
         const bool aligned = (((uintptr_t)g | (RESID != 0 ? (uintptr_t)data : 0)) & 15) == 0;
         if (PREFETCH && aligned && threadIdx.x < 8 && s + parts < count) {
@@ -698,8 +737,9 @@ __global__ void __launch_bounds__(512, 1)
         const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
         if (stx < 0 || sty < 0) continue;
         {
-            const float2 *in = g + (size_t)fid * 128 * 128;
-            const float *din = RESID ? data + (size_t)fid * 128 * 128 : nullptr;
+            const int q = fresh(q0), rt = fresh(rt0);
+            const float2 *in = g + (size_t)fid * 128 * 128 + rt * 128 + q;
+            const float *din = RESID ? data + (size_t)fid * 128 * 128 + rt * 128 + q : nullptr;
             // all 32 frame values (and counts) are loaded before the first
             // residual: its branches would otherwise hold each later load back
             float2 v[2][16];
@@ -708,57 +748,53 @@ __global__ void __launch_bounds__(512, 1)
             for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int m = 0; m < 16; ++m) {
-                    const int e = (r0 + 4 * c + 8 * m) * 128 + q;
-                    v[c][m] = ld_once(&in[e]);
-                    if constexpr (RESID != 0) d[c][m] = ld_once(&din[e]);
+                    v[c][m] = ld_once(&in[(4 * c + 8 * m) * 128]);
+                    if constexpr (RESID != 0) d[c][m] = ld_once(&din[(4 * c + 8 * m) * 128]);
                 }
-            if constexpr (RESID != 0) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
+            for (int c = 0; c < 2; ++c) {
+                if constexpr (RESID != 0) {
 #pragma unroll
                     for (int m = 0; m < 16; ++m) v[c][m] = resid_of<RESID>(v[c][m], d[c][m] * dscale);
+                }
+                f128_r1<+1, true>(v[c], ex, q, rt + 4 * c, tw4);
             }
-            frame_r1<+1>(v, ex, tw4);
         }
         __syncthreads();
         const float2 ph = phase[fid];
-        frame_r2<+1>(ex, make_float2(scale * ph.x, -scale * ph.y), w128);
+        f128_r2<+1, true>(ex, fresh(threadIdx.x), make_float2(scale * ph.x, -scale * ph.y), w128);
         __syncthreads();
         float2 w[32];
-        frame_r3_read(w, ex);
-        __syncthreads();  // E2 fully read: the next frame's R1 may write
-        ptfft::Dft<32, +1>::run(w);
+        const int u = fresh(threadIdx.x & 127), off = FULL ? 0 : fresh(off0);
+        f128_r3_read(w, ex, u, grp);
+        group_sync(grp);  // the group's rows are read: its next R1 may write
+        ptfft::Dft<32, +1, true>::run(w);
         // object: slab += conj(probe) x value; probe: partial += conj(psi) x value
-        const float2 *mul = PROBE ? psi + ((size_t)th * nz + sty) * n + stx
-                                  : (SUB ? prbT + (size_t)sid[fid] * P * P : prbT);  // sub-pixel: the frame's shifted probe
-        // an opaque per-frame copy of the multiplier pointer: the 32 row
-        // addresses are formed here, not hoisted out of the frame loop into
-        // registers; likewise the row window's offset and its 32 tests
-        int offf = off;
-        asm volatile("mov.b64 %0, %0;" : "+l"(mul));
-        asm volatile("mov.b32 %0, %0;" : "+r"(offf));
-        const int px = q - offf;
+        const int px = u - off;
         if (!FULL && (px < 0 || px >= P)) continue;
-        float2 *col = PROBE ? slab + px : slab + (size_t)sty * n + stx + px;
-        const size_t cs = PROBE ? P : n;                // row stride of col
+        const float2 *mul = (PROBE ? psi + ((size_t)th * nz + sty) * n + stx
+                                   : (SUB ? prbT + (size_t)sid[fid] * P * P : prbT)) + px;
         const int ms = PROBE ? n : (FULL ? 128 : P);  // row stride of mul (a constant for the probe table)
-        // RB rows at a time: their multiplier and slab loads are issued
-        // before the first store
+        float2 *col = PROBE ? slab + px : slab + (size_t)sty * n + stx + px;
+        const size_t cs = PROBE ? P : n;              // row stride of col
+        // RB rows at a time: their multiplier loads are issued before the first add
         constexpr int RB = 8;
 #pragma unroll
         for (int h = 0; h < 32; h += RB) {
-            float2 cur[RB], pv[RB];
+            float2 pv[RB];
 #pragma unroll
             for (int j = 0; j < RB; ++j) {
-                const int py = r0 + 4 * (h + j) - offf;
+                const int py = grp + 4 * (h + j) - off;
                 const bool ok = FULL || (py >= 0 && py < P);
-                pv[j] = ok ? mul[(size_t)py * ms + px] : czero();
-                cur[j] = ok ? col[py * cs] : czero();
+                if (TAB && (FULL ? h + j < P128_ATAB / 4096 : py < rows))
+                    pv[j] = ok ? tab[py * ms + px] : czero();
+                else
+                    pv[j] = ok ? mul[(size_t)py * ms] : czero();
             }
 #pragma unroll
             for (int j = 0; j < RB; ++j) {
-                const int py = r0 + 4 * (h + j) - offf;
-                if (FULL || (py >= 0 && py < P)) col[py * cs] = cur[j] + cmulc(pv[j], w[h + j]);
+                const int py = grp + 4 * (h + j) - off;
+                if (FULL || (py >= 0 && py < P)) add_l2(&col[py * cs], cmulc(pv[j], w[h + j]));
             }
         }
     }
@@ -925,17 +961,17 @@ int ptycho_attrs()
         PT_ATTR((k_ptycho_adj_small<DET, 1>), s);
         PT_ATTR((k_ptycho_adj_small<DET, 2>), s);
     } else if constexpr (DET == 128) {
-        PT_ATTR((k_ptycho_fwd128<true>), P128_SMEM);
-        PT_ATTR((k_ptycho_fwd128<false>), P128_SMEM);
-        PT_ATTR((k_ptycho_fwd128<true, true>), P128_SMEM);
-        PT_ATTR((k_ptycho_fwd128<false, true>), P128_SMEM);
+        PT_ATTR((k_ptycho_fwd128<true>), P128_FSMEM);
+        PT_ATTR((k_ptycho_fwd128<false>), P128_FSMEM);
+        PT_ATTR((k_ptycho_fwd128<true, true>), P128_FSMEM);
+        PT_ATTR((k_ptycho_fwd128<false, true>), P128_FSMEM);
 #define PT_ATTR_ADJ(RESID)                                                  \
-    PT_ATTR((k_ptycho_adj128<true, RESID>), P128_SMEM);                     \
-    PT_ATTR((k_ptycho_adj128<false, RESID>), P128_SMEM);                    \
-    PT_ATTR((k_ptycho_adj128<true, RESID, true>), P128_SMEM);               \
-    PT_ATTR((k_ptycho_adj128<false, RESID, true>), P128_SMEM);              \
-    PT_ATTR((k_ptycho_adj128<true, RESID, false, true>), P128_SMEM);        \
-    PT_ATTR((k_ptycho_adj128<false, RESID, false, true>), P128_SMEM);
+    PT_ATTR((k_ptycho_adj128<true, RESID>), P128_ASMEM);                     \
+    PT_ATTR((k_ptycho_adj128<false, RESID>), P128_ASMEM);                    \
+    PT_ATTR((k_ptycho_adj128<true, RESID, true>), P128_ASMEM);               \
+    PT_ATTR((k_ptycho_adj128<false, RESID, true>), P128_ASMEM);              \
+    PT_ATTR((k_ptycho_adj128<true, RESID, false, true>), P128_ASMEM);        \
+    PT_ATTR((k_ptycho_adj128<false, RESID, false, true>), P128_ASMEM);
         PT_ATTR_ADJ(0)
         PT_ATTR_ADJ(1)
         PT_ATTR_ADJ(2)
@@ -975,7 +1011,7 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
         auto go = [&](auto full, auto sub) {
             constexpr bool FU = decltype(full)::value, S = decltype(sub)::value;
             if constexpr (DET == 128)
-                k_ptycho_adj128<FU, RESID, S><<<grid, 512, P128_SMEM, st>>>(
+                k_ptycho_adj128<FU, RESID, S><<<grid, 512, P128_ASMEM, st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, h->shift_ids());
             else
@@ -1014,7 +1050,7 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
         auto go = [&](auto full, auto sub) {
             constexpr bool FU = decltype(full)::value, S = decltype(sub)::value;
             if constexpr (DET == 128) {
-                k_ptycho_fwd128<FU, S><<<std::min(nframes, h->nsm), 512, P128_SMEM, st>>>(
+                k_ptycho_fwd128<FU, S><<<std::min(nframes, h->nsm), 512, P128_FSMEM, st>>>(
                     in, out, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, nframes, h->P, scale,
                     h->tw128, h->tw, h->shift_ids());
             } else {
@@ -1072,7 +1108,7 @@ int probe_adj_launch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 
         auto go = [&](auto full) {
             constexpr bool FU = decltype(full)::value;
             if constexpr (DET == 128)
-                k_ptycho_adj128<FU, RESID, false, true><<<h->prb_blocks, 512, P128_SMEM, st>>>(
+                k_ptycho_adj128<FU, RESID, false, true><<<h->prb_blocks, 512, P128_ASMEM, st>>>(
                     in, h->prb_part, h->corner, h->phase, h->prbT, h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, nullptr, psi, nframes);
             else
