@@ -194,7 +194,9 @@ struct FR {
     static constexpr int R2C = 256 / NT;                 // (k1, qb) pairs per thread
     static constexpr int BPS = 768 / BLOCK;              // resident blocks per SM at 80 registers a thread
     static constexpr int BPSP = 512 / BLOCK;             // probe adjoint: 128 registers
-    static constexpr size_t SMEM = (size_t)FPB * DET * DET * sizeof(float2);
+    // frames per trip: two for a probe smaller than the detector
+    static constexpr int nf(bool full) { return full || FPB > 1 ? 1 : 2; }
+    static constexpr size_t smem(bool full) { return (size_t)FPB * nf(full) * DET * DET * sizeof(float2); }
     static_assert(DET * RT == NT, "R1 and R3 give every thread one line of 16");
 };
 
@@ -289,6 +291,30 @@ __device__ __forceinline__ int fresh(int t)
     return t;
 }
 
+// *p += v in L2, without waiting for the sum (one FP32 addition per component,
+// as a load, an add and a store round it).  Each frame adds to a pixel at most
+// once and the frames of a block are separated by its barriers, so the order of
+// the sums, and the result, is that of the frames.
+__device__ __forceinline__ void add_l2(float2 *p, float2 v)
+{
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
+}
+
+// The lines of R1 (forward) or R3 (adjoint): RT lines of each window column,
+// px + P r.  Thread t takes line t of the trip's first frame (A) and, with two
+// frames per trip, a line of the second (B), on the threads that A leaves idle
+// first, so a narrow probe's two frames run on different warps.
+template <int DET, bool FULL, int FRAME>
+__device__ __forceinline__ void fr_line(int t, int PW, int &px, int &r)
+{
+    const int lines = PW * FR<DET>::RT;
+    const int l = FRAME == 0 ? t : (t >= lines ? t - lines : t + FR<DET>::NT - lines);
+    px = l % PW;
+    r = l / PW;      // valid if below RT
+}
+
+// Forward, grid-stride over frames (two consecutive ones per trip for a probe
+// smaller than the detector: three barriers for both).
 template <int DET, bool FULL, bool SUB = false>
 __global__ void __launch_bounds__(FR<DET>::BLOCK, FR<DET>::BPS)
     k_ptycho_fwd(const float2 *__restrict__ psi, float2 *__restrict__ g, const int *__restrict__ corner,
@@ -296,21 +322,30 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, FR<DET>::BPS)
                  int nframes, int P, float scale, const float2 *__restrict__ w, const int *__restrict__ sid = nullptr)
 {
     using F = FR<DET>;
+    constexpr int NF = F::nf(FULL);
     extern __shared__ float4 sm4[];
     const int t0 = threadIdx.x % F::NT, sub = threadIdx.x / F::NT;
     float2 *ex = reinterpret_cast<float2 *>(sm4) + sub * DET * DET;
     const int PW = FULL ? DET : P, off0 = FULL ? 0 : (DET - P) / 2;
-    // R1's line: column px of the window, rows rt + RT m
-    const int px0 = t0 % PW, rt0 = t0 / PW;
-    const bool line = rt0 < F::RT;
-    for (int f0 = blockIdx.x * F::FPB; f0 < nframes; f0 += gridDim.x * F::FPB) {
-        const int fid = f0 + sub;
-        const bool have = fid < nframes;
-        const int stx = have ? corner[2 * fid] : -1, sty = have ? corner[2 * fid + 1] : -1;
-        const bool act = stx >= 0 && sty >= 0;
-        const int t = fresh(t0), px = fresh(px0), rt = fresh(rt0), off = FULL ? 0 : fresh(off0);
-        if (act && line) {
-            const float2 *src = psi + ((size_t)(fid / nscan) * nz + sty) * n + stx + px;
+    int px0[NF], r0[NF];
+    fr_line<DET, FULL, 0>(t0, PW, px0[0], r0[0]);
+    if constexpr (NF == 2) fr_line<DET, FULL, 1>(t0, PW, px0[1], r0[1]);
+    for (int f0 = blockIdx.x * F::FPB * NF; f0 < nframes; f0 += gridDim.x * F::FPB * NF) {
+        int stx[NF], sty[NF];
+        bool act[NF];
+#pragma unroll
+        for (int j = 0; j < NF; ++j) {
+            const int fid = f0 + sub + j;
+            stx[j] = fid < nframes ? corner[2 * fid] : -1;
+            sty[j] = fid < nframes ? corner[2 * fid + 1] : -1;
+            act[j] = stx[j] >= 0 && sty[j] >= 0;
+        }
+        const int t = fresh(t0), off = FULL ? 0 : fresh(off0);
+#pragma unroll
+        for (int j = 0; j < NF; ++j) {
+            if (!act[j] || r0[j] >= F::RT) continue;
+            const int fid = f0 + sub + j, px = fresh(px0[j]), rt = fresh(r0[j]);
+            const float2 *src = psi + ((size_t)(fid / nscan) * nz + sty[j]) * n + stx[j] + px;
             const float2 *pr = (SUB ? prbT + (size_t)sid[fid] * P * P : prbT) + px;  // sub-pixel: the frame's shifted probe
             float2 v[16];
 #pragma unroll
@@ -318,35 +353,43 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, FR<DET>::BPS)
                 const int py = rt + F::RT * m - off;
                 v[m] = FULL || (py >= 0 && py < P) ? cmul(__ldg(&pr[py * PW]), __ldg(&src[(size_t)py * n])) : czero();
             }
-            fr_r1<DET, -1>(v, ex, off + px, rt, w);
+            fr_r1<DET, -1>(v, ex + j * DET * DET, off + px, rt, w);
         }
         __syncthreads();
-        if (act)
-            fr_r2<DET, -1>(ex, t, scale * phase[fid], w, [&](int q) { return FULL || (q >= off && q < off + P); },
-                           [](int) { return true; });
+#pragma unroll
+        for (int j = 0; j < NF; ++j)
+            if (act[j])
+                fr_r2<DET, -1>(ex + j * DET * DET, t, scale * phase[f0 + sub + j], w,
+                               [&](int q) { return FULL || (q >= off && q < off + P); }, [](int) { return true; });
         __syncthreads();
-        float2 v[16];
         const int u = t % DET, v1 = t / DET;
-        if (act) fr_r3_read<DET>(v, ex, u, v1);
-        __syncthreads();  // read: the next frame's R1 may write
-        if (!have) continue;
-        float2 *out = g + (size_t)fid * DET * DET;
-        if (act) {
-            ptfft::Dft<16, -1, true>::run(v);
-        } else {   // skipped scan: the reference leaves a zero frame
 #pragma unroll
-            for (int v2 = 0; v2 < 16; ++v2) v[v2] = czero();
+        for (int j = 0; j < NF; ++j) {
+            float2 v[16];
+            if (act[j]) fr_r3_read<DET>(v, ex + j * DET * DET, u, v1);
+            if (j == NF - 1) __syncthreads();  // read: the next trip's R1 may write
+            const int fid = f0 + sub + j;
+            if (fid >= nframes) continue;
+            float2 *out = g + (size_t)fid * DET * DET + v1 * DET + u;   // frame[kx = v1 + QA v2][ky = u]
+            if (act[j]) {
+                ptfft::Dft<16, -1, true>::run(v);
+            } else {   // skipped scan: the reference leaves a zero frame
+#pragma unroll
+                for (int v2 = 0; v2 < 16; ++v2) v[v2] = czero();
+            }
+#pragma unroll
+            for (int v2 = 0; v2 < 16; ++v2) __stcs(&out[F::QA * v2 * DET], v[v2]);
         }
-#pragma unroll
-        for (int v2 = 0; v2 < 16; ++v2) __stcs(&out[(v1 + F::QA * v2) * DET + u], v[v2]);  // frame[kx][ky = u]
     }
 }
 
 // Object adjoint: grid (parts, ntheta), block (part, angle) owns slab
-// dst[angle][part].  PROBE (the adjoint with respect to the probe): grid
-// (blocks, 1), block b walks frames b, b + gridDim.x, ... < nframes (FPB at a
-// time) and sums conj(psi patch) x frame into its P x P partial dst[b]; each
-// element belongs to one thread, which keeps it in registers (FPB = 1).
+// dst[angle][part] and walks scans part, part + parts, ... (two per trip for a
+// probe smaller than the detector).  PROBE (the adjoint with respect to the
+// probe): grid (blocks, 1), block b walks frames b, b + gridDim.x, ... <
+// nframes and sums conj(psi patch) x frame into its P x P partial dst[b] (one
+// per frame of the block); each element belongs to one thread, which keeps it
+// in registers.
 template <int DET, bool FULL, int RESID, bool SUB = false, bool PROBE = false>
 __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET>::BPS)
     k_ptycho_adj(const float2 *__restrict__ g, float2 *dst, const int *__restrict__ corner,
@@ -355,14 +398,16 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
                  const int *__restrict__ sid = nullptr, const float2 *psi = nullptr, int nframes = 0)
 {
     using F = FR<DET>;
+    constexpr int NF = PROBE ? 1 : F::nf(FULL);
     extern __shared__ float4 sm4[];
     const int t0 = threadIdx.x % F::NT, sub = threadIdx.x / F::NT;
     float2 *ex = reinterpret_cast<float2 *>(sm4) + sub * DET * DET;
     const int part = blockIdx.x, parts = gridDim.x, th0 = blockIdx.y;
     const int PW = FULL ? DET : P, off0 = FULL ? 0 : (DET - P) / 2;
-    // R3's line: window column px (= u - off), rows v1 + QA v2
-    const int px0 = t0 % PW, v10 = t0 / PW;
-    const bool line = v10 < F::QA;
+    // R3's lines: window column px (= u - off), rows r + QA v2
+    int px0[NF], r0[NF];
+    fr_line<DET, FULL, 0>(t0, PW, px0[0], r0[0]);
+    if constexpr (NF == 2) fr_line<DET, FULL, 1>(t0, PW, px0[1], r0[1]);
     float2 *slab = PROBE ? dst + (size_t)(part * F::FPB + sub) * P * P : dst + ((size_t)th0 * parts + part) * nz * n;
     if (!PROBE)
         for (int e = threadIdx.x; e < nz * n; e += F::BLOCK) slab[e] = czero();
@@ -372,17 +417,26 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
         for (int v2 = 0; v2 < 16; ++v2) acc[v2] = czero();
     }
     const int count = PROBE ? nframes : nscan;
-    for (int s0 = part * F::FPB; s0 < count; s0 += parts * F::FPB) {
-        const int s = s0 + sub;
-        const int fid = PROBE ? s : th0 * nscan + s;
-        const bool have = s < count;
-        const int stx = have ? corner[2 * fid] : -1, sty = have ? corner[2 * fid + 1] : -1;
-        const bool act = stx >= 0 && sty >= 0;
-        if (F::FPB == 1 && !act) continue;
-        const int t = fresh(t0), px = fresh(px0), v1 = fresh(v10), off = FULL ? 0 : fresh(off0);
-        if (act) {
+    // frame j of the trip that starts at s0
+    const int jstep = F::FPB > 1 ? 1 : parts;
+    for (int s0 = part * F::FPB; s0 < count; s0 += parts * F::FPB * NF) {
+        int stx[NF], sty[NF];
+        bool act[NF];
+#pragma unroll
+        for (int j = 0; j < NF; ++j) {
+            const int s = s0 + sub + j * jstep, fid = PROBE ? s : th0 * nscan + s;
+            stx[j] = s < count ? corner[2 * fid] : -1;
+            sty[j] = s < count ? corner[2 * fid + 1] : -1;
+            act[j] = stx[j] >= 0 && sty[j] >= 0;
+        }
+        if (F::FPB == 1 && !act[0] && !(NF == 2 && act[NF - 1])) continue;
+        const int t = fresh(t0), off = FULL ? 0 : fresh(off0);
+        auto frame = [&](int j) { return (PROBE ? 0 : th0 * nscan) + s0 + sub + j * jstep; };
+#pragma unroll
+        for (int j = 0; j < NF; ++j) {
+            if (!act[j]) continue;
             const int ky = t % DET, rt = t / DET;
-            const size_t e0 = (size_t)fid * DET * DET + rt * DET + ky;
+            const size_t e0 = (size_t)frame(j) * DET * DET + rt * DET + ky;
             float2 v[16];
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = __ldcs(&g[e0 + m * F::RT * DET]);
@@ -393,63 +447,78 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
 #pragma unroll
                 for (int m = 0; m < 16; ++m) v[m] = resid_of<RESID>(v[m], d[m] * dscale);
             }
-            fr_r1<DET, +1>(v, ex, ky, rt, w);
+            fr_r1<DET, +1>(v, ex + j * DET * DET, ky, rt, w);
         }
         __syncthreads();
-        if (act) {
-            const float2 ph = phase[fid];
-            fr_r2<DET, +1>(ex, t, make_float2(scale * ph.x, -scale * ph.y), w, [](int) { return true; },
-                           [&](int u) { return FULL || (u >= off && u < off + P); });
+#pragma unroll
+        for (int j = 0; j < NF; ++j) {
+            if (!act[j]) continue;
+            const float2 ph = phase[frame(j)];
+            fr_r2<DET, +1>(ex + j * DET * DET, t, make_float2(scale * ph.x, -scale * ph.y), w,
+                           [](int) { return true; }, [&](int u) { return FULL || (u >= off && u < off + P); });
         }
         __syncthreads();
-        float2 v[16];
-        if (act && line) fr_r3_read<DET>(v, ex, off + px, v1);
-        __syncthreads();  // read: the next frame's R1 may write
-        if (act && line) ptfft::Dft<16, +1, true>::run(v);
         // object: slab += conj(probe) x value; probe: sum of conj(psi) x value
-        const float2 *mul = PROBE ? psi + ((size_t)(fid / nscan) * nz + sty) * n + stx + px
-                                  : (SUB ? prbT + (size_t)(act ? sid[fid] : 0) * P * P : prbT) + px;
-        const size_t ms = PROBE ? n : PW;
-        // frames of one block that share a slab add to it one after the other
+        auto add = [&](int j, const float2 (&v)[16]) {
+            const int px = fresh(px0[j]), v1 = fresh(r0[j]), fid = frame(j);
+            const float2 *mul = (PROBE ? psi + ((size_t)(fid / nscan) * nz + sty[j]) * n + stx[j]
+                                       : (SUB ? prbT + (size_t)sid[fid] * P * P : prbT)) + px;
+            const size_t ms = PROBE ? n : PW;
+            float2 *col = slab + (size_t)sty[j] * n + stx[j] + px;
+            constexpr int RB = 8;   // multiplier loads in flight
 #pragma unroll
-        for (int o = 0; o < (PROBE ? 1 : F::FPB); ++o) {
-            if (!PROBE && o > 0) __syncthreads();
-            if (!act || !line || (!PROBE && F::FPB > 1 && sub != o)) continue;
-            if constexpr (PROBE) {
+            for (int h = 0; h < 16; h += RB) {
+                float2 pv[RB];
 #pragma unroll
-                for (int v2 = 0; v2 < 16; ++v2) {
-                    const int py = v1 + F::QA * v2 - off;
-                    if (FULL || (py >= 0 && py < P)) acc[v2] = acc[v2] + cmulc(__ldg(&mul[py * ms]), v[v2]);
+                for (int i = 0; i < RB; ++i) {
+                    const int py = v1 + F::QA * (h + i) - off;
+                    pv[i] = FULL || (py >= 0 && py < P) ? __ldg(&mul[py * ms]) : czero();
                 }
-            } else {
-                float2 *col = slab + (size_t)sty * n + stx + px;
-                // RB rows at a time: their loads are issued before the first store
-                constexpr int RB = FULL ? 8 : 4;
 #pragma unroll
-                for (int h = 0; h < 16; h += RB) {
-                    float2 cur[RB], pv[RB];
-#pragma unroll
-                    for (int j = 0; j < RB; ++j) {
-                        const int py = v1 + F::QA * (h + j) - off;
-                        const bool ok = FULL || (py >= 0 && py < P);
-                        pv[j] = ok ? __ldg(&mul[py * ms]) : czero();
-                        cur[j] = ok ? col[(size_t)py * n] : czero();
-                    }
-#pragma unroll
-                    for (int j = 0; j < RB; ++j) {
-                        const int py = v1 + F::QA * (h + j) - off;
-                        if (FULL || (py >= 0 && py < P)) col[(size_t)py * n] = cur[j] + cmulc(pv[j], v[h + j]);
-                    }
+                for (int i = 0; i < RB; ++i) {
+                    const int py = v1 + F::QA * (h + i) - off;
+                    if (!FULL && (py < 0 || py >= P)) continue;
+                    if constexpr (PROBE)
+                        acc[h + i] = acc[h + i] + cmulc(pv[i], v[h + i]);
+                    else
+                        add_l2(&col[(size_t)py * n], cmulc(pv[i], v[h + i]));
                 }
+            }
+        };
+        float2 v[16];
+        if constexpr (NF == 2) {
+            // frame A's sums are queued before the barrier, B's after it
+            if (act[0] && r0[0] < F::QA) {
+                fr_r3_read<DET>(v, ex, off + fresh(px0[0]), r0[0]);
+                ptfft::Dft<16, +1, true>::run(v);
+                add(0, v);
+            }
+            const bool b = act[1] && r0[1] < F::QA;
+            if (b) {
+                fr_r3_read<DET>(v, ex + DET * DET, off + fresh(px0[1]), r0[1]);
+                ptfft::Dft<16, +1, true>::run(v);
+            }
+            __syncthreads();  // read: the next trip's R1 may write
+            if (b) add(1, v);
+        } else {
+            const bool a = act[0] && r0[0] < F::QA;
+            if (a) fr_r3_read<DET>(v, ex, off + fresh(px0[0]), r0[0]);
+            __syncthreads();  // read: the next trip's R1 may write
+            if (a) ptfft::Dft<16, +1, true>::run(v);
+            // frames of one block that share a slab add to it one after the other
+#pragma unroll
+            for (int o = 0; o < (PROBE ? 1 : F::FPB); ++o) {
+                if (!PROBE && o > 0) __syncthreads();
+                if (a && (PROBE || F::FPB == 1 || sub == o)) add(0, v);
             }
         }
     }
     if constexpr (PROBE) {
-        if (line) {
+        if (r0[0] < F::QA) {
 #pragma unroll
             for (int v2 = 0; v2 < 16; ++v2) {
-                const int py = v10 + F::QA * v2 - off0;
-                if (FULL || (py >= 0 && py < P)) slab[(size_t)py * P + px0] = acc[v2];
+                const int py = r0[0] + F::QA * v2 - off0;
+                if (FULL || (py >= 0 && py < P)) slab[(size_t)py * P + px0[0]] = acc[v2];
             }
         }
     }
@@ -679,15 +748,6 @@ __global__ void __launch_bounds__(512, 1)
         stx = nsx;
         sty = nsy;
     }
-}
-
-// *p += v in L2, without waiting for the sum (one FP32 addition per component,
-// as a load, an add and a store round it).  Each frame adds to a pixel at most
-// once and the frames of a block are separated by its barriers, so the order of
-// the sums, and the result, is that of the frames.
-__device__ __forceinline__ void add_l2(float2 *p, float2 v)
-{
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
 }
 
 // The adjoints (see k_ptycho_fwd128).  Object adjoint: grid (parts, ntheta),
@@ -976,6 +1036,16 @@ int ptycho_attrs()
         PT_ATTR_ADJ(1)
         PT_ATTR_ADJ(2)
 #undef PT_ATTR_ADJ
+    } else if constexpr (FR<DET>::smem(false) > 48 * 1024) {
+        constexpr size_t s = FR<DET>::smem(false);
+        PT_ATTR((k_ptycho_fwd<DET, false>), s);
+        PT_ATTR((k_ptycho_fwd<DET, false, true>), s);
+        PT_ATTR((k_ptycho_adj<DET, false, 0>), s);
+        PT_ATTR((k_ptycho_adj<DET, false, 1>), s);
+        PT_ATTR((k_ptycho_adj<DET, false, 2>), s);
+        PT_ATTR((k_ptycho_adj<DET, false, 0, true>), s);
+        PT_ATTR((k_ptycho_adj<DET, false, 1, true>), s);
+        PT_ATTR((k_ptycho_adj<DET, false, 2, true>), s);
     }
 #undef PT_ATTR
     return PT_OK;
@@ -1015,7 +1085,7 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, h->shift_ids());
             else
-                k_ptycho_adj<DET, FU, RESID, S><<<grid, FR<DET>::BLOCK, FR<DET>::SMEM, st>>>(
+                k_ptycho_adj<DET, FU, RESID, S><<<grid, FR<DET>::BLOCK, FR<DET>::smem(FU), st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw,
                     data, dscale, h->shift_ids());
         };
@@ -1055,8 +1125,9 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
                     h->tw128, h->tw, h->shift_ids());
             } else {
                 using F = FR<DET>;
-                const int grid = std::min((nframes + F::FPB - 1) / F::FPB, h->nsm * F::BPS);
-                k_ptycho_fwd<DET, FU, S><<<grid, F::BLOCK, F::SMEM, st>>>(in, out, h->corner, h->phase_tab(),
+                const int per = F::FPB * F::nf(FU);
+                const int grid = std::min((nframes + per - 1) / per, h->nsm * F::BPS);
+                k_ptycho_fwd<DET, FU, S><<<grid, F::BLOCK, F::smem(FU), st>>>(in, out, h->corner, h->phase_tab(),
                                                                          h->probe_tab(), h->nz, h->n, h->nscan,
                                                                          nframes, h->P, scale, h->tw, h->shift_ids());
             }
@@ -1113,7 +1184,7 @@ int probe_adj_launch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 
                     h->tw, data, dscale, nullptr, psi, nframes);
             else
                 k_ptycho_adj<DET, FU, RESID, false, true>
-                    <<<h->prb_blocks / FR<DET>::FPB, FR<DET>::BLOCK, FR<DET>::SMEM, st>>>(
+                    <<<h->prb_blocks / FR<DET>::FPB, FR<DET>::BLOCK, FR<DET>::smem(true), st>>>(
                         in, h->prb_part, h->corner, h->phase, h->prbT, h->nz, h->n, h->nscan, h->P, scale, h->tw, data,
                         dscale, nullptr, psi, nframes);
         };
