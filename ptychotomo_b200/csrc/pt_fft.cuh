@@ -401,7 +401,7 @@ __device__ __forceinline__ void dft_half(const float2 (&in)[R / 2], float2 (&v)[
 // k1 alone and sit in the twiddle table.
 __host__ __device__ constexpr int split_r1(int L)
 {
-    return L == 12 ? 2 : L == 24 ? 4 : L <= 96 ? 8 : L <= 384 ? 16 : 32;
+    return L == 12 ? 2 : L == 24 ? 4 : L <= 96 ? 8 : L <= 384 ? 16 : L == 768 ? 24 : 32;
 }
 __host__ __device__ constexpr int split_r2(int L) { return L / split_r1(L); }
 

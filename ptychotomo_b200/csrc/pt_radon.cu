@@ -168,6 +168,12 @@ __global__ void k_takexy(float *x, float *y, const float *theta, int N, int nthe
     y[tx + ty * N] = yv;
 }
 
+// Resident blocks that the two-round kernels of length G are compiled for: 80
+// registers a thread at 768 and below without spills (256^3 forward 1.42 ->
+// 1.36 ms against two blocks of 128), one block at 1536 (48 x 32 values).
+template <int G>
+constexpr int row_blocks() { return G > 768 ? 1 : G > 384 ? 3 : 2; }
+
 // The forward's four kernels work on up to RSETS chunks of ZC slices per
 // launch, one per buffer set: the chunk is the last grid dimension, `set` the
 // distance of two sets in float2.
@@ -182,7 +188,7 @@ __global__ void k_takexy(float *x, float *y, const float *theta, int N, int nthe
 // with one trip through shared memory between: 12.4 us for 8 slices at 256
 // wide (four Stockham passes and two staging copies: 21.7 us).
 template <int G>
-__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
+__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, row_blocks<G>())
     k_fwd_rows(const float2 *__restrict__ u, float2 *__restrict__ rbuf, size_t set, int nz, int z0,
                const float *__restrict__ fac, const float4 *__restrict__ tw)
 {
@@ -238,7 +244,7 @@ constexpr int GH_PAIRS = NPAIR - 1;
 // outside N/2 .. 3N/2 - 1 are zero; the table is K1's.
 // 17.5 us for 8 slices at 256 wide (Stockham passes: 30.6 us).
 template <int G>
-__global__ void __launch_bounds__(ptfft::Exchange<G, CK * ZH>::NT, G > 768 ? 1 : 2)
+__global__ void __launch_bounds__(ptfft::Exchange<G, CK * ZH>::NT, row_blocks<G>())
     k_fwd_cols(const float2 *__restrict__ rbuf, float2 *__restrict__ fg, size_t set, const float4 *__restrict__ tw)
 {
     constexpr int NF = CK * ZH;
@@ -356,19 +362,24 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
 
 // The same gather with the grid staged in shared memory.  Points were sorted
 // at setobj by the 16 x 16-cell tile of their window origin; a block takes a
-// chunk of at most TCH points of one tile, loads the part of the haloed grid
+// chunk of at most tile_points points of one tile, loads the part of the haloed grid
 // that their windows cover (rows ty0 .. ty0 + 16 + W - 2, column pairs
 // tx0/2 .. tx0/2 + 11, clipped to the haloed grid) and the points' records
 // once, and gathers from there.  Weights, loads and the order of the sums are
 // those of k_fwd_gather_pts, so the results are bit-identical.
-constexpr int TCH = 128;   // points per block of the tiled gather
+// points per block of the tiled gather: up to 128 wide there are too few blocks
+// of 128 points to fill the GPU evenly (64^3 forward 64 -> 53 us, 128^3 208 ->
+// 204); at 256 wide half-empty blocks cost more than they balance (1.42 and
+// 1.45 ms)
+template <int N>
+constexpr int tile_points() { return N <= 192 ? 64 : 128; }
 template <int W>
 constexpr int tile_rows() { return GTILE + W - 1; }
 constexpr int TILE_PAIRS = GTILE / 2 - 1 + NPAIR;
 template <int W>
 constexpr size_t tile_bytes() { return (size_t)tile_rows<W>() * TILE_PAIRS * ZC * sizeof(float4); }
-template <int W>
-constexpr size_t tile_smem() { return tile_bytes<W>() + (size_t)TCH * REC4 * sizeof(float4); }
+template <int N, int W>
+constexpr size_t tile_smem() { return tile_bytes<W>() + (size_t)tile_points<N>() * REC4 * sizeof(float4); }
 
 // The gather of one chunk's points from its staged tile and records (both tiled kernels).
 template <int W>
@@ -422,8 +433,8 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
 // 128-byte aligned base; checked, and a misaligned base is recorded in *err
 // instead of issuing the copy).
 constexpr int TMA_SPIN = 1 << 24;
-template <int W>
-constexpr size_t tma_smem() { return tile_smem<W>() + 16; }
+template <int N, int W>
+constexpr size_t tma_smem() { return tile_smem<N, W>() + 16; }
 struct GridMaps {
     CUtensorMap m[RSETS];   // one per buffer set
 };
@@ -436,7 +447,7 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
     // check != 0 (the status test only): the blocks first wait on a second
     // barrier that nothing arrives at, so that wait runs out on purpose; the
     // failure path then waits for the copies themselves before returning
-    constexpr unsigned TB = (unsigned)tile_bytes<W>(), END = (unsigned)tile_smem<W>();
+    constexpr unsigned TB = (unsigned)tile_bytes<W>(), END = (unsigned)tile_smem<N, W>();
     static_assert(TB % 128 == 0 && END % 16 == 0, "the records and the mbarriers follow the tile");
     extern __shared__ __align__(128) float4 tsm_tma[];
     float4 *tsm = tsm_tma, *rsm = tsm_tma + TB / sizeof(float4);
@@ -728,7 +739,7 @@ __device__ __forceinline__ void adj_row_round1(const float2 *__restrict__ src, i
 // grid (n, nzp / ZC); reads rbuf[(r * G + kx) * nzp + z].  tw: W^(i2 k1)
 // (-1)^i2, inverse (the sign of the grid column; that of the output is in fac).
 template <int G>
-__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
+__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, row_blocks<G>())
     k_adj_rows(const float2 *__restrict__ rbuf, float2 *__restrict__ out, int nz, int nzp,
                const float *__restrict__ fac, float scale, const float4 *__restrict__ tw)
 {
@@ -766,7 +777,7 @@ __global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
 // the crop goes to out, a margin row (ty <= c0 or ty >= c0 + n - 1) to its
 // slot of mbuf [n/2 + 2][nz][n] for the fold along y.
 template <int G>
-__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, G > 768 ? 1 : 2)
+__global__ void __launch_bounds__(ptfft::Exchange<G, ZC>::NT, row_blocks<G>())
     k_adj_rows_exact(const float2 *__restrict__ rbuf, float2 *__restrict__ out, float2 *__restrict__ mbuf, int nz,
                      int nzp, const float *__restrict__ fac, float scale, const float4 *__restrict__ tw)
 {
@@ -970,10 +981,10 @@ int set_attrs()
     PT_ATTR(k_fwd_lines<N>, ex_smem<N>());
     PT_ATTR(k_adj_lines<N>, ex_smem<N>());
     PT_ATTR((k_adj_lines<N, true>), ex_smem<N>());
-    PT_ATTR((k_fwd_gather_tile<N, WKB>), tile_smem<WKB>());
-    PT_ATTR((k_fwd_gather_tile<N, WGAUSS>), tile_smem<WGAUSS>());
-    PT_ATTR((k_fwd_gather_tma<N, WKB>), tma_smem<WKB>());
-    PT_ATTR((k_fwd_gather_tma<N, WGAUSS>), tma_smem<WGAUSS>());
+    PT_ATTR((k_fwd_gather_tile<N, WKB>), (tile_smem<N, WKB>()));
+    PT_ATTR((k_fwd_gather_tile<N, WGAUSS>), (tile_smem<N, WGAUSS>()));
+    PT_ATTR((k_fwd_gather_tma<N, WKB>), (tma_smem<N, WKB>()));
+    PT_ATTR((k_fwd_gather_tma<N, WGAUSS>), (tma_smem<N, WGAUSS>()));
 #undef PT_ATTR
     return PT_OK;
 }
@@ -1007,11 +1018,11 @@ int run_fwd(pt_radon *h, float2 *g, const float2 *f, float scale, cudaStream_t s
         k_fwd_cols<G><<<dim3(G / CK, ZC / ZH, cnt), EG::NT, EG::BYTES, s>>>(rb, fg, stride, h->tw_fwd);
         PT_LAUNCHED("k_fwd_cols");
         if (h->gather == 2) {
-            k_fwd_gather_tma<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tma_smem<W>(), s>>>(
+            k_fwd_gather_tma<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tma_smem<N, W>(), s>>>(
                 h->tmap, k, ln, h->rec, h->chunks, npts, h->tma_err);
             PT_LAUNCHED("k_fwd_gather_tma");
         } else if (h->gather == 1) {
-            k_fwd_gather_tile<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tile_smem<W>(), s>>>(fg, stride, ln, h->rec,
+            k_fwd_gather_tile<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tile_smem<N, W>(), s>>>(fg, stride, ln, h->rec,
                                                                                            h->chunks, npts);
             PT_LAUNCHED("k_fwd_gather_tile");
         } else {
@@ -1106,7 +1117,7 @@ template <int G, int W>
 int run_tma_wait_check(pt_radon *h, cudaStream_t st)
 {
     constexpr int N = G / 2;
-    k_fwd_gather_tma<N, W><<<h->nchunks, GPB * ZC, tma_smem<W>(), st>>>(h->tmap, 0, h->lines, h->rec, h->chunks,
+    k_fwd_gather_tma<N, W><<<h->nchunks, GPB * ZC, tma_smem<N, W>(), st>>>(h->tmap, 0, h->lines, h->rec, h->chunks,
                                                                         h->ntheta * N, h->tma_err, 256, 1);
     PT_LAUNCHED("k_fwd_gather_tma");
     return PT_OK;
@@ -1400,14 +1411,15 @@ extern "C" int pt_radon_setobj(pt_radon *h, const float *theta, void *stream)
             k_point_records<WGAUSS><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts,
                                                             radon_pre(h));
         PT_LAUNCHED("k_point_records");
-        // the tiled gather's blocks: runs of one tile in perm order, at most TCH points each
+        // the tiled gather's blocks: runs of one tile in perm order, at most tile_points points each
         std::vector<int4> chunks;
         for (size_t i = 0; i < npts;) {
             size_t j = i;
             while (j < npts && tile[perm[j]] == tile[perm[i]]) ++j;
             const int t = (int)tile[perm[i]];
-            for (size_t f = i; f < j; f += TCH)
-                chunks.push_back(make_int4(t / TPR, t % TPR, (int)f, (int)std::min<size_t>(TCH, j - f)));
+            const size_t most = N <= 192 ? tile_points<192>() : tile_points<384>();
+            for (size_t f = i; f < j; f += most)
+                chunks.push_back(make_int4(t / TPR, t % TPR, (int)f, (int)std::min(most, j - f)));
             i = j;
         }
         if ((int)chunks.size() > h->chunks_cap) {
