@@ -40,28 +40,38 @@ __device__ __forceinline__ void block_reduce_store(double (&acc)[K], double *wor
     }
 }
 
-// one block: out[k] = sum_b work[k * nblk + b] (fixed order per thread, then tree)
-__global__ void k_finish(const double *__restrict__ work, double *__restrict__ out, int K, int nblk, int op_max,
-                         const double *__restrict__ skip = nullptr)
+// out[k] = sum_b work[k * nblk + b], warp k of one block (K warps), in the order
+// of 256 strided sums and a binary tree over them: lane l holds the strided
+// sums l, l + 32, ..., l + 224, whose loads are independent, and the last five
+// levels are shuffles.  No shared memory and no barrier (with 256 threads per
+// value and nine barriers, one value after the other, 4.8 us; now 3.3).
+__global__ void __launch_bounds__(32 * MAXK) k_finish(const double *__restrict__ work, double *__restrict__ out,
+                                                      int nblk, int op_max, const double *__restrict__ skip = nullptr)
 {
     if (skip != nullptr && *skip != 0.0) return;   // a pass the caller's device-side decision made unnecessary
-    __shared__ double red[RT];
-    for (int k = 0; k < K; ++k) {
-        double s = op_max ? -1.0 : 0.0;
-        for (int b = threadIdx.x; b < nblk; b += RT) {
-            const double v = work[(size_t)k * nblk + b];
-            s = op_max ? fmax(s, v) : s + v;
-        }
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = RT / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) red[threadIdx.x] = op_max ? fmax(red[threadIdx.x], red[threadIdx.x + w])
-                                                           : red[threadIdx.x] + red[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[k] = red[0];
-        __syncthreads();
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double *p = work + (size_t)k * nblk;
+    constexpr int S = RT / 32;
+    double s[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) s[j] = op_max ? -1.0 : 0.0;
+    for (int b0 = lane; b0 < nblk; b0 += RT) {
+        double v[S];
+#pragma unroll
+        for (int j = 0; j < S; ++j) v[j] = b0 + 32 * j < nblk ? p[b0 + 32 * j] : (op_max ? -1.0 : 0.0);
+#pragma unroll
+        for (int j = 0; j < S; ++j) s[j] = op_max ? fmax(s[j], v[j]) : s[j] + v[j];
     }
+#pragma unroll
+    for (int w = S / 2; w > 0; w >>= 1)
+#pragma unroll
+        for (int j = 0; j < w; ++j) s[j] = op_max ? fmax(s[j], s[j + w]) : s[j] + s[j + w];
+    double r = s[0];
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_down_sync(0xffffffffu, r, o);
+        r = op_max ? fmax(r, v) : r + v;
+    }
+    if (lane == 0) out[k] = r;
 }
 
 // ---- generic reductions over complex64 arrays --------------------------------
@@ -73,41 +83,64 @@ __global__ void k_finish(const double *__restrict__ work, double *__restrict__ o
 // op 5: ||a - b||^2                     -> 1 value
 // op 6: sum_i sqrt(|a_i|^2 + |a_{i+n}|^2 + |a_{i+2n}|^2) (a has 3n entries) -> 1 value
 // op 7: max |angle(a)|                  -> 1 value
-__global__ void __launch_bounds__(RT) k_reduce(int op, const float2 *__restrict__ a, const float2 *__restrict__ b,
-                                               size_t n, int c0, int c1, int ncol, double *__restrict__ work)
+// The values of element i are added to acc.
+template <int OP>
+__device__ __forceinline__ void reduce_value(double (&acc)[3], float2 x, float2 y, float2 z, bool in_band)
 {
-    double acc[3] = {0, 0, 0};
-    const bool is_max = (op == 3 || op == 7);
-    if (is_max) acc[0] = -1.0;
-    for (size_t i = (size_t)blockIdx.x * RT + threadIdx.x; i < n; i += (size_t)gridDim.x * RT) {
-        const float2 x = a[i];
-        if (op == 5) {
-            const float2 y = b[i];
-            const double dx = (double)x.x - y.x, dy = (double)x.y - y.y;
-            acc[0] += dx * dx + dy * dy;
-        } else if (op == 6) {
-            const float2 y = a[i + n], z = a[i + 2 * n];
-            acc[0] += (double)sqrtf(x.x * x.x + x.y * x.y + y.x * y.x + y.y * y.y + z.x * z.x + z.y * z.y);
-        } else if (op == 7) {
-            acc[0] = fmax(acc[0], (double)fabsf(atan2f(x.y, x.x)));
-        } else if (op == 0) {
-            acc[0] += (double)x.x * x.x + (double)x.y * x.y;
-        } else if (op == 1) {
-            const float2 y = b[i];
-            acc[0] += (double)x.x * y.x + (double)x.y * y.y;
-            acc[1] += (double)x.x * y.y - (double)x.y * y.x;
-        } else if (op == 2) {
-            const float2 y = b[i];
-            acc[0] += (double)x.x * x.x + (double)x.y * x.y;
-            acc[1] += (double)x.x * y.x + (double)x.y * y.y;
-            acc[2] += (double)y.x * y.x + (double)y.y * y.y;
-        } else if (op == 3) {
-            acc[0] = fmax(acc[0], (double)hypotf(x.x, x.y));
-        } else {
-            const int col = (int)(i % ncol);
-            if (col >= c0 && col < c1) acc[0] += (double)atan2f(x.y, x.x);
-        }
+    if (OP == 5) {
+        const double dx = (double)x.x - y.x, dy = (double)x.y - y.y;
+        acc[0] += dx * dx + dy * dy;
+    } else if (OP == 6) {
+        acc[0] += (double)sqrtf(x.x * x.x + x.y * x.y + y.x * y.x + y.y * y.y + z.x * z.x + z.y * z.y);
+    } else if (OP == 7) {
+        acc[0] = fmax(acc[0], (double)fabsf(atan2f(x.y, x.x)));
+    } else if (OP == 0) {
+        acc[0] += (double)x.x * x.x + (double)x.y * x.y;
+    } else if (OP == 1) {
+        acc[0] += (double)x.x * y.x + (double)x.y * y.y;
+        acc[1] += (double)x.x * y.y - (double)x.y * y.x;
+    } else if (OP == 2) {
+        acc[0] += (double)x.x * x.x + (double)x.y * x.y;
+        acc[1] += (double)x.x * y.x + (double)x.y * y.y;
+        acc[2] += (double)y.x * y.x + (double)y.y * y.y;
+    } else if (OP == 3) {
+        acc[0] = fmax(acc[0], (double)hypotf(x.x, x.y));
+    } else {
+        if (in_band) acc[0] += (double)atan2f(x.y, x.x);
     }
+}
+
+// Bound by memory once U elements per thread are loaded before the first is
+// added; eight reductions of pairs of 1.4 and 4.1 M elements take 74 us.
+template <int OP>
+__global__ void __launch_bounds__(RT) k_reduce(const float2 *__restrict__ a, const float2 *__restrict__ b, size_t n,
+                                               int c0, int c1, int ncol, double *__restrict__ work)
+{
+    constexpr bool TWO = OP == 1 || OP == 2 || OP == 5, is_max = OP == 3 || OP == 7;
+    constexpr int U = OP == 6 ? 2 : 4;
+    double acc[3] = {is_max ? -1.0 : 0.0, 0, 0};
+    const size_t stride = (size_t)gridDim.x * RT;
+    size_t i = (size_t)blockIdx.x * RT + threadIdx.x;
+    auto in_band = [&](size_t e) {
+        if (OP != 4) return false;
+        const int col = (int)(e % ncol);
+        return col >= c0 && col < c1;
+    };
+    for (; i + (U - 1) * stride < n; i += U * stride) {
+        float2 x[U], y[U], z[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const size_t e = i + u * stride;
+            x[u] = a[e];
+            y[u] = TWO ? b[e] : (OP == 6 ? a[e + n] : czero());
+            z[u] = OP == 6 ? a[e + 2 * n] : czero();
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) reduce_value<OP>(acc, x[u], y[u], z[u], in_band(i + u * stride));
+    }
+    for (; i < n; i += stride)
+        reduce_value<OP>(acc, a[i], TWO ? b[i] : (OP == 6 ? a[i + n] : czero()), OP == 6 ? a[i + 2 * n] : czero(),
+                         in_band(i));
     if (is_max) {
         // max: reduce with max instead of sum
         __shared__ double red[RT];
@@ -320,25 +353,92 @@ struct Lin4 {
     float2 c[4];
 };
 
-// out = sum_{i<k} c_i x_i  (out may alias any x_i)
-__global__ void k_lincomb(float2 *__restrict__ out, size_t n, int k, Lin4 p)
+// out = sum_{i<K} c_i x_i  (out may alias any x_i: every element is read and
+// written by one thread).  Memory-bound: V complex values per access (2 where
+// every array is 16-byte aligned), U accesses a stride apart loaded first: 23
+// launches of a tomography CG at 84 x 128 x 128 take 161 us, with one 8-byte
+// access per term and trip 24 took 299.
+template <int K, int V, int U>
+__global__ void __launch_bounds__(256) k_lincomb(float2 *out, size_t n, Lin4 p)
 {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    struct alignas(V * sizeof(float2)) Pack {
+        float2 v[V];
+    };
+    const size_t stride = (size_t)gridDim.x * blockDim.x, np = n / V;
+    auto sum = [&](const Pack (&x)[K]) {
+        Pack r;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            float2 acc = czero();
+#pragma unroll
+            for (int j = 0; j < K; ++j) acc = acc + cmul(p.c[j], x[j].v[e]);
+            r.v[e] = acc;
+        }
+        return r;
+    };
+    auto at = [&](int j, size_t i) { return reinterpret_cast<const Pack *>(p.x[j])[i]; };
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + (U - 1) * stride < np; i += U * stride) {
+        Pack x[U][K];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int j = 0; j < K; ++j) x[u][j] = at(j, i + u * stride);
+#pragma unroll
+        for (int u = 0; u < U; ++u) reinterpret_cast<Pack *>(out)[i + u * stride] = sum(x[u]);
+    }
+    for (; i < np; i += stride) {
+        Pack x[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) x[j] = at(j, i);
+        reinterpret_cast<Pack *>(out)[i] = sum(x);
+    }
+    if (V > 1 && blockIdx.x == 0 && threadIdx.x < n % V) {   // the elements past the last whole access
+        const size_t e = np * V + threadIdx.x;
         float2 acc = czero();
-        for (int j = 0; j < k; ++j) acc = acc + cmul(p.c[j], p.x[j][i]);
-        out[i] = acc;
+#pragma unroll
+        for (int j = 0; j < K; ++j) acc = acc + cmul(p.c[j], p.x[j][e]);
+        out[e] = acc;
     }
 }
 
-// mode 0: out = a * b;  mode 1: out = conj(a) * (b - c);  mode 2: out = conj(a) * b
-__global__ void k_cmul(float2 *__restrict__ out, const float2 *__restrict__ a, const float2 *__restrict__ b,
-                       const float2 *__restrict__ c, size_t n, int mode)
+// MODE 0: out = a * b;  1: out = conj(a) * (b - c);  2: out = conj(a) * b; out
+// may alias an input.  V and U as in k_lincomb.
+template <int MODE, int V, int U>
+__global__ void __launch_bounds__(256) k_cmul(float2 *out, const float2 *a, const float2 *b, const float2 *c, size_t n)
 {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float2 x = a[i];
-        float2 y = b[i];
-        if (mode == 1) y = y - c[i];
-        out[i] = mode == 0 ? cmul(x, y) : cmulc(x, y);
+    struct alignas(V * sizeof(float2)) Pack {
+        float2 v[V];
+    };
+    auto product = [](float2 x, float2 y, float2 z) {
+        if (MODE == 1) y = y - z;
+        return MODE == 0 ? cmul(x, y) : cmulc(x, y);
+    };
+    auto at = [](const float2 *p, size_t i) { return reinterpret_cast<const Pack *>(p)[i]; };
+    const size_t stride = (size_t)gridDim.x * blockDim.x, np = n / V;
+    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i < np; i += U * stride) {
+        Pack x[U], y[U], z[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const size_t e = i + u * stride;
+            if (e >= np) break;
+            x[u] = at(a, e);
+            y[u] = at(b, e);
+            if (MODE == 1) z[u] = at(c, e);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i + u * stride >= np) break;
+            Pack r;
+#pragma unroll
+            for (int k = 0; k < V; ++k) r.v[k] = product(x[u].v[k], y[u].v[k], MODE == 1 ? z[u].v[k] : czero());
+            reinterpret_cast<Pack *>(out)[i + u * stride] = r;
+        }
+    }
+    if (V > 1 && blockIdx.x == 0 && threadIdx.x < n % V) {   // the elements past the last whole access
+        const size_t e = np * V + threadIdx.x;
+        out[e] = product(a[e], b[e], MODE == 1 ? c[e] : czero());
     }
 }
 
@@ -409,30 +509,45 @@ __global__ void k_abs2(float *__restrict__ out, const float2 *__restrict__ x, si
 }
 
 // ---- TV regulariser J, J* (solver.py:128-146) --------------------------------
+// A thread walks rows (z, y) of the volume at one x or at x, x + blockDim.x,
+// ...: one 32-bit division per row instead of two 64-bit ones per voxel (J* at
+// 84 x 128 x 128: 12.8 -> 10.8 us, J stays at 10.6, bound by its stores).
+template <typename Body>
+__device__ __forceinline__ void for_voxels(int nz, int ny, int nx, Body body)
+{
+    const size_t rows = (size_t)nz * ny;
+    const bool narrow = rows < ((size_t)1 << 32);
+    for (size_t r = blockIdx.x * blockDim.y + threadIdx.y; r < rows; r += gridDim.x * blockDim.y) {
+        const size_t z = narrow ? (unsigned)r / (unsigned)ny : r / ny;
+        const int y = (int)(r - z * ny);
+        for (int x = threadIdx.x; x < nx; x += blockDim.x) body(r * nx + x, x, y, (int)z);
+    }
+}
+
 // u [nz][ny][nx]; res [3][nz][ny][nx]: forward differences along x, y, z times s
-__global__ void k_reg_fwd(float2 *__restrict__ res, const float2 *__restrict__ u, int nz, int ny, int nx, float s)
+__global__ void __launch_bounds__(256)
+    k_reg_fwd(float2 *__restrict__ res, const float2 *__restrict__ u, int nz, int ny, int nx, float s)
 {
     const size_t vol = (size_t)nz * ny * nx;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < vol; i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
+    for_voxels(nz, ny, nx, [&](size_t i, int x, int y, int z) {
         const float2 c = u[i];
         res[i] = x < nx - 1 ? s * (u[i + 1] - c) : czero();
         res[vol + i] = y < ny - 1 ? s * (u[i + nx] - c) : czero();
         res[2 * vol + i] = z < nz - 1 ? s * (u[i + (size_t)nx * ny] - c) : czero();
-    }
+    });
 }
 
-__global__ void k_reg_adj(float2 *__restrict__ res, const float2 *__restrict__ g, int nz, int ny, int nx, float s)
+__global__ void __launch_bounds__(256)
+    k_reg_adj(float2 *__restrict__ res, const float2 *__restrict__ g, int nz, int ny, int nx, float s)
 {
     const size_t vol = (size_t)nz * ny * nx;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < vol; i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
-        const float2 *g0 = g, *g1 = g + vol, *g2 = g + 2 * vol;
+    const float2 *g0 = g, *g1 = g + vol, *g2 = g + 2 * vol;
+    for_voxels(nz, ny, nx, [&](size_t i, int x, int y, int z) {
         float2 r = x > 0 ? g0[i] - g0[i - 1] : g0[i];
         r = r + (y > 0 ? g1[i] - g1[i - nx] : g1[i]);
         r = r + (z > 0 ? g2[i] - g2[i - (size_t)nx * ny] : g2[i]);
         res[i] = s * r;
-    }
+    });
 }
 
 // the entries of g [3][nz][ny][nx] outside the range of J: x = nx-1 of
@@ -477,6 +592,20 @@ __global__ void k_solve_reg(float2 *__restrict__ z, const float2 *__restrict__ u
     }
 }
 
+// launch shape of for_voxels: the block's x extent covers a row (at most 256)
+struct VoxelShape {
+    dim3 block;
+    unsigned grid;
+};
+VoxelShape voxel_shape(int nz, int ny, int nx)
+{
+    unsigned bx = 32;
+    while (bx < 256 && bx < (unsigned)nx) bx *= 2;
+    const unsigned by = 256 / bx;
+    const size_t rows = (size_t)nz * ny, blocks = (rows + by - 1) / by;
+    return {dim3(bx, by), (unsigned)(blocks < 148 * 32 ? blocks : 148 * 32)};
+}
+
 unsigned ew_blocks(size_t n)
 {
     size_t b = (n + 255) / 256;
@@ -497,9 +626,16 @@ extern "C" int pt_reduce_c64(int op, const void *a, const void *b, size_t n, int
     PT_CHECK_ARG(op != 4 || (ncol > 0 && c0 >= 0 && c1 <= ncol), "reduce: bad column band");
     cudaStream_t st = (cudaStream_t)stream;
     const int K = op == 1 ? 2 : (op == 2 ? 3 : 1);
-    k_reduce<<<RB, RT, 0, st>>>(op, (const float2 *)a, (const float2 *)b, n, c0, c1, ncol, (double *)work);
+    switch (op) {
+#define PT_CASE(OP)                                                                                                   \
+    case OP:                                                                                                          \
+        k_reduce<OP><<<RB, RT, 0, st>>>((const float2 *)a, (const float2 *)b, n, c0, c1, ncol, (double *)work);       \
+        break;
+        PT_CASE(0) PT_CASE(1) PT_CASE(2) PT_CASE(3) PT_CASE(4) PT_CASE(5) PT_CASE(6) PT_CASE(7)
+#undef PT_CASE
+    }
     PT_LAUNCHED("k_reduce");
-    k_finish<<<1, RT, 0, st>>>((const double *)work, (double *)out, K, RB, op == 3 || op == 7);
+    k_finish<<<1, 32 * K, 0, st>>>((const double *)work, (double *)out, RB, op == 3 || op == 7);
     PT_LAUNCHED("k_finish");
     return PT_OK;
 }
@@ -516,7 +652,7 @@ extern "C" int pt_ls_frames(const void *f, const void *d, const float *data, flo
     const int rc = launch_ls_frames((const float2 *)f, (const float2 *)d, data, dscale, n, model, gammas, J,
                                     (double *)work, st, &nblk);
     if (rc != PT_OK) return rc;
-    k_finish<<<1, RT, 0, st>>>((const double *)work, (double *)out, J, nblk, 0);
+    k_finish<<<1, 32 * J, 0, st>>>((const double *)work, (double *)out, nblk, 0);
     PT_LAUNCHED("k_finish");
     return PT_OK;
 }
@@ -533,7 +669,7 @@ extern "C" int pt_ls_frames_advance(void *f, const void *d, const float *data, f
     const int rc = launch_ls_frames((const float2 *)f, (const float2 *)d, data, dscale, n, model, gammas, J,
                                     (double *)work, st, &nblk, (float2 *)f);
     if (rc != PT_OK) return rc;
-    k_finish<<<1, RT, 0, st>>>((const double *)work, (double *)out, J, nblk, 0);
+    k_finish<<<1, 32 * J, 0, st>>>((const double *)work, (double *)out, nblk, 0);
     PT_LAUNCHED("k_finish");
     return PT_OK;
 }
@@ -550,7 +686,7 @@ extern "C" int pt_ls_frames_dev(const void *f, const void *d, const float *data,
     const int rc = launch_ls_frames((const float2 *)f, (const float2 *)d, data, dscale, n, model, gammas, J,
                                     (double *)work, st, &nblk, nullptr, skip);
     if (rc != PT_OK) return rc;
-    k_finish<<<1, RT, 0, st>>>((const double *)work, (double *)out, J, nblk, 0, skip);
+    k_finish<<<1, 32 * J, 0, st>>>((const double *)work, (double *)out, nblk, 0, skip);
     PT_LAUNCHED("k_finish");
     return PT_OK;
 }
@@ -563,7 +699,7 @@ extern "C" int pt_lagr_frames(const void *f, const float *data, float dscale, si
     cudaStream_t st = (cudaStream_t)stream;
     k_lagr_frames<<<RB, RT, 0, st>>>((const float2 *)f, data, dscale, n, model, (double *)work);
     PT_LAUNCHED("k_lagr_frames");
-    k_finish<<<1, RT, 0, st>>>((const double *)work, (double *)out, 1, RB, 0);
+    k_finish<<<1, 32 * 1, 0, st>>>((const double *)work, (double *)out, RB, 0);
     PT_LAUNCHED("k_finish");
     return PT_OK;
 }
@@ -578,7 +714,26 @@ extern "C" int pt_lincomb_c64(void *out, size_t n, int k, const void *const *x, 
         p.c[j] = j < k ? make_float2(coef[2 * j], coef[2 * j + 1]) : czero();
         PT_CHECK_ARG(j >= k || p.x[j], "lincomb: null term %d", j);
     }
-    k_lincomb<<<ew_blocks(n), 256, 0, (cudaStream_t)stream>>>((float2 *)out, n, k, p);
+    uintptr_t low = (uintptr_t)out;
+    for (int j = 0; j < k; ++j) low |= (uintptr_t)x[j];
+    cudaStream_t st = (cudaStream_t)stream;
+    float2 *o = (float2 *)out;
+    if (low % 16 == 0) {
+        const unsigned blocks = ew_blocks((n + 1) / 2);
+        switch (k) {
+        case 1: k_lincomb<1, 2, 4><<<blocks, 256, 0, st>>>(o, n, p); break;
+        case 2: k_lincomb<2, 2, 2><<<blocks, 256, 0, st>>>(o, n, p); break;
+        case 3: k_lincomb<3, 2, 2><<<blocks, 256, 0, st>>>(o, n, p); break;
+        default: k_lincomb<4, 2, 1><<<blocks, 256, 0, st>>>(o, n, p);
+        }
+    } else {
+        switch (k) {
+        case 1: k_lincomb<1, 1, 4><<<ew_blocks(n), 256, 0, st>>>(o, n, p); break;
+        case 2: k_lincomb<2, 1, 4><<<ew_blocks(n), 256, 0, st>>>(o, n, p); break;
+        case 3: k_lincomb<3, 1, 2><<<ew_blocks(n), 256, 0, st>>>(o, n, p); break;
+        default: k_lincomb<4, 1, 2><<<ew_blocks(n), 256, 0, st>>>(o, n, p);
+        }
+    }
     PT_LAUNCHED("k_lincomb");
     return PT_OK;
 }
@@ -587,8 +742,19 @@ extern "C" int pt_cmul_c64(void *out, const void *a, const void *b, const void *
 {
     pt::clear_error();
     PT_CHECK_ARG(out && a && b && (mode != 1 || c) && mode >= 0 && mode <= 2, "cmul: bad arguments");
-    k_cmul<<<ew_blocks(n), 256, 0, (cudaStream_t)stream>>>((float2 *)out, (const float2 *)a, (const float2 *)b,
-                                                           (const float2 *)c, n, mode);
+    const bool wide = (((uintptr_t)out | (uintptr_t)a | (uintptr_t)b | (mode == 1 ? (uintptr_t)c : 0)) & 15) == 0;
+    const unsigned blocks = ew_blocks(wide ? (n + 1) / 2 : n);
+    cudaStream_t st = (cudaStream_t)stream;
+    float2 *o = (float2 *)out;
+    const float2 *x = (const float2 *)a, *y = (const float2 *)b, *z = (const float2 *)c;
+    switch (2 * mode + wide) {
+    case 0: k_cmul<0, 1, 2><<<blocks, 256, 0, st>>>(o, x, y, z, n); break;
+    case 1: k_cmul<0, 2, 2><<<blocks, 256, 0, st>>>(o, x, y, z, n); break;
+    case 2: k_cmul<1, 1, 2><<<blocks, 256, 0, st>>>(o, x, y, z, n); break;
+    case 3: k_cmul<1, 2, 2><<<blocks, 256, 0, st>>>(o, x, y, z, n); break;
+    case 4: k_cmul<2, 1, 2><<<blocks, 256, 0, st>>>(o, x, y, z, n); break;
+    default: k_cmul<2, 2, 2><<<blocks, 256, 0, st>>>(o, x, y, z, n);
+    }
     PT_LAUNCHED("k_cmul");
     return PT_OK;
 }
@@ -626,8 +792,8 @@ extern "C" int pt_reg_fwd_c64(void *res, const void *u, int nz, int ny, int nx, 
 {
     pt::clear_error();
     PT_CHECK_ARG(res && u && nz > 0 && ny > 0 && nx > 0, "reg_fwd: bad arguments");
-    k_reg_fwd<<<ew_blocks((size_t)nz * ny * nx), 256, 0, (cudaStream_t)stream>>>((float2 *)res, (const float2 *)u,
-                                                                                  nz, ny, nx, s);
+    const VoxelShape v = voxel_shape(nz, ny, nx);
+    k_reg_fwd<<<v.grid, v.block, 0, (cudaStream_t)stream>>>((float2 *)res, (const float2 *)u, nz, ny, nx, s);
     PT_LAUNCHED("k_reg_fwd");
     return PT_OK;
 }
@@ -636,8 +802,8 @@ extern "C" int pt_reg_adj_c64(void *res, const void *g, int nz, int ny, int nx, 
 {
     pt::clear_error();
     PT_CHECK_ARG(res && g && nz > 0 && ny > 0 && nx > 0, "reg_adj: bad arguments");
-    k_reg_adj<<<ew_blocks((size_t)nz * ny * nx), 256, 0, (cudaStream_t)stream>>>((float2 *)res, (const float2 *)g,
-                                                                                  nz, ny, nx, s);
+    const VoxelShape v = voxel_shape(nz, ny, nx);
+    k_reg_adj<<<v.grid, v.block, 0, (cudaStream_t)stream>>>((float2 *)res, (const float2 *)g, nz, ny, nx, s);
     PT_LAUNCHED("k_reg_adj");
     return PT_OK;
 }
@@ -781,7 +947,7 @@ extern "C" int pt_ls_frames_noalloc(const void *f, const void *d, const float *d
     const int rc2 =
         launch_ls_frames((const float2 *)f, (const float2 *)d, data, dscale, n, model, gammas, J, work, st, &nblk);
     if (rc2 != PT_OK) return rc2;
-    k_finish<<<1, RT, 0, st>>>(work, (double *)out, J, nblk, 0);
+    k_finish<<<1, 32 * J, 0, st>>>(work, (double *)out, nblk, 0);
     PT_LAUNCHED("k_finish");
     return PT_OK;
 }
