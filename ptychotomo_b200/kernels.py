@@ -41,6 +41,8 @@ class Reducer:
         self.out = torch.empty(16, dtype=torch.float64, device=device)
         self.gam = torch.empty(16, dtype=torch.float64, device=device)
         self.outm = torch.empty(64, dtype=torch.float64, device=device)
+        # 2, 1, 1/2, ...: the step lengths of every line search, which start at 2 and only halve
+        self.halvings = torch.tensor([2.0 ** (1 - k) for k in range(64)], dtype=torch.float64, device=device)
 
     def _run(self, op, a, b=None, n=None, c0=0, c1=0, ncol=1, k=1):
         n = a.numel() if n is None else n
@@ -103,18 +105,36 @@ class Reducer:
     def maxangle(self, a):
         return self._run(7, a)[0]
 
-    def ls_frames(self, f, d, data, dscale, model, gammas, advance=False):
+    def _steps(self, gammas):
+        """Device address of the step lengths: inside the table of halvings, or a copy."""
+        J = len(gammas)
+        if gammas[0] > 0 and math.frexp(gammas[0])[0] == 0.5 and all(b == 0.5 * a for a, b in zip(gammas, gammas[1:])):
+            k = 2 - math.frexp(gammas[0])[1]          # gammas[0] = 2^(1 - k)
+            if 0 <= k and k + J <= len(self.halvings):
+                return self.halvings.data_ptr() + 8 * k
+        self.gam[:J].copy_(torch.tensor(gammas, dtype=torch.float64), non_blocking=False)
+        return _p(self.gam)
+
+    def ls_frames(self, f, d, data, dscale, model, gammas, advance=False, quad3=None):
         """Ptycho data term for each step length in `gammas` (<= 16).
 
         ``advance``: afterwards f <- f + gammas[0] d in place (pt_ls_frames_advance).
+        ``quad3``: a pair (a, b); quad3(a, b)'s three values follow the data
+        terms in the result, in the same read-back.
         """
         J = len(gammas)
-        self.gam[:J].copy_(torch.tensor(gammas, dtype=torch.float64), non_blocking=False)
+        k = J
+        base = self.outm.data_ptr()
+        if quad3 is not None:
+            a, b = quad3
+            check(lib().pt_reduce_c64(2, _c64(a), _c64(b), a.numel(), 0, 0, 1, _p(self.work), base + 8 * J,
+                                      current_stream()), "reduce")
+            k += 3
         fn = lib().pt_ls_frames_advance if advance else lib().pt_ls_frames
         check(fn(_c64(f), _c64(d) if d is not None else None, _p(data), float(dscale),
-                 f.numel(), model, _p(self.gam), J, _p(self.work), _p(self.out),
+                 f.numel(), model, self._steps(gammas), J, _p(self.work), base,
                  current_stream()), "ls_frames")
-        return self.out[:J].tolist()
+        return self.outm[:k].tolist()
 
     def lagr_frames(self, f, data, dscale, model):
         check(lib().pt_lagr_frames(_c64(f), _p(data), float(dscale), f.numel(), model, _p(self.work),

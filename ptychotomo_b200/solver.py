@@ -399,7 +399,6 @@ class Solver:
                 K.lincomb(d, [(-1.0, grad), (beta, d)])
             grad0 = grad
             fd = self.fwd_ptycho(d)
-            _, w_d, d2 = red.quad3(w, d)
             # minf(psi) - minf(psi + g d) = data-term decrease (per element, FP64)
             #   + rho (2 g Re<w, d> - g^2 ||d||^2)  for the penalty rho ||w - g d||^2
             npass = 0
@@ -413,7 +412,10 @@ class Solver:
                     fpsi = self.fwd_ptycho(psi)
                     advanced = None
                 npass += 1
-                vals = red.ls_frames(fpsi, fd, data, dscale, mdl, gs, advance=adv)
+                # the first pass also reads back Re<w, d> and ||d||^2
+                vals = red.ls_frames(fpsi, fd, data, dscale, mdl, gs, advance=adv, quad3=(w, d) if npass == 1 else None)
+                if npass == 1:
+                    _, w_d, d2 = vals[J:]
                 if adv:
                     advanced = gs[0]
                 chosen = None
