@@ -610,8 +610,8 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
 // The probe table (128 KB) does not stay in the 100 KB of L1 that the exchange
 // buffer leaves: rereading it cyclically hit 10 % (forward).  Its first 96 KB
 // sit in shared memory instead, the rest is read through L2.
-// 256^3, 384 angles x 169 scans: forward 3.75 -> 3.42 ms (a table of 64 KB:
-// 3.47; without the early patch loads 3.59), adjoint 4.26 -> 3.70 ms.  The
+// 256^3, 384 angles x 169 scans: forward 3.75 -> 3.34 ms (a table of 64 KB
+// costs 0.05, later patch loads 0.17 more), adjoint 4.26 -> 3.70 ms.  The
 // adjoint keeps 32 KB only: with 96 KB in the table the L1 left for loads in
 // flight is too small (4.00 ms; 16 KB 3.83, 48 KB 3.75).  The arithmetic and
 // the exchange alone take 2.1 ms of the forward, the exchange 1.1 ms.
@@ -751,6 +751,16 @@ __global__ void __launch_bounds__(512, 1)
     auto source = [&](int fid, int sx, int sy, int px) {
         return psi + ((size_t)(fid / nscan) * nz + sy) * n + sx + px;
     };
+    // the thread's probe values below the table, rows rt0 + 4 c + 8 m, m >= KT,
+    // the same for every frame: kept in registers (3.42 -> 3.34 ms)
+    constexpr int KT = P128_FTAB / 8192;
+    float2 pk[2][16 - KT];
+    if (FULL && !SUB) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int m = KT; m < 16; ++m) pk[c][m - KT] = __ldg(&prbT[(rt0 + 4 * c + 8 * m) * 128 + q0]);
+    }
     int fid = blockIdx.x;
     int stx = corner[2 * fid], sty = corner[2 * fid + 1];
     float2 pre[16];
@@ -773,19 +783,20 @@ __global__ void __launch_bounds__(512, 1)
             const float2 *src = source(fid, stx, sty, px);
             const float2 *pr = (SUB ? prbT + (size_t)sid[fid] * P * P : prbT) + px;  // sub-pixel: the frame's shifted probe
             const float2 *ps = tab + px;
-            auto probe = [&](int m, int py) {
+            auto probe = [&](int c, int m, int py) {
+                if (FULL && !SUB && m >= KT) return pk[c][m - KT];
                 if (!FULL && !(px >= 0 && px < P && py >= 0 && py < P)) return czero();
-                if (!SUB && (FULL ? m < P128_FTAB / 8192 : py < rows)) return ps[py * PS];
+                if (!SUB && (FULL || py < rows)) return ps[py * PS];
                 return __ldg(&pr[py * PS]);
             };
             float2 v[16];
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = patch(src, px, rt + 4 + 8 * m - off, off);
 #pragma unroll
-            for (int m = 0; m < 16; ++m) pre[m] = cmul(probe(m, rt + 8 * m - off), pre[m]);
+            for (int m = 0; m < 16; ++m) pre[m] = cmul(probe(0, m, rt + 8 * m - off), pre[m]);
             f128_r1<-1, false>(pre, ex, q, rt, tw4);
 #pragma unroll
-            for (int m = 0; m < 16; ++m) v[m] = cmul(probe(m, rt + 4 + 8 * m - off), v[m]);
+            for (int m = 0; m < 16; ++m) v[m] = cmul(probe(1, m, rt + 4 + 8 * m - off), v[m]);
             f128_r1<-1, false>(v, ex, q, rt + 4, tw4);
             __syncthreads();
             f128_r2<-1, false>(ex, fresh(threadIdx.x), scale * phase[fid], w128);
