@@ -1058,6 +1058,7 @@ struct pt_ptycho {
     int device = -1, nsm = 148;
     bool ready = false;
     float c = 0.f;
+    char *tables = nullptr;   // one allocation: tw, tw128, prb, prbT, prbT2, angles, phase, corner, frac
     float2 *tw = nullptr, *prb = nullptr, *prbT = nullptr, *phase = nullptr, *partial = nullptr;
     float4 *tw128 = nullptr;  // det = 128: the twiddles in twiddle16's pair layout
     int *corner = nullptr;
@@ -1379,8 +1380,7 @@ bool set_parts(pt_ptycho *h, int parts)
 
 void ptycho_free(pt_ptycho *h)
 {
-    void *bufs[] = {h->tw,     h->tw128,  h->prb,  h->prbT, h->phase, h->partial, h->corner,
-                    h->prbT2,  h->prb_part, h->frac, h->prbS, h->ones, h->sid, h->angles};
+    void *bufs[] = {h->tables, h->partial, h->prb_part, h->prbS, h->ones, h->sid};
     for (void *p : bufs)
         if (p) cudaFree(p);
 }
@@ -1551,16 +1551,28 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
     } else if (detx >= 16) {
         parts = choose_parts(*h, nullptr);
     }
-    bool ok = cudaMalloc((void **)&h->tw, detx * sizeof(float2)) == cudaSuccess &&
-              cudaMalloc((void **)&h->tw128, 64 * sizeof(float4)) == cudaSuccess &&
-              cudaMalloc((void **)&h->prb, nprb * nprb * sizeof(float2)) == cudaSuccess &&
-              cudaMalloc((void **)&h->prbT, nprb * nprb * sizeof(float2)) == cudaSuccess &&
-              set_parts(h, parts) &&
-              cudaMalloc((void **)&h->angles, ntheta * sizeof(int)) == cudaSuccess &&
-              cudaMalloc((void **)&h->phase, ntheta * nscan * sizeof(float2)) == cudaSuccess &&
-              cudaMalloc((void **)&h->corner, 2 * ntheta * nscan * sizeof(int)) == cudaSuccess &&
-              cudaMalloc((void **)&h->frac, 2 * ntheta * nscan * sizeof(float)) == cudaSuccess &&
-              cudaMalloc((void **)&h->prbT2, nprb * nprb * sizeof(float2)) == cudaSuccess;
+    // the small tables are cuts of one allocation, each on a 256-byte boundary
+    const size_t P2 = nprb * nprb, nf = ntheta * nscan;
+    size_t used = 0;
+    auto cuts = [&](auto &&cut) {
+        used = 0;
+        cut(h->tw, detx);
+        cut(h->tw128, (size_t)64);
+        cut(h->prb, P2);
+        cut(h->prbT, P2);
+        cut(h->prbT2, P2);
+        cut(h->angles, ntheta);
+        cut(h->phase, nf);
+        cut(h->corner, 2 * nf);
+        cut(h->frac, 2 * nf);
+    };
+    auto place = [&](auto *&p, size_t count) {
+        if (h->tables) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(h->tables + used);
+        used += (count * sizeof(*p) + 255) / 256 * 256;
+    };
+    cuts(place);
+    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && set_parts(h, parts);
+    if (ok) cuts(place);
     // probe adjoint: one partial per frame in flight
     const Residency res = residency((int)detx);
     const size_t inflight = (size_t)nsm * res.probe_blocks;

@@ -102,7 +102,7 @@ constexpr int WKB = 8, WGAUSS = 9;   // cells per axis: Kaiser-Bessel (default),
 template <int W>
 constexpr int win_left() { return W == WKB ? WKB / 2 - 1 : WGAUSS / 2; }   // first cell: floor(2N x) - win_left
 // the rms error is flat about its minimum: 3.9e-8 to 4.9e-8 from 2.30 W to 2.36 W
-constexpr double KB_BETA = 2.36 * WKB;
+constexpr double KB_BETA = 2.35 * WKB;
 
 // wtab[p][0..W-1], [W..2W-1]: the window's values in x and y at the W cells
 // of point p's window (first cell floor(2N x) - win_left).  Kaiser-Bessel
@@ -126,7 +126,8 @@ __global__ void k_window(const float *__restrict__ xt, const float *__restrict__
     }
 }
 
-// The forward gather's record of a point, in visiting order (six float4):
+// The forward gather's record of a point, in visiting order (perm; null: in
+// point order) (six float4):
 // floats 0..9 the x weights of the five column pairs that cover the window (0
 // for the columns outside it), 10..18 the y weights times the sample's scale
 // pre, 20 the point's index, 21 and 22 its
@@ -141,7 +142,7 @@ __global__ void k_point_records(const int *__restrict__ perm, const int *__restr
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npts) return;
-    const int p = perm[i];
+    const int p = perm ? perm[i] : i;
     const int ox = org[2 * p], oy = org[2 * p + 1], odd = ox & 1;
     const float *wx = wtab + (size_t)p * 2 * W, *wy = wx + W;
     float *r = rec + (size_t)i * REC4 * 4;
@@ -534,6 +535,56 @@ __global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
     }
 }
 
+// K3a and K3b in one launch for short lines: a block gathers the N points of
+// one angle through L1 into shared memory and transforms them (the same sums
+// and rounds as k_fwd_gather_pts and k_fwd_lines).  rec is in point order.
+// One launch and one pass over the lines buffer less: 32 wide, 9 slices 24.8 ->
+// 20.9 us (bound by the launches), 64^3 61 -> 58 us.  From 128 wide the tiles in
+// shared memory win.
+constexpr int FUSED_N = 96;   // longest line (64 wide)
+template <int N, int W>
+__global__ void __launch_bounds__(GPB *ZC, 4)
+    k_fwd_gather_lines(const float2 *__restrict__ fg, size_t set, const float4 *__restrict__ rec,
+                       float2 *__restrict__ out, int nz, int z0, float scale, const float4 *__restrict__ tw)
+{
+    using E = ptfft::Exchange<N, ZC>;
+    constexpr int G = 2 * N, PS = G / 2 + GH_PAIRS, n = 2 * N / 3, c0 = N / 6, R1 = E::R1, R2 = E::R2;
+    static_assert(W - 1 <= GH_ROWS && E::NT <= GPB * ZC, "the halo covers the window, the block the transform");
+    __shared__ float2 line[N * ZC], sm[E::BYTES / sizeof(float2)];
+    const int th = blockIdx.x;
+    const int q = threadIdx.x % ZC, b = threadIdx.x / ZC;
+    const float4 *g4 = reinterpret_cast<const float4 *>(fg + blockIdx.y * set) + q;
+    for (int k = b; k < N; k += GPB) {
+        const float4 *r = rec + ((size_t)th * N + k) * REC4;
+        const float4 o = __ldg(&r[5]);
+        line[k * ZC + q] = window_sum<W>(g4 + ((size_t)__float_as_int(o.y) * PS + __float_as_int(o.z)) * ZC,
+                                         (size_t)PS * ZC, r, [](const float4 *p) { return __ldg(p); });
+    }
+    __syncthreads();
+    if (b < R2) {
+        float2 v[R1];
+#pragma unroll
+        for (int i1 = 0; i1 < R1; ++i1) v[i1] = line[(i1 * R2 + b) * ZC + q];
+        ptfft::Dft<R1, +1, true>::run(v);
+        ptfft::twiddle_pairs<R1, R2>(v, b, tw);
+        E::put(sm, v, b, q);
+    }
+    __syncthreads();
+    const int z = z0 + blockIdx.y * ZC + q;
+    if (b < R1 && z < nz) {
+        float2 w[R2];
+        E::get(sm, w, b, q);
+        ptfft::Dft<R2, +1, true>::run(w);
+        float2 *dst = out + ((size_t)th * nz + z) * n;
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) {
+            if (R1 * k2 + R1 <= c0 || R1 * k2 >= c0 + n) continue;   // wholly cropped
+            const int j = b + R1 * k2 - c0;
+            if (j >= 0 && j < n) dst[j] = scale * w[k2];
+        }
+    }
+}
+
 // ---- A1: pad (kernels.cuh:189-206) + fftshift1c/FFT/fftshift1c -------------
 // grid (ntheta, nzp / ZC); writes lines[(theta*N + k) * nzp + z].  ZP: the
 // exact adjoint's zero padding (the adjoint of the forward's crop) instead
@@ -591,9 +642,9 @@ __global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
 constexpr int ZQ = 16;
 constexpr int CG = 4;  // cells per group
 template <int G>
-constexpr int col_threads() { return G >= 1024 ? 1024 : G >= 384 ? 512 : 256; }
+constexpr int col_threads() { return G >= 1024 ? 1024 : G >= 96 ? 512 : 256; }   // 64^3: 40 us with 256, 36 with 512
 template <int G, bool ALL = false>
-__global__ void __launch_bounds__(col_threads<G>(), (G >= 1024 ? 1 : G >= 384 ? 2 : 4))
+__global__ void __launch_bounds__(col_threads<G>(), (G >= 1024 ? 1 : G >= 96 ? 2 : 4))
     k_adj_colgather(const float2 *__restrict__ lines, float2 *__restrict__ rbuf, const int *__restrict__ goff,
                     const int *__restrict__ gpt, const float4 *__restrict__ gw, const int *__restrict__ col_order,
                     int nzp, const float2 *__restrict__ tw1, const float2 *__restrict__ tw2)
@@ -860,6 +911,7 @@ struct pt_radon {
     float *wtab = nullptr;    // the window's values, [point][x: W, y: W]
     int *perm = nullptr;      // the forward gather's point order (grid tiles)
     float4 *rec = nullptr;    // each point's gather record, in that order
+    float4 *rec_pt = nullptr; // the records in point order (N <= FUSED_N)
     int4 *chunks = nullptr;   // the tiled gather's blocks: (tile row, tile column, first, count)
     int nchunks = 0, chunks_cap = 0;
     int gather = 2;           // 0: gather through L1 (k_fwd_gather_pts), 1: shared-memory tiles, 2: TMA-staged tiles
@@ -1017,6 +1069,14 @@ int run_fwd(pt_radon *h, float2 *g, const float2 *f, float scale, cudaStream_t s
         PT_LAUNCHED("k_fwd_rows");
         k_fwd_cols<G><<<dim3(G / CK, ZC / ZH, cnt), EG::NT, EG::BYTES, s>>>(rb, fg, stride, h->tw_fwd);
         PT_LAUNCHED("k_fwd_cols");
+        if constexpr (N <= FUSED_N) {
+            if (h->gather == 0) {
+                k_fwd_gather_lines<N, W><<<dim3(h->ntheta, cnt), GPB * ZC, 0, s>>>(fg, stride, h->rec_pt, g, h->nz, z0,
+                                                                                   scale, h->tw_inv_line);
+                PT_LAUNCHED("k_fwd_gather_lines");
+                continue;
+            }
+        }
         if (h->gather == 2) {
             k_fwd_gather_tma<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tma_smem<N, W>(), s>>>(
                 h->tmap, k, ln, h->rec, h->chunks, npts, h->tma_err);
@@ -1275,6 +1335,7 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
         cut(h->wtab, 2 * (size_t)h->W * npts);
         cut(h->perm, npts);
         cut(h->rec, REC4 * npts);
+        if (N <= FUSED_N) cut(h->rec_pt, REC4 * npts);
         cut(h->deap, N * N);
         if (h->W == WKB) cut(h->inv1, N);
         cut(h->goff, (size_t)G * (G / CG) + 1);
@@ -1289,12 +1350,13 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
     });
     if (rc == PT_OK && cudaMemset(h->tma_err, 0, sizeof(int)) == cudaSuccess)
         h->tma_ok = encode_grid_maps(h);   // gather 2 is offered only if every map encodes
-    // default variant: two pipelines of two chunks per launch, TMA-staged tiles.
+    // default variant: two pipelines of two chunks per launch, TMA-staged tiles
+    // (up to 64 wide the gather and the lines in one launch).
     // Against four pipelines of one (us): 32 wide, 9 slices 25 and 42; 64^3 55
     // and 123; 128 x 84 slices 140 and 144; 128^3 231 and 215; 256^3 1437 and
     // 1443.  One pipeline of four is slower from 64^3 up (60, 148, 237, 1598)
     h->streams = 2;
-    h->gather = h->tma_ok ? 2 : 1;
+    h->gather = N <= FUSED_N ? 0 : h->tma_ok ? 2 : 1;
     if (rc == PT_OK && cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess) rc = PT_ERR_CUDA;
     for (int k = 0; k < RSETS - 1 && rc == PT_OK; ++k)
         if (cudaStreamCreateWithFlags(&h->side[k], cudaStreamNonBlocking) != cudaSuccess ||
@@ -1404,12 +1466,16 @@ extern "C" int pt_radon_setobj(pt_radon *h, const float *theta, void *stream)
         std::stable_sort(perm.begin(), perm.end(), [&](int i, int j) { return key(i) < key(j); });
         PT_CUDA(cudaMemcpyAsync(h->perm, perm.data(), npts * sizeof(int), cudaMemcpyHostToDevice, st));
         const unsigned blocks = (unsigned)((npts + 255) / 256);
-        if (W == WKB)
-            k_point_records<WKB><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts,
-                                                         radon_pre(h));
-        else
-            k_point_records<WGAUSS><<<blocks, 256, 0, st>>>(h->perm, h->org, h->wtab, (float *)h->rec, (int)npts,
-                                                            radon_pre(h));
+        auto records = [&](const int *order, float4 *rec) {
+            if (W == WKB)
+                k_point_records<WKB><<<blocks, 256, 0, st>>>(order, h->org, h->wtab, (float *)rec, (int)npts,
+                                                             radon_pre(h));
+            else
+                k_point_records<WGAUSS><<<blocks, 256, 0, st>>>(order, h->org, h->wtab, (float *)rec, (int)npts,
+                                                                radon_pre(h));
+        };
+        records(h->perm, h->rec);
+        if (h->rec_pt) records(nullptr, h->rec_pt);
         PT_LAUNCHED("k_point_records");
         // the tiled gather's blocks: runs of one tile in perm order, at most tile_points points each
         std::vector<int4> chunks;
