@@ -258,9 +258,16 @@ struct FR {
     static constexpr int R2C = 256 / NT;                 // (k1, qb) pairs per thread
     static constexpr int BPS = 768 / BLOCK;              // resident blocks per SM at 80 registers a thread
     static constexpr int BPSP = 512 / BLOCK;             // probe adjoint: 128 registers
-    // frames per trip: two for a probe smaller than the detector
-    static constexpr int nf(bool full) { return full || FPB > 1 ? 1 : 2; }
-    static constexpr size_t smem(bool full) { return (size_t)FPB * nf(full) * DET * DET * sizeof(float2); }
+    // Frames per trip, three barriers for both: two pay where a trip is long,
+    // at 64 x 64 with a probe smaller than the detector.  Forward, where the
+    // window lines of both fit the threads (P <= DET / 2) and every resident
+    // block has two frames (280 x 15 scans, P 24: 53 -> 47 us; P 33 to 52
+    // gain nothing, few frames lose 2 us); adjoint with the residual (70 x 341
+    // scans, P 33: 468 -> 408 us; without it 178 x 66 scans, P 26: 137 ->
+    // 147 us).  32 x 32 frames lose in all forms (5 x 340 scans, P 29:
+    // forward 10 -> 14 us, adjoint 57 -> 79 us).
+    static constexpr int nf_adj(bool full, bool resid) { return DET == 64 && !full && resid ? 2 : 1; }
+    static constexpr size_t smem(int nf) { return (size_t)FPB * nf * DET * DET * sizeof(float2); }
     static_assert(DET * RT == NT, "R1 and R3 give every thread one line of 16");
 };
 
@@ -377,16 +384,14 @@ __device__ __forceinline__ void fr_line(int t, int PW, int &px, int &r)
     r = l / PW;      // valid if below RT
 }
 
-// Forward, grid-stride over frames (two consecutive ones per trip for a probe
-// smaller than the detector: three barriers for both).
-template <int DET, bool FULL, bool SUB = false>
+// Forward, grid-stride over frames, NF consecutive ones per trip.
+template <int DET, bool FULL, bool SUB = false, int NF = 1>
 __global__ void __launch_bounds__(FR<DET>::BLOCK, FR<DET>::BPS)
     k_ptycho_fwd(const float2 *__restrict__ psi, float2 *__restrict__ g, const int *__restrict__ corner,
                  const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan,
                  int nframes, int P, float scale, const float2 *__restrict__ w, const int *__restrict__ sid = nullptr)
 {
     using F = FR<DET>;
-    constexpr int NF = F::nf(FULL);
     extern __shared__ float4 sm4[];
     const int t0 = threadIdx.x % F::NT, sub = threadIdx.x / F::NT;
     float2 *ex = reinterpret_cast<float2 *>(sm4) + sub * DET * DET;
@@ -448,8 +453,7 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, FR<DET>::BPS)
 }
 
 // Object adjoint: grid (parts, ntheta), block (part, angles[y]) owns slab
-// dst[angle][part] and walks scans part, part + parts, ... (two per trip for a
-// probe smaller than the detector).  PROBE (the adjoint with respect to the
+// dst[angle][part] and walks scans part, part + parts, ...  PROBE (the adjoint with respect to the
 // probe): grid (blocks, 1), block b walks frames b, b + gridDim.x, ... <
 // nframes and sums conj(psi patch) x frame into its P x P partial dst[b] (one
 // per frame of the block); each element belongs to one thread, which keeps it
@@ -463,7 +467,7 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
                  const float2 *psi = nullptr, int nframes = 0)
 {
     using F = FR<DET>;
-    constexpr int NF = PROBE ? 1 : F::nf(FULL);
+    constexpr int NF = PROBE ? 1 : F::nf_adj(FULL, RESID != 0);
     extern __shared__ float4 sm4[];
     const int t0 = threadIdx.x % F::NT, sub = threadIdx.x / F::NT;
     float2 *ex = reinterpret_cast<float2 *>(sm4) + sub * DET * DET;
@@ -1114,14 +1118,13 @@ int ptycho_attrs()
         PT_ATTR_ADJ(1)
         PT_ATTR_ADJ(2)
 #undef PT_ATTR_ADJ
-    } else if constexpr (FR<DET>::smem(false) > 48 * 1024) {
-        constexpr size_t s = FR<DET>::smem(false);
-        PT_ATTR((k_ptycho_fwd<DET, false>), s);
-        PT_ATTR((k_ptycho_fwd<DET, false, true>), s);
-        PT_ATTR((k_ptycho_adj<DET, false, 0>), s);
+    } else if constexpr (DET == 64) {   // two frames per trip
+        constexpr size_t s = FR<DET>::smem(2);
+        static_assert(FR<32>::smem(2) <= 48 * 1024, "no attribute needed");
+        PT_ATTR((k_ptycho_fwd<DET, false, false, 2>), s);
+        PT_ATTR((k_ptycho_fwd<DET, false, true, 2>), s);
         PT_ATTR((k_ptycho_adj<DET, false, 1>), s);
         PT_ATTR((k_ptycho_adj<DET, false, 2>), s);
-        PT_ATTR((k_ptycho_adj<DET, false, 0, true>), s);
         PT_ATTR((k_ptycho_adj<DET, false, 1, true>), s);
         PT_ATTR((k_ptycho_adj<DET, false, 2, true>), s);
     }
@@ -1163,7 +1166,8 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, h->angles, h->shift_ids());
             else
-                k_ptycho_adj<DET, FU, RESID, S><<<grid, FR<DET>::BLOCK, FR<DET>::smem(FU), st>>>(
+                k_ptycho_adj<DET, FU, RESID, S>
+                    <<<grid, FR<DET>::BLOCK, FR<DET>::smem(FR<DET>::nf_adj(FU, RESID != 0)), st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw,
                     data, dscale, h->angles, h->shift_ids());
         };
@@ -1203,11 +1207,21 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
                     h->tw128, h->tw, h->shift_ids());
             } else {
                 using F = FR<DET>;
-                const int per = F::FPB * F::nf(FU);
-                const int grid = std::min((nframes + per - 1) / per, h->nsm * F::BPS);
-                k_ptycho_fwd<DET, FU, S><<<grid, F::BLOCK, F::smem(FU), st>>>(in, out, h->corner, h->phase_tab(),
-                                                                         h->probe_tab(), h->nz, h->n, h->nscan,
-                                                                         nframes, h->P, scale, h->tw, h->shift_ids());
+                auto trips = [&](auto frames) {
+                    constexpr int NF = decltype(frames)::value;
+                    const int per = F::FPB * NF, grid = std::min((nframes + per - 1) / per, h->nsm * F::BPS);
+                    k_ptycho_fwd<DET, FU, S, NF><<<grid, F::BLOCK, F::smem(NF), st>>>(
+                        in, out, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, nframes, h->P,
+                        scale, h->tw, h->shift_ids());
+                };
+                if constexpr (DET == 64 && !FU) {
+                    if (2 * h->P <= DET && nframes >= 2 * h->nsm * F::BPS)
+                        trips(std::integral_constant<int, 2>{});
+                    else
+                        trips(std::integral_constant<int, 1>{});
+                } else {
+                    trips(std::integral_constant<int, 1>{});
+                }
             }
         };
         by_kind(h, go);
@@ -1262,7 +1276,7 @@ int probe_adj_launch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 
                     h->tw, data, dscale, nullptr, nullptr, psi, nframes);
             else
                 k_ptycho_adj<DET, FU, RESID, false, true>
-                    <<<h->prb_blocks / FR<DET>::FPB, FR<DET>::BLOCK, FR<DET>::smem(true), st>>>(
+                    <<<h->prb_blocks / FR<DET>::FPB, FR<DET>::BLOCK, FR<DET>::smem(1), st>>>(
                         in, h->prb_part, h->corner, h->phase, h->prbT, h->nz, h->n, h->nscan, h->P, scale, h->tw, data,
                         dscale, nullptr, nullptr, psi, nframes);
         };
@@ -1293,60 +1307,95 @@ int probe_adj_dispatch(pt_ptycho *h, float2 *gprb, const float2 *in, const float
 }
 
 // Blocks of the probe adjoint that an SM holds, and the frames a block works on at a time.
+// Times of the adjoint's parts, per cell of an object slab where they scale
+// with it (a thread's and an SM's share of the clear, the sum of the parts).
+struct SplitCost {
+    double lone, frame, clear, clear_sm, sum, sum_cell;
+};
 struct Residency {
-    int probe_blocks, frames;
+    int probe_blocks, frames, blocks, threads;
+    SplitCost cost;
 };
 Residency residency(int det)
 {
     switch (det) {
-    case 16: return {FR<16>::BPSP, FR<16>::FPB};
-    case 32: return {FR<32>::BPSP, FR<32>::FPB};
-    case 64: return {FR<64>::BPSP, FR<64>::FPB};
-    default: return {1, 1};
+    case 16: return {FR<16>::BPSP, FR<16>::FPB, FR<16>::BPS, FR<16>::BLOCK, {2.03, 0.081, 2.7e-3, 2.2e-4, 2.9, 1.7e-6}};
+    case 32: return {FR<32>::BPSP, FR<32>::FPB, FR<32>::BPS, FR<32>::BLOCK, {2.21, 0.30, 5.3e-4, 1.9e-4, 5.9, 1.5e-6}};
+    case 64: return {FR<64>::BPSP, FR<64>::FPB, FR<64>::BPS, FR<64>::BLOCK, {3.05, 1.21, 2.0e-3, 1.15e-4, 5.5, 1.8e-6}};
+    // a unit is a frame; a block alone or with neighbours clears a slab's worth
+    // of frames at 0.375 of one, and once more for the sum
+    default: return {1, 1, 1, 512, {1, 1, 0, 0.375 / (128 * 128), 0, 0}};
     }
 }
 
 // The adjoint's split of an angle's scans over blocks: the number of parts with
-// the earliest end of the last block.  A block works off its scans one after
-// the other, LONE units each (the time of one frame on a full SM; smaller
-// detectors run three blocks per SM, and a block alone is about as slow as
-// with two neighbours), and clears its slab; with more than one part the
-// reduction reads it again (SLAB units per frame's worth of it and pass).
+// the earliest end.  In microseconds, with R the blocks on an SM:
+//   a block    clears its slab, at the SM's store rate, and takes trips of
+//              max(lone, R frames) each: a few blocks wait on latency, many on
+//              the SM;
+//   the sum    of more than one part reads every slab once, after a launch.
 // counts: the scans of each angle that are not skipped, in launch order, where
-// they differ: the blocks are then placed on the SMs one by one; else every
-// SM gets the same rounds of equal blocks.
-// 45 angles with 100 to 400 scans of a 128 x 128 detector: 6 parts and the
-// angles with most scans first instead of 3 parts in angle order, Gaussian
-// gradient 1.48 -> 1.09 ms, Poisson 1.43 -> 0.90 ms.
+// they differ: the blocks are then placed on the SMs one by one; else whole
+// waves of equal blocks and what is left.
+// More than 16 parts are tried only while all blocks run at once.
+// The constants are the best over 52 calls of 16- to 64-pixel detectors timed at
+// every split (4 to 351 angles, 10 to 378 scans, objects of 33 to 254): the
+// chosen split is 1 to 5 % from the best one on average.  16 x 16 frames run 24
+// blocks per SM and 32 x 32 frames 12; counting three as for 64 x 64 took 4 x
+// 325 scans from 39 to 51 us (33 us now) and 195 x 241 to 157 us (77 us now);
+// clears counted too low took 48 x 14 scans on a 251 x 254 object from 57 to
+// 96 us (45 us now).
+// Det 128, one block per SM, in units of a frame: 45 angles with 100 to 400 scans:
+// 6 parts and the angles with most scans first instead of 3 parts in angle
+// order, Gaussian gradient 1.48 -> 1.09 ms, Poisson 1.43 -> 0.90 ms.
 int choose_parts(const pt_ptycho &h, const std::vector<int> *counts)
 {
-    const bool one = h.det == 128;
-    const int frames = residency(h.det).frames;
-    const size_t slots = (size_t)h.nsm * (one ? 1 : 3);
-    const double LONE = one ? 1.0 : 3.0, SLAB = (one ? 0.375 : 0.5) * h.nz * h.n / ((double)h.det * h.det);
+    const Residency res = residency(h.det);
+    const double cells = (double)h.nz * h.n;
+    const size_t slots = (size_t)h.nsm * res.blocks;
+    const SplitCost &c = res.cost;
     int best_p = 1;
     double best = 1e300;
-    for (int p = 1; p <= std::min(h.nscan, 16); ++p) {
-        const double slab = SLAB * (p > 1 ? 2 : 1);
-        auto block = [&](int scans) { return std::ceil((double)scans / (p * frames)) * frames * LONE + slab; };
-        double cost = 0;
+    auto time = [&](int p) {
+        const size_t blocks = (size_t)h.ntheta * p;
+        const int passes = h.det == 128 && p > 1 ? 2 : 1;
+        auto block = [&](int scans, size_t sharing) {   // sharing: blocks on the SM
+            const double trips = std::ceil((double)scans / (p * res.frames));
+            return std::max(c.clear * cells / res.threads, passes * sharing * c.clear_sm * cells) +
+                   trips * std::max(c.lone, (double)sharing * res.frames * c.frame);
+        };
+        auto sharing = [&](size_t n) { return (std::min(n, slots) + h.nsm - 1) / h.nsm; };
+        const double sum = p > 1 ? c.sum + c.sum_cell * cells * h.ntheta * (p + 1) : 0;
+        double end = 0;
         if (!counts) {
-            cost = std::ceil((double)h.ntheta * p / slots) * block(h.nscan);
+            const size_t waves = blocks / slots, rest = blocks % slots;
+            end = waves * block(h.nscan, res.blocks) + (rest ? block(h.nscan, sharing(rest)) : 0);
+        } else if (blocks <= slots) {   // all at once: the one with most scans ends last
+            end = block(counts->front(), sharing(blocks));
         } else {
+            const size_t R = sharing(blocks);
+            double all = 0;
+            for (int n : *counts) all += p * block(n, R);
+            if (all / slots + sum >= best) return 1e300;   // no placement ends early enough
             std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
-            for (int c : *counts)
+            for (int n : *counts)
                 for (int k = 0; k < p; ++k) {
                     double start = 0;
                     if (ends.size() == slots) {
                         start = ends.top();
                         ends.pop();
                     }
-                    ends.push(start + block(c));
-                    cost = std::max(cost, start + block(c));
+                    ends.push(start + block(n, R));
+                    end = std::max(end, start + block(n, R));
                 }
         }
-        if (cost < best - 1e-9) {
-            best = cost;
+        return end + sum;
+    };
+    for (int p : {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 24, 32, 48, 64}) {
+        if (p > h.nscan || (p > 16 && (h.det == 128 || (size_t)h.ntheta * p > slots))) break;
+        const double end = time(p);
+        if (end < best - 1e-9) {
+            best = end;
             best_p = p;
         }
     }
