@@ -592,6 +592,134 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
     }
 }
 
+// ---- det 16 and 32, few frames: the adjoint with four threads per line -------
+// Where few blocks are in flight, a frame's latency counts, not the SM's
+// instruction slots: k_ptycho_adj takes 16 values per thread (16 or 64 threads
+// per frame), this kernel 4 or 8 (64 or 128 threads), row transforms, a
+// transpose through shared memory, column transforms.  choose_split compares
+// their modelled times.  16 x 16 frames, adjoint: 9 x 74 scans 18.5 -> 14.4 us,
+// 65 x 14 scans on a 145 x 152 object 29 -> 20 us (more threads to clear its
+// slabs); but 224 x 146 scans take 94 us here and 66 us there.
+template <int DET>
+struct PF {
+    static constexpr int N2 = 4;                           // threads per line
+    static constexpr int N1 = DET / N2;                    // points per thread
+    static constexpr int KPT = N1 / N2;                    // k1 values per thread after the exchange
+    static constexpr int NT = DET * N2;                    // threads per block
+    static constexpr int P = DET + 8;                      // frame pitch (P = 8 mod 16)
+    static constexpr size_t SMEM = (size_t)(DET * P + DET) * sizeof(float2);
+};
+
+// frame swizzle: row r, column c live at r * P + (c ^ fswz(r))
+template <int DET>
+__device__ __forceinline__ int fswz(int r)
+{
+    return ((r / PF<DET>::KPT) % PF<DET>::N2) * 2;
+}
+
+// DFT of one line held as v[m] = x[t + N2 m] by the N2 threads t of a group.
+// On return v[j N2 + k2] = X[t KPT + j + N1 k2].  `sc` is the group's
+// scratch (DET + 1 complex), `tws` the table exp(-2 pi i m / DET).
+template <int DET, int DIR>
+__device__ __forceinline__ void line_dft(float2 (&v)[PF<DET>::N1], int t, float2 *sc, const float2 *tws)
+{
+    using F = PF<DET>;
+    ptfft::Dft<F::N1, DIR>::run(v);
+#pragma unroll
+    for (int k1 = 1; k1 < F::N1; ++k1) {
+        float2 w = tws[t * k1];
+        if (DIR > 0) w.y = -w.y;
+        v[k1] = cmul(v[k1], w);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k1 = 0; k1 < F::N1; ++k1) sc[t * F::N1 + ((k1 + t * F::KPT) % F::N1)] = v[k1];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < F::KPT; ++j) {
+        float2 u[F::N2];
+        const int k1 = t * F::KPT + j;
+#pragma unroll
+        for (int n2 = 0; n2 < F::N2; ++n2) u[n2] = sc[n2 * F::N1 + ((k1 + n2 * F::KPT) % F::N1)];
+        ptfft::Dft<F::N2, DIR>::run(u);
+#pragma unroll
+        for (int k2 = 0; k2 < F::N2; ++k2) v[j * F::N2 + k2] = u[k2];
+    }
+}
+
+// grid (parts, ntheta): block (part, angles[y]) owns slab dst[angle][part]
+template <int DET, int RESID, bool SUB = false>
+__global__ void __launch_bounds__(PF<DET>::NT, 1)
+    k_ptycho_adj_few(const float2 *__restrict__ g, float2 *__restrict__ dst, const int *__restrict__ corner,
+                 const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan,
+                 int P, float scale, const float2 *__restrict__ tw, const float *__restrict__ data, float dscale,
+                 const int *__restrict__ angles, const int *__restrict__ sid)
+{
+    using F = PF<DET>;
+    extern __shared__ float2 sm[];
+    float2 *fr = sm;
+    float2 *tws = sm + DET * F::P;
+    const int part = blockIdx.x, parts = gridDim.x, th = angles[blockIdx.y];
+    float2 *slab = dst + ((size_t)th * parts + part) * nz * n;
+    for (int i = threadIdx.x; i < DET; i += F::NT) tws[i] = tw[i];
+    for (int e = threadIdx.x; e < nz * n; e += F::NT) slab[e] = czero();
+    const int t = threadIdx.x % F::N2, grp = threadIdx.x / F::N2;
+    float2 *sc = fr + grp * (DET + 1);
+    const int off = (DET - P) / 2;
+    __syncthreads();
+    for (int s = part; s < nscan; s += parts) {
+        const int fid = th * nscan + s;
+        const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
+        if (stx < 0 || sty < 0) continue;
+        const float2 ph = phase[fid];
+        const float2 *pr = SUB ? prbT + (size_t)sid[fid] * P * P : prbT;
+        const float2 *in = g + (size_t)fid * DET * DET;
+        float2 v[F::N1];
+        // along the detector row: line kx = grp, points ky = t + N2 m (contiguous)
+#pragma unroll
+        for (int m = 0; m < F::N1; ++m) {
+            const int e = grp * DET + t + F::N2 * m;
+            v[m] = scale * cmulc(ph, resid<RESID>(__ldg(&in[e]), data, (size_t)fid * DET * DET + e, dscale));
+        }
+        line_dft<DET, +1>(v, t, sc, tws);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < F::KPT; ++j)
+#pragma unroll
+            for (int k2 = 0; k2 < F::N2; ++k2) {
+                const int iy = t * F::KPT + j + F::N1 * k2;
+                fr[iy * F::P + (grp ^ fswz<DET>(iy))] = v[j * F::N2 + k2];
+            }
+        __syncthreads();
+        const int sw = fswz<DET>(grp);
+#pragma unroll
+        for (int m = 0; m < F::N1; ++m) v[m] = fr[grp * F::P + ((t + F::N2 * m) ^ sw)];
+        __syncthreads();
+        line_dft<DET, +1>(v, t, sc, tws);
+        const int py = grp - off;
+        if (py >= 0 && py < P) {
+            float2 *row = slab + (size_t)(sty + py) * n + stx;
+            float2 cur[F::N1];
+#pragma unroll
+            for (int k2 = 0; k2 < F::N2; ++k2)
+#pragma unroll
+                for (int j = 0; j < F::KPT; ++j) {
+                    const int px = t * F::KPT + j + F::N1 * k2 - off;
+                    cur[j * F::N2 + k2] = (px >= 0 && px < P) ? row[px] : czero();
+                }
+#pragma unroll
+            for (int k2 = 0; k2 < F::N2; ++k2)
+#pragma unroll
+                for (int j = 0; j < F::KPT; ++j) {
+                    const int px = t * F::KPT + j + F::N1 * k2 - off;
+                    if (px >= 0 && px < P)
+                        row[px] = cur[j * F::N2 + k2] + cmulc(__ldg(&pr[py * P + px]), v[j * F::N2 + k2]);
+                }
+        }
+        __syncthreads();
+    }
+}
+
 // ---- det = 128 ---------------------------------------------------------
 // The same three rounds for a 128 x 128 frame, 32 values per thread and one
 // 512-thread block per SM (the frame's exchange buffer takes 128 KB):
@@ -1069,6 +1197,7 @@ struct pt_ptycho {
     // the object adjoint's order of angles: most scans first (as uploaded: order)
     int *angles = nullptr;
     std::vector<int> order;
+    bool few = false;           // det 16, 32: k_ptycho_adj_few
     bool parts_set = false;     // the split was chosen by the caller, the autotuner or the environment
     size_t slabs = 0;           // slabs per angle that `partial` holds
     // probe retrieval: a second transposed probe table (forward with a given
@@ -1144,6 +1273,16 @@ void by_kind(const pt_ptycho *h, Go go)
         full ? go(std::true_type{}, std::false_type{}) : go(std::false_type{}, std::false_type{});
 }
 
+template <int DET, int RESID, bool SUB>
+void launch_few(dim3 grid, pt_ptycho *h, const float2 *in, float2 *dst, float scale, const float *data, float dscale,
+                cudaStream_t st)
+{
+    if constexpr (DET <= 32)
+        k_ptycho_adj_few<DET, RESID, SUB><<<grid, PF<DET>::NT, PF<DET>::SMEM, st>>>(
+            in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw, data, dscale,
+            h->angles, h->shift_ids());
+}
+
 template <int DET, int RESID>
 int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, const float *data, float dscale,
                       cudaStream_t st)
@@ -1165,6 +1304,8 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
                 k_ptycho_adj128<FU, RESID, S><<<grid, 512, P128_ASMEM, st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, h->angles, h->shift_ids());
+            else if (DET <= 32 && h->few)
+                launch_few<DET, RESID, S>(grid, h, in, dst, scale, data, dscale, st);
             else
                 k_ptycho_adj<DET, FU, RESID, S>
                     <<<grid, FR<DET>::BLOCK, FR<DET>::smem(FR<DET>::nf_adj(FU, RESID != 0)), st>>>(
@@ -1310,7 +1451,7 @@ int probe_adj_dispatch(pt_ptycho *h, float2 *gprb, const float2 *in, const float
 // Times of the adjoint's parts, per cell of an object slab where they scale
 // with it (a thread's and an SM's share of the clear, the sum of the parts).
 struct SplitCost {
-    double lone, frame, clear, clear_sm, sum, sum_cell;
+    double lone, frame, clear, clear_sm, sum, sum_cell, fixed;
 };
 struct Residency {
     int probe_blocks, frames, blocks, threads;
@@ -1319,7 +1460,7 @@ struct Residency {
 Residency residency(int det)
 {
     switch (det) {
-    case 16: return {FR<16>::BPSP, FR<16>::FPB, FR<16>::BPS, FR<16>::BLOCK, {2.03, 0.081, 2.7e-3, 2.2e-4, 2.9, 1.7e-6}};
+    case 16: return {FR<16>::BPSP, FR<16>::FPB, FR<16>::BPS, FR<16>::BLOCK, {2.03, 0.081, 2.7e-3, 2.2e-4, 2.9, 1.7e-6, 2.9}};
     case 32: return {FR<32>::BPSP, FR<32>::FPB, FR<32>::BPS, FR<32>::BLOCK, {2.21, 0.30, 5.3e-4, 1.9e-4, 5.9, 1.5e-6}};
     case 64: return {FR<64>::BPSP, FR<64>::FPB, FR<64>::BPS, FR<64>::BLOCK, {3.05, 1.21, 2.0e-3, 1.15e-4, 5.5, 1.8e-6}};
     // a unit is a frame; a block alone or with neighbours clears a slab's worth
@@ -1327,9 +1468,15 @@ Residency residency(int det)
     default: return {1, 1, 1, 512, {1, 1, 0, 0.375 / (128 * 128), 0, 0}};
     }
 }
+// k_ptycho_adj_few
+Residency residency_few(int det)
+{
+    if (det == 16) return {0, 1, 16, PF<16>::NT, {0.95, 0.262, 1.15e-3, 2.1e-4, 2.9, 1.6e-6, 0}};
+    return {0, 1, 4, PF<32>::NT, {0.83, 1.45, 1.4e-3, 3.5e-4, 2.5, 8.5e-7, 2.9}};
+}
 
 // The adjoint's split of an angle's scans over blocks: the number of parts with
-// the earliest end.  In microseconds, with R the blocks on an SM:
+// the earliest end, and for 16 and 32 pixels the kernel.  In microseconds, with R the blocks on an SM:
 //   a block    clears its slab, at the SM's store rate, and takes trips of
 //              max(lone, R frames) each: a few blocks wait on latency, many on
 //              the SM;
@@ -1338,9 +1485,9 @@ Residency residency(int det)
 // they differ: the blocks are then placed on the SMs one by one; else whole
 // waves of equal blocks and what is left.
 // More than 16 parts are tried only while all blocks run at once.
-// The constants are the best over 52 calls of 16- to 64-pixel detectors timed at
-// every split (4 to 351 angles, 10 to 378 scans, objects of 33 to 254): the
-// chosen split is 1 to 5 % from the best one on average.  16 x 16 frames run 24
+// The constants are the best over 116 calls of 16- to 64-pixel detectors timed at
+// every split (4 to 351 angles, 9 to 397 scans, objects of 33 to 254): the
+// choice is 3 to 7 % from the best one on average, over 64 further calls too.  16 x 16 frames run 24
 // blocks per SM and 32 x 32 frames 12; counting three as for 64 x 64 took 4 x
 // 325 scans from 39 to 51 us (33 us now) and 195 x 241 to 157 us (77 us now);
 // clears counted too low took 48 x 14 scans on a 251 x 254 object from 57 to
@@ -1348,15 +1495,18 @@ Residency residency(int det)
 // Det 128, one block per SM, in units of a frame: 45 angles with 100 to 400 scans:
 // 6 parts and the angles with most scans first instead of 3 parts in angle
 // order, Gaussian gradient 1.48 -> 1.09 ms, Poisson 1.43 -> 0.90 ms.
-int choose_parts(const pt_ptycho &h, const std::vector<int> *counts)
+struct Split {
+    int parts;
+    bool few;
+};
+Split choose_split(const pt_ptycho &h, const std::vector<int> *counts)
 {
-    const Residency res = residency(h.det);
     const double cells = (double)h.nz * h.n;
-    const size_t slots = (size_t)h.nsm * res.blocks;
-    const SplitCost &c = res.cost;
-    int best_p = 1;
+    Split best_split = {1, false};
     double best = 1e300;
-    auto time = [&](int p) {
+    auto time = [&](int p, const Residency &res) {
+        const size_t slots = (size_t)h.nsm * res.blocks;
+        const SplitCost &c = res.cost;
         const size_t blocks = (size_t)h.ntheta * p;
         const int passes = h.det == 128 && p > 1 ? 2 : 1;
         auto block = [&](int scans, size_t sharing) {   // sharing: blocks on the SM
@@ -1365,7 +1515,7 @@ int choose_parts(const pt_ptycho &h, const std::vector<int> *counts)
                    trips * std::max(c.lone, (double)sharing * res.frames * c.frame);
         };
         auto sharing = [&](size_t n) { return (std::min(n, slots) + h.nsm - 1) / h.nsm; };
-        const double sum = p > 1 ? c.sum + c.sum_cell * cells * h.ntheta * (p + 1) : 0;
+        const double sum = c.fixed + (p > 1 ? c.sum + c.sum_cell * cells * h.ntheta * (p + 1) : 0);
         double end = 0;
         if (!counts) {
             const size_t waves = blocks / slots, rest = blocks % slots;
@@ -1391,15 +1541,19 @@ int choose_parts(const pt_ptycho &h, const std::vector<int> *counts)
         }
         return end + sum;
     };
-    for (int p : {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 24, 32, 48, 64}) {
-        if (p > h.nscan || (p > 16 && (h.det == 128 || (size_t)h.ntheta * p > slots))) break;
-        const double end = time(p);
-        if (end < best - 1e-9) {
-            best = end;
-            best_p = p;
+    for (const bool few : {false, true}) {
+        if (few && h.det > 32) break;
+        const Residency res = few ? residency_few(h.det) : residency(h.det);
+        for (int p : {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 24, 32, 48, 64}) {
+            if (p > h.nscan || (p > 16 && (h.det == 128 || (size_t)h.ntheta * p > (size_t)h.nsm * res.blocks))) break;
+            const double end = time(p, res);
+            if (end < best - 1e-9) {
+                best = end;
+                best_split = {p, few};
+            }
         }
     }
-    return best_p;
+    return best_split;
 }
 
 void release_slabs(pt_ptycho *h)
@@ -1598,7 +1752,9 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
         parts = std::min<int>(atoi(env_parts), (int)nscan);
         h->parts_set = true;
     } else if (detx >= 16) {
-        parts = choose_parts(*h, nullptr);
+        const Split split = choose_split(*h, nullptr);
+        parts = split.parts;
+        h->few = split.few;
     }
     // the small tables are cuts of one allocation, each on a 256-byte boundary
     const size_t P2 = nprb * nprb, nf = ntheta * nscan;
@@ -1713,7 +1869,9 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
     if (!h->parts_set && h->det >= 16) {
         std::sort(counts.begin(), counts.end(), std::greater<int>());
         const bool even = counts.front() == h->nscan && counts.back() == h->nscan;
-        set_parts(h, choose_parts(*h, even ? nullptr : &counts));   // one part if its slabs do not fit
+        const Split split = choose_split(*h, even ? nullptr : &counts);
+        h->few = split.few;
+        set_parts(h, split.parts);   // one part if its slabs do not fit
     }
     h->ready = true;
     if (h->quant) {   // new offsets or probe: new shifted tables (on failure the model is switched off)
