@@ -659,7 +659,9 @@ __global__ void __launch_bounds__(PF<DET>::NT, 1)
     extern __shared__ float2 sm[];
     float2 *fr = sm;
     float2 *tws = sm + DET * F::P;
-    const int part = blockIdx.x, parts = gridDim.x, th = angles[blockIdx.y];
+    // angles: null where all angles have the same number of scans (one load less
+    // before the first frame: 1 us of 15)
+    const int part = blockIdx.x, parts = gridDim.x, th = angles ? angles[blockIdx.y] : blockIdx.y;
     float2 *slab = dst + ((size_t)th * parts + part) * nz * n;
     for (int i = threadIdx.x; i < DET; i += F::NT) tws[i] = tw[i];
     for (int e = threadIdx.x; e < nz * n; e += F::NT) slab[e] = czero();
@@ -1197,6 +1199,7 @@ struct pt_ptycho {
     // the object adjoint's order of angles: most scans first (as uploaded: order)
     int *angles = nullptr;
     std::vector<int> order;
+    bool ordered = false;       // that order is not 0, 1, 2, ...
     bool few = false;           // det 16, 32: k_ptycho_adj_few
     bool parts_set = false;     // the split was chosen by the caller, the autotuner or the environment
     size_t slabs = 0;           // slabs per angle that `partial` holds
@@ -1280,7 +1283,7 @@ void launch_few(dim3 grid, pt_ptycho *h, const float2 *in, float2 *dst, float sc
     if constexpr (DET <= 32)
         k_ptycho_adj_few<DET, RESID, SUB><<<grid, PF<DET>::NT, PF<DET>::SMEM, st>>>(
             in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw, data, dscale,
-            h->angles, h->shift_ids());
+            h->ordered ? h->angles : nullptr, h->shift_ids());
 }
 
 template <int DET, int RESID>
@@ -1861,6 +1864,7 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
     for (int i = 0; i < nf; ++i) counts[i / h->nscan] += corner[2 * i] >= 0 && corner[2 * i + 1] >= 0;
     for (int t = 0; t < h->ntheta; ++t) order[t] = t;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return counts[a] > counts[b]; });
+    h->ordered = !std::is_sorted(order.begin(), order.end());
     if (order != h->order) {
         PT_CUDA(cudaMemcpyAsync(h->angles, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, st));
         PT_CUDA(cudaStreamSynchronize(st));

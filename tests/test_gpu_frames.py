@@ -95,3 +95,35 @@ def test_gaussian_residual_out_of_range_values(det):
     f = torch.empty((1, n, n), dtype=torch.complex64, device="cuda")
     op.adj_resid(f, T(h), T(d), 1.0, 1)
     assert rel(f.cpu().numpy(), orc.adj(r)) <= 1e-5
+
+
+@pytest.mark.parametrize("nt,nz,n,ns,det,P", [
+    (4, 60, 61, 325, 16, 10), (2, 41, 40, 130, 32, 32),       # more than 16 parts
+    (33, 61, 60, 14, 16, 13), (6, 50, 47, 20, 32, 31),        # few frames: four threads per line
+    (148, 33, 33, 36, 16, 16), (60, 40, 41, 40, 32, 29),      # many
+    (1, 70, 71, 887, 64, 32), (8, 70, 71, 111, 64, 32)])      # forward: one and two frames per trip
+@pytest.mark.parametrize("uneven", [False, True])
+def test_dispatch_edges_against_oracle(nt, nz, n, ns, det, P, uneven):
+    """The forms that the numbers of frames and scans choose between.  The
+    tolerances of the test above; sums over several hundred scans of one pixel
+    add at most sqrt(400) x 2^-24 = 1.2e-6 to the adjoint's: 4e-6."""
+    from ptychotomo_b200 import ptychofft
+    rng = np.random.default_rng(det + 7 * ns)
+    scan = np.stack([rng.uniform(0, n - P, (nt, ns)), rng.uniform(0, nz - P, (nt, ns))]).astype(np.float32)
+    if uneven:
+        for t in range(nt):
+            scan[:, t, ns - rng.integers(0, ns // 2):] = -1
+    prb, psi = crand(rng, (P, P)), crand(rng, (nt, nz, n))
+    op, orc = ptychofft(nt, nz, n, nt, ns, det, det, P), PtychoFFT(nt, nz, n, nt, ns, det, det, P)
+    op.setobj(T(scan), T(prb))
+    orc.setobj(scan, prb)
+    g = torch.full((nt, ns, det, det), float("nan"), dtype=torch.complex64, device="cuda")
+    op.fwd(g, T(psi))
+    assert rel(g.cpu().numpy(), orc.fwd(psi)) <= 2e-6
+    h = crand(rng, g.shape)
+    f = torch.full((nt, nz, n), float("nan"), dtype=torch.complex64, device="cuda")
+    op.adj(f, T(h))
+    assert rel(f.cpu().numpy(), orc.adj(h)) <= 4e-6
+    data = (np.abs(h) ** 2 * rng.uniform(0.25, 0.75, h.shape)).astype(np.float32)
+    op.adj_resid(f, T(h), T(data), 1.0, 0)
+    assert rel(f.cpu().numpy(), orc.adj(h - data * h / np.abs(h) ** 2)) <= 1e-5
