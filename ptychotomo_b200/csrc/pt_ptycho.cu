@@ -11,10 +11,11 @@
 //  adjoint  psi = Q* F* g (ptychofft.cu:78-93): the same transform in reverse;
 //    block (part, angle) walks scans s = part, part + parts, ... in order and
 //    accumulates conj(probe) x frame into its own slab; with parts > 1 the
-//    slabs are summed in a fixed order by a second kernel.  Deterministic,
-//    no atomics.
+//    slabs are summed in a fixed order by a second kernel.  Deterministic:
+//    one block adds to a slab, and its frames' sums keep their order.
 //  Detector 128x128 has its own kernels (k_ptycho_fwd128, k_ptycho_adj128): 32
-//    values per thread, one 512-thread block per SM.
+//    values per thread, one 512-thread block per SM.  Few frames of 16x16 and
+//    32x32 take k_ptycho_adj_few in the adjoint (choose_split).
 //  The adjoints also serve the residual-on-load and probe adjoints.
 //  Detector 8x8 uses a plain shared-memory Stockham path.
 #include <algorithm>
