@@ -1203,7 +1203,10 @@ struct pt_ptycho {
     bool ordered = false;       // that order is not 0, 1, 2, ...
     bool few = false;           // det 16, 32: k_ptycho_adj_few
     bool parts_set = false;     // the split was chosen by the caller, the autotuner or the environment
-    size_t slabs = 0;           // slabs per angle that `partial` holds
+    // slabs per angle that `partial` holds, and whether a launch has used them:
+    // a captured graph may hold their address, so setobj leaves them where they are
+    size_t slabs = 0;
+    bool slabs_used = false;
     // probe retrieval: a second transposed probe table (forward with a given
     // probe) and one P x P partial per block of the probe adjoint
     float2 *prbT2 = nullptr, *prb_part = nullptr;
@@ -1299,6 +1302,7 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
         return PT_OK;
     } else {
         float2 *dst = h->parts > 1 ? h->partial : out;
+        h->slabs_used |= h->parts > 1;
         const dim3 grid(h->parts, h->ntheta);
         // SUB: the sub-pixel model's per-frame probe tables (a separate
         // instantiation, so the reference model's kernels are unchanged)
@@ -1488,7 +1492,8 @@ Residency residency_few(int det)
 // counts: the scans of each angle that are not skipped, in launch order, where
 // they differ: the blocks are then placed on the SMs one by one; else whole
 // waves of equal blocks and what is left.
-// More than 16 parts are tried only while all blocks run at once.
+// More than 16 parts are tried only while all blocks run at once and their
+// slabs take at most 1 GiB; at most `most` parts.
 // The constants are the best over 116 calls of 16- to 64-pixel detectors timed at
 // every split (4 to 351 angles, 9 to 397 scans, objects of 33 to 254): the
 // choice is 3 to 7 % from the best one on average, over 64 further calls too.  16 x 16 frames run 24
@@ -1503,7 +1508,7 @@ struct Split {
     int parts;
     bool few;
 };
-Split choose_split(const pt_ptycho &h, const std::vector<int> *counts)
+Split choose_split(const pt_ptycho &h, const std::vector<int> *counts, size_t most)
 {
     const double cells = (double)h.nz * h.n;
     Split best_split = {1, false};
@@ -1549,7 +1554,9 @@ Split choose_split(const pt_ptycho &h, const std::vector<int> *counts)
         if (few && h.det > 32) break;
         const Residency res = few ? residency_few(h.det) : residency(h.det);
         for (int p : {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 24, 32, 48, 64}) {
-            if (p > h.nscan || (p > 16 && (h.det == 128 || (size_t)h.ntheta * p > (size_t)h.nsm * res.blocks))) break;
+            const size_t blocks = (size_t)h.ntheta * p;
+            if (p > h.nscan || (size_t)p > most) break;
+            if (p > 16 && (h.det == 128 || blocks > (size_t)h.nsm * res.blocks || blocks * cells > (1u << 27))) break;
             const double end = time(p, res);
             if (end < best - 1e-9) {
                 best = end;
@@ -1565,6 +1572,7 @@ void release_slabs(pt_ptycho *h)
     if (h->partial) cudaFree(h->partial);
     h->partial = nullptr;
     h->slabs = 0;
+    h->slabs_used = false;
 }
 
 // Uses `parts` parts from now on, with slabs for them; one part if they do not fit.
@@ -1756,9 +1764,7 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
         parts = std::min<int>(atoi(env_parts), (int)nscan);
         h->parts_set = true;
     } else if (detx >= 16) {
-        const Split split = choose_split(*h, nullptr);
-        parts = split.parts;
-        h->few = split.few;
+        h->parts = choose_split(*h, nullptr, SIZE_MAX).parts;   // setobj chooses again, for the scans that are there
     }
     // the small tables are cuts of one allocation, each on a 256-byte boundary
     const size_t P2 = nprb * nprb, nf = ntheta * nscan;
@@ -1780,7 +1786,7 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
         used += (count * sizeof(*p) + 255) / 256 * 256;
     };
     cuts(place);
-    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && set_parts(h, parts);
+    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && (!h->parts_set || set_parts(h, parts));
     if (ok) cuts(place);
     // probe adjoint: one partial per frame in flight
     const Residency res = residency((int)detx);
@@ -1874,9 +1880,14 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
     if (!h->parts_set && h->det >= 16) {
         std::sort(counts.begin(), counts.end(), std::greater<int>());
         const bool even = counts.front() == h->nscan && counts.back() == h->nscan;
-        const Split split = choose_split(*h, even ? nullptr : &counts);
-        h->few = split.few;
-        set_parts(h, split.parts);   // one part if its slabs do not fit
+        auto choose = [&](size_t most) {
+            const Split split = choose_split(*h, even ? nullptr : &counts, most);
+            h->few = split.few;
+            return set_parts(h, split.parts);
+        };
+        // never more parts than slabs that a launch has used hold: those stay
+        // (one part if new ones cannot be allocated)
+        if (!choose(h->slabs_used ? h->slabs : SIZE_MAX)) choose(1);
     }
     h->ready = true;
     if (h->quant) {   // new offsets or probe: new shifted tables (on failure the model is switched off)
