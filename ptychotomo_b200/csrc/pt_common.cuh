@@ -27,13 +27,16 @@ __host__ __device__ __forceinline__ float2 czero() { return make_float2(0.f, 0.f
 // D = measured intensity (already scaled).  Poisson: x - D x / (|x|^2 + 1e-32),
 // the quotient as D times the correctly rounded reciprocal of the divisor (a
 // normal number >= 1e-32), so zero counts, which are common, take the same
-// path as the rest.  Gaussian: x - sqrt(D) exp(i angle(x)), formed as
+// path as the rest; where D / (|x|^2 + 1e-32) is out of range (weak x under
+// more than 1e6 counts) D x / (...) need not be, and is D times (x / (...)).
+// Gaussian: x - sqrt(D) exp(i angle(x)), formed as
 // x (1 - sqrt(D) / |x|) with rsqrtf for 1/|x| (within 2 ulp; the reference's
 // angle/exp pair is itself a few ulp from exact); for |x|^2 < 1e-30 (and
 // x = 0, where angle is 0) through atan2 as written.
 __device__ __forceinline__ float2 pt_residual_poisson(float2 x, float D)
 {
-    const float q = D * __frcp_rn(x.x * x.x + x.y * x.y + 1e-32f);
+    const float r = __frcp_rn(x.x * x.x + x.y * x.y + 1e-32f), q = D * r;
+    if (fabsf(q) > 1e38f) return make_float2(x.x - D * (x.x * r), x.y - D * (x.y * r));
     return make_float2(x.x - q * x.x, x.y - q * x.y);
 }
 // the rare |x|^2 < 1e-30 case, kept out of line so that unrolled callers stay small

@@ -78,9 +78,9 @@ __device__ __forceinline__ float rcp_normal(float x)
 // approximation; Gaussian x (1 - sqrt(D) / |x|): sqrt(D) is one Heron step from
 // D / sqrt(D), and 1 / |x| the approximation that pt_residual_gaussian takes.
 // Either step leaves the correctly rounded value but for rare last bits.  A
-// value out of range (|x|^2 above 1e37; Gaussian also |x|^2 below 1e-30, or D
-// not zero and outside these bounds, negative or not finite) makes the thread
-// take pt_residual_* for it afterwards.  With a test and a call site per value
+// value out of range (|x|^2 above 1e37; Poisson also D / b above 1e38; Gaussian
+// also |x|^2 below 1e-30, or D not zero and outside these bounds, negative or
+// not finite) makes the thread take pt_residual_* for it afterwards.  With a test and a call site per value
 // and the rounded reciprocal or square root of the library, the det-128
 // gradient of 45 angles with 100 to 400 scans took 1.81 ms Gaussian; it takes
 // 1.48 ms.
@@ -97,7 +97,7 @@ __device__ __forceinline__ void resid_line(float2 (&v)[M], float (&d)[M], float 
             if constexpr (RESID == 1) {
                 const float b = a2 + 1e-32f, y = rcp_normal(b);
                 d[m] = D * fmaf(fmaf(-b, y, 1.f), y, y);
-                if (!(b <= 1e37f)) rare |= 1u << m;
+                if (!(b <= 1e37f && fabsf(d[m]) <= 1e38f)) rare |= 1u << m;
                 continue;
             }
             const float z = rsqrt_normal(D), s0 = D * z;
