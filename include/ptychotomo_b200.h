@@ -155,6 +155,9 @@ int pt_ptycho_adj_resid(pt_ptycho *h, void *f, const void *fpsi, const float *da
  *       fwd with respect to the probe for the object psi [Ntheta][Nz][N];
  *   pt_ptycho_adj_probe_resid: the same with g = the data-term residual of
  *       fpsi (as pt_ptycho_adj_resid): the data term's probe gradient;
+ *   pt_ptycho_adj_probe_resid64: the same as complex128, the FP64 sum before
+ *       it is rounded, for a caller that adds the gradients of several parts
+ *       of the angles;
  *   pt_ptycho_fwd_probe:       fwd(g, psi) with the probe prb [P][P] instead
  *       of the one given to setobj (which stays in place).
  * Deterministic (fixed-order sum of per-block partials).  Detectors 16..128;
@@ -162,6 +165,8 @@ int pt_ptycho_adj_resid(pt_ptycho *h, void *f, const void *fpsi, const float *da
 int pt_ptycho_adj_probe(pt_ptycho *h, void *gprb, const void *g, const void *psi, float scale, void *stream);
 int pt_ptycho_adj_probe_resid(pt_ptycho *h, void *gprb, const void *psi, const void *fpsi, const float *data,
                               float dscale, int model, float scale, void *stream);
+int pt_ptycho_adj_probe_resid64(pt_ptycho *h, void *gprb, const void *psi, const void *fpsi, const float *data,
+                                float dscale, int model, float scale, void *stream);
 int pt_ptycho_fwd_probe(pt_ptycho *h, void *g, const void *psi, const void *prb, float scale, void *stream);
 /* Autotuner (no counterpart in the reference): the adjoint splits each
  * angle's scans over `parts` blocks (own slabs, then a fixed-order sum);

@@ -63,6 +63,7 @@ SIGNATURES = {
     "pt_ptycho_adj_resid": (_int, [_vp, _vp, _vp, _vp, _f, _int, _f, _vp]),
     "pt_ptycho_adj_probe": (_int, [_vp, _vp, _vp, _vp, _f, _vp]),
     "pt_ptycho_adj_probe_resid": (_int, [_vp, _vp, _vp, _vp, _vp, _f, _int, _f, _vp]),
+    "pt_ptycho_adj_probe_resid64": (_int, [_vp, _vp, _vp, _vp, _vp, _f, _int, _f, _vp]),
     "pt_ptycho_fwd_probe": (_int, [_vp, _vp, _vp, _vp, _f, _vp]),
     "pt_ptycho_autotune": (_int, [_vp, _vp, _vp, _int, ctypes.POINTER(_int), _vp]),
     "pt_ptycho_get_parts": (_int, [_vp, ctypes.POINTER(_int)]),

@@ -1102,10 +1102,11 @@ __global__ void k_probe_t(const float2 *__restrict__ prb, float2 *__restrict__ p
 
 // gprb[px P + py] = c sum_b part[b][py P + px].  A block takes 32 elements; its
 // eight warps sum the partials b = warp, warp + 8, ..., then the eight sums are
-// added in warp order, in FP64: the order (one rank's partials or two ranks')
-// then shows in the last bit at most.
+// added in warp order, in FP64: the order then shows in the last bit at most.
+// T double2: the sum as it is, for a caller that adds several.
+template <typename T>
 __global__ void __launch_bounds__(256)
-    k_probe_reduce(const float2 *__restrict__ part, float2 *__restrict__ gprb, int nblk, int P, float c)
+    k_probe_reduce(const float2 *__restrict__ part, T *__restrict__ gprb, int nblk, int P, float c)
 {
     __shared__ double2 sums[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1126,7 +1127,10 @@ __global__ void __launch_bounds__(256)
         s.y += sums[k][lane].y;
     }
     const int py = i / P, px = i % P;
-    gprb[px * P + py] = make_float2((float)(c * s.x), (float)(c * s.y));
+    T r;
+    r.x = c * s.x;
+    r.y = c * s.y;
+    gprb[px * P + py] = r;
 }
 
 }  // namespace
@@ -1409,8 +1413,8 @@ int ptycho_dispatch(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float
 }
 
 template <int DET, int RESID>
-int probe_adj_launch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 *psi, float scale, const float *data,
-                     float dscale, cudaStream_t st)
+int probe_adj_launch(pt_ptycho *h, void *gprb, bool fp64, const float2 *in, const float2 *psi, float scale,
+                     const float *data, float dscale, cudaStream_t st)
 {
     if constexpr (DET < 16) {
         pt::set_error("ptychofft.adj_probe: not compiled for detector %d (16 to 128)", DET);
@@ -1434,20 +1438,24 @@ int probe_adj_launch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 
         else
             go(std::false_type{});
         PT_LAUNCHED("k_ptycho_adj_probe");
-        k_probe_reduce<<<(h->P * h->P + 31) / 32, 256, 0, st>>>(h->prb_part, gprb, h->prb_blocks, h->P, h->c);
+        const unsigned blocks = (unsigned)((h->P * h->P + 31) / 32);
+        if (fp64)
+            k_probe_reduce<<<blocks, 256, 0, st>>>(h->prb_part, (double2 *)gprb, h->prb_blocks, h->P, h->c);
+        else
+            k_probe_reduce<<<blocks, 256, 0, st>>>(h->prb_part, (float2 *)gprb, h->prb_blocks, h->P, h->c);
         PT_LAUNCHED("k_probe_reduce");
         return PT_OK;
     }
 }
 
-int probe_adj_dispatch(pt_ptycho *h, float2 *gprb, const float2 *in, const float2 *psi, float scale, int resid_mode,
-                       const float *data, float dscale, cudaStream_t st)
+int probe_adj_dispatch(pt_ptycho *h, void *gprb, bool fp64, const float2 *in, const float2 *psi, float scale,
+                       int resid_mode, const float *data, float dscale, cudaStream_t st)
 {
-#define PT_CASE(D)                                                                               \
-    if (h->det == D) {                                                                           \
-        if (resid_mode == 1) return probe_adj_launch<D, 1>(h, gprb, in, psi, scale, data, dscale, st); \
-        if (resid_mode == 2) return probe_adj_launch<D, 2>(h, gprb, in, psi, scale, data, dscale, st); \
-        return probe_adj_launch<D, 0>(h, gprb, in, psi, scale, data, dscale, st);                \
+#define PT_CASE(D)                                                                                               \
+    if (h->det == D) {                                                                                           \
+        if (resid_mode == 1) return probe_adj_launch<D, 1>(h, gprb, fp64, in, psi, scale, data, dscale, st);      \
+        if (resid_mode == 2) return probe_adj_launch<D, 2>(h, gprb, fp64, in, psi, scale, data, dscale, st);      \
+        return probe_adj_launch<D, 0>(h, gprb, fp64, in, psi, scale, data, dscale, st);                          \
     }
     PT_PTYCHO_DETS(PT_CASE)
 #undef PT_CASE
@@ -2056,20 +2064,34 @@ extern "C" int pt_ptycho_adj_probe(pt_ptycho *h, void *gprb, const void *g, cons
     const int rc = probe_checks(h, "adj_probe");
     if (rc != PT_OK) return rc;
     PT_CHECK_ARG(gprb && g && psi, "ptychofft.adj_probe: null array pointer");
-    return probe_adj_dispatch(h, (float2 *)gprb, (const float2 *)g, (const float2 *)psi, scale, 0, nullptr, 1.f,
+    return probe_adj_dispatch(h, gprb, false, (const float2 *)g, (const float2 *)psi, scale, 0, nullptr, 1.f,
                               (cudaStream_t)stream);
 }
 
-extern "C" int pt_ptycho_adj_probe_resid(pt_ptycho *h, void *gprb, const void *psi, const void *fpsi,
-                                         const float *data, float dscale, int model, float scale, void *stream)
+namespace {
+int adj_probe_resid(pt_ptycho *h, void *gprb, bool fp64, const void *psi, const void *fpsi, const float *data,
+                    float dscale, int model, float scale, void *stream)
 {
     pt::clear_error();
     const int rc = probe_checks(h, "adj_probe_resid");
     if (rc != PT_OK) return rc;
     PT_CHECK_ARG(gprb && psi && fpsi && data, "ptychofft.adj_probe_resid: null array pointer");
     PT_CHECK_ARG(model == 0 || model == 1, "ptychofft.adj_probe_resid: model 0 (poisson) or 1 (gaussian)");
-    return probe_adj_dispatch(h, (float2 *)gprb, (const float2 *)fpsi, (const float2 *)psi, scale, model + 1, data,
-                              dscale, (cudaStream_t)stream);
+    return probe_adj_dispatch(h, gprb, fp64, (const float2 *)fpsi, (const float2 *)psi, scale, model + 1, data, dscale,
+                              (cudaStream_t)stream);
+}
+}  // namespace
+
+extern "C" int pt_ptycho_adj_probe_resid(pt_ptycho *h, void *gprb, const void *psi, const void *fpsi,
+                                         const float *data, float dscale, int model, float scale, void *stream)
+{
+    return adj_probe_resid(h, gprb, false, psi, fpsi, data, dscale, model, scale, stream);
+}
+
+extern "C" int pt_ptycho_adj_probe_resid64(pt_ptycho *h, void *gprb, const void *psi, const void *fpsi,
+                                           const float *data, float dscale, int model, float scale, void *stream)
+{
+    return adj_probe_resid(h, gprb, true, psi, fpsi, data, dscale, model, scale, stream);
 }
 
 extern "C" int pt_ptycho_fwd_probe(pt_ptycho *h, void *g, const void *psi, const void *prb, float scale,

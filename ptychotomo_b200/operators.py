@@ -185,6 +185,12 @@ class ptychofft:  # noqa: N801 - reference class name
                                               float(dscale), int(model), float(scale), _s(stream)),
               "ptychofft.adj_probe_resid")
 
+    def adj_probe_resid64(self, gprb, psi, fpsi, data, dscale, model, scale=1.0, stream=None):
+        """adj_probe_resid as complex128: the FP64 sum, for adding the gradients of parts of the angles."""
+        check(lib().pt_ptycho_adj_probe_resid64(self._h, as_ptr(gprb), as_ptr(psi), as_ptr(fpsi), as_ptr(data),
+                                                float(dscale), int(model), float(scale), _s(stream)),
+              "ptychofft.adj_probe_resid64")
+
     def fwd_probe(self, g, psi, prb, scale=1.0, stream=None):
         """fwd(g, psi) with the probe prb instead of the one given to setobj."""
         check(lib().pt_ptycho_fwd_probe(self._h, as_ptr(g), as_ptr(psi), as_ptr(prb), float(scale), _s(stream)),

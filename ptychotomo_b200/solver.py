@@ -473,12 +473,14 @@ class Solver:
         grad0 = d = None
         for i in range(piter):
             fp = [fwd(p, ids, op) for ids, op in chunks]
-            grad = torch.zeros_like(p)
-            gk = torch.empty_like(p)
+            # summed over the chunks and the ranks in FP64 and rounded once: CG
+            # amplifies its rounding, and the sum does not depend on the split
+            grad = torch.zeros(p.shape, dtype=torch.complex128, device=self.device)
+            gk = torch.empty_like(grad)
             for (ids, op), f in zip(chunks, fp):
-                op.adj_probe_resid(gk, psi[ids].contiguous(), f, data[ids], self.coefdata, mdl, scale=self.coefptycho)
-                K.lincomb(grad, [(1.0, grad), (1.0, gk)])
-            grad = self._sum_probe(grad)
+                op.adj_probe_resid64(gk, psi[ids].contiguous(), f, data[ids], self.coefdata, mdl, scale=self.coefptycho)
+                grad += gk
+            grad = self._sum_probe(grad).to(torch.complex64)
             if i == 0:
                 d = K.lincomb(torch.empty_like(grad), [(-1.0, grad)])
             else:
