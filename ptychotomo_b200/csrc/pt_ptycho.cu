@@ -14,8 +14,9 @@
 //    slabs are summed in a fixed order by a second kernel.  Deterministic:
 //    one block adds to a slab, and its frames' sums keep their order.
 //  Detector 128x128 has its own kernels (k_ptycho_fwd128, k_ptycho_adj128): 32
-//    values per thread, one 512-thread block per SM.  Few frames of 16x16 and
-//    32x32 take k_ptycho_adj_few in the adjoint (choose_split).
+//    values per thread, one 512-thread block per SM.  Few frames of 16x16 to
+//    64x64 take k_ptycho_fwd_few (few_frames), of 16x16 and 32x32 in the adjoint
+//    k_ptycho_adj_few (choose_split).
 //  The adjoints also serve the residual-on-load and probe adjoints.
 //  Detector 8x8 uses a plain shared-memory Stockham path.
 #include <algorithm>
@@ -593,17 +594,17 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
     }
 }
 
-// ---- det 16 and 32, few frames: the adjoint with four threads per line -------
+// ---- few frames: four or eight threads per line -------------------------------
 // Where few blocks are in flight, a frame's latency counts, not the SM's
-// instruction slots: k_ptycho_adj takes 16 values per thread (16 or 64 threads
-// per frame), this kernel 4 or 8 (64 or 128 threads), row transforms, a
-// transpose through shared memory, column transforms.  choose_split compares
-// their modelled times.  16 x 16 frames, adjoint: 9 x 74 scans 18.5 -> 14.4 us,
+// instruction slots: the kernels above take 16 values per thread (16, 64 or 256
+// threads per frame), these 4 or 8 (64, 128 or 512 threads): row transforms, a
+// transpose through shared memory, column transforms.
+// Adjoint, det 16 and 32: choose_split compares the modelled times.  16 x 16 frames, adjoint: 9 x 74 scans 18.5 -> 14.4 us,
 // 65 x 14 scans on a 145 x 152 object 29 -> 20 us (more threads to clear its
 // slabs); but 224 x 146 scans take 94 us here and 66 us there.
 template <int DET>
 struct PF {
-    static constexpr int N2 = 4;                           // threads per line
+    static constexpr int N2 = DET == 64 ? 8 : 4;           // threads per line
     static constexpr int N1 = DET / N2;                    // points per thread
     static constexpr int KPT = N1 / N2;                    // k1 values per thread after the exchange
     static constexpr int NT = DET * N2;                    // threads per block
@@ -646,6 +647,77 @@ __device__ __forceinline__ void line_dft(float2 (&v)[PF<DET>::N1], int t, float2
 #pragma unroll
         for (int k2 = 0; k2 < F::N2; ++k2) v[j * F::N2 + k2] = u[k2];
     }
+}
+
+// Forward: one frame per block, up to few_frames frames per SM.
+template <int DET, bool SUB>
+__global__ void __launch_bounds__(PF<DET>::NT, 1)
+    k_ptycho_fwd_few(const float2 *__restrict__ psi, float2 *__restrict__ g, const int *__restrict__ corner,
+                     const float2 *__restrict__ phase, const float2 *__restrict__ prbT, int nz, int n, int nscan, int P,
+                     float scale, const float2 *__restrict__ tw, const int *__restrict__ sid)
+{
+    using F = PF<DET>;
+    extern __shared__ float2 sm[];
+    float2 *fr = sm;
+    float2 *tws = sm + DET * F::P;
+    const int fid = blockIdx.x;
+    const int stx = corner[2 * fid], sty = corner[2 * fid + 1];
+    float2 *out = g + (size_t)fid * DET * DET;
+    if (stx < 0 || sty < 0) {   // skipped scan: the reference leaves a zero frame
+        for (int e = threadIdx.x; e < DET * DET; e += F::NT) out[e] = czero();
+        return;
+    }
+    for (int i = threadIdx.x; i < DET; i += F::NT) tws[i] = tw[i];
+    const int t = threadIdx.x % F::N2, grp = threadIdx.x / F::N2;
+    float2 *sc = fr + grp * (DET + 1);
+    const int off = (DET - P) / 2, py = grp - off;
+    const float2 *src = psi + ((size_t)(fid / nscan) * nz + sty) * n + stx;
+    const float2 *pr = SUB ? prbT + (size_t)sid[fid] * P * P : prbT;  // sub-pixel: the frame's shifted probe
+    // along the object row: line = detector column iy = grp, points ix = t + N2 m
+    float2 v[F::N1];
+#pragma unroll
+    for (int m = 0; m < F::N1; ++m) {
+        const int px = t + F::N2 * m - off;
+        v[m] = py >= 0 && py < P && px >= 0 && px < P
+                   ? cmul(__ldg(&pr[py * P + px]), __ldg(&src[(size_t)py * n + px]))
+                   : czero();
+    }
+    __syncthreads();
+    line_dft<DET, -1>(v, t, sc, tws);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < F::KPT; ++j)
+#pragma unroll
+        for (int k2 = 0; k2 < F::N2; ++k2) {
+            const int kx = t * F::KPT + j + F::N1 * k2;
+            fr[kx * F::P + (grp ^ fswz<DET>(kx))] = v[j * F::N2 + k2];
+        }
+    __syncthreads();
+    const int sw = fswz<DET>(grp);
+#pragma unroll
+    for (int m = 0; m < F::N1; ++m) v[m] = fr[grp * F::P + ((t + F::N2 * m) ^ sw)];
+    __syncthreads();
+    const float2 ph = scale * phase[fid];
+    line_dft<DET, -1>(v, t, sc, tws);
+#pragma unroll
+    for (int k2 = 0; k2 < F::N2; ++k2)
+#pragma unroll
+        for (int j = 0; j < F::KPT; ++j)
+            out[grp * DET + t * F::KPT + j + F::N1 * k2] = cmul(v[j * F::N2 + k2], ph);
+}
+
+// Frames per SM up to which k_ptycho_fwd_few is the faster forward (us, this
+// kernel and k_ptycho_fwd; P the probe's width; a probe smaller than the
+// detector costs k_ptycho_fwd two launch steps of 1 us, this kernel nothing):
+// det 16, P 16: 444 frames 4.1 and 5.7, 1776 6.2 and 6.2, 2072 7.2 and 6.2;
+//         P 15: 444 frames 4.1 and 8.2, 2072 6.7 and 8.2, 2664 8.2 and 8.2;
+// det 32, P 32: 148 frames 4.6 and 6.2, 296 6.2 and 6.2, 592 8.2 and 6.2;
+//         P 24: 148 frames 4.1 and 8.2, 592 6.5 and 8.2, 1184 10.3 and 9.0;
+// det 64, P 64: 148 frames 6.2 and 8.2, 222 9.2 and 8.2;
+//         P 48: 148 frames 6.2 and 8.7, 296 8.2 and 10.2, 370 12.3 and 10.3.
+constexpr int few_frames(int det, bool full)
+{
+    return det == 16 ? (full ? 12 : 16) : det == 32 ? (full ? 2 : 5) : (full ? 1 : 2);
 }
 
 // grid (parts, ntheta): block (part, angles[y]) owns slab dst[angle][part]
@@ -1351,7 +1423,7 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
         k_ptycho_fwd_small<DET><<<dim3(h->nscan, h->ntheta), ptycho_block<DET>(), s, st>>>(
             in, out, h->corner, h->phase, h->prb, h->nz, h->n, h->nscan, h->P, h->c, scale, h->tw);
     } else {
-        // the resident blocks walk the frames (grid-stride)
+        // the resident blocks walk the frames (grid-stride); few frames, a block each
         auto go = [&](auto full, auto sub) {
             constexpr bool FU = decltype(full)::value, S = decltype(sub)::value;
             if constexpr (DET == 128) {
@@ -1360,6 +1432,12 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
                     h->tw128, h->tw, h->shift_ids());
             } else {
                 using F = FR<DET>;
+                if (nframes <= few_frames(DET, FU) * h->nsm) {
+                    k_ptycho_fwd_few<DET, S><<<nframes, PF<DET>::NT, PF<DET>::SMEM, st>>>(
+                        in, out, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw,
+                        h->shift_ids());
+                    return;
+                }
                 auto trips = [&](auto frames) {
                     constexpr int NF = decltype(frames)::value;
                     const int per = F::FPB * NF, grid = std::min((nframes + per - 1) / per, h->nsm * F::BPS);
