@@ -36,8 +36,9 @@ __host__ __device__ __forceinline__ float2 czero() { return make_float2(0.f, 0.f
 __device__ __forceinline__ float2 pt_residual_poisson(float2 x, float D)
 {
     const float r = __frcp_rn(x.x * x.x + x.y * x.y + 1e-32f), q = D * r;
-    if (fabsf(q) > 1e38f) return make_float2(x.x - D * (x.x * r), x.y - D * (x.y * r));
-    return make_float2(x.x - q * x.x, x.y - q * x.y);
+    const bool far = fabsf(q) > 1e38f;                 // selects, no branch: callers unroll this
+    const float a = far ? D : q, s = far ? r : 1.f;
+    return make_float2(x.x - a * (s * x.x), x.y - a * (s * x.y));
 }
 // the rare |x|^2 < 1e-30 case, kept out of line so that unrolled callers stay small
 static __device__ __noinline__ float2 pt_residual_gaussian_tiny(float2 x, float sq)
