@@ -127,11 +127,11 @@ int pt_ptycho_destroy(pt_ptycho *h);
  * Scans with roundf(x)<0 or roundf(y)<0 are skipped (the reference's
  * sentinel, kernels.cuh:256); a patch reaching past the object is rejected
  * with PT_ERR_ARG (the reference reads out of bounds).  Chooses the adjoint's
- * split for the scans that are not skipped, and allocates its slabs; slabs
- * that a launch or a captured graph has used stay where they are, and bound
- * the splits of later calls, so such a graph may be replayed after setobj
- * with other scans (not with the sub-pixel model, whose tables it rebuilds).
- * Blocks the host. */
+ * split for the scans that are not skipped (one for each residual), and
+ * allocates its slabs; slabs that a launch or a captured graph has used stay
+ * where they are, and bound the splits of later calls, so such a graph may be
+ * replayed after setobj with other scans (not with the sub-pixel model, whose
+ * tables it rebuilds).  Blocks the host. */
 int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb, void *stream);
 /* ptychofft::fwd(g, f) — src/cuda/ptychofft.cu:58-76.  g = F Q f. */
 int pt_ptycho_fwd(pt_ptycho *h, void *g, const void *f, void *stream);
@@ -180,7 +180,7 @@ int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int trials, int *pa
  * the slabs that were there: an adjoint captured in a graph before them must
  * not be replayed. */
 int pt_ptycho_set_parts(pt_ptycho *h, int parts);
-/* The adjoint's current split. */
+/* The adjoint's current split (the residual adjoints may have their own). */
 int pt_ptycho_get_parts(const pt_ptycho *h, int *parts);
 /* Sub-pixel scan model (no counterpart in the reference, which rounds each
  * scan position to the grid and applies a constant per-scan phase,

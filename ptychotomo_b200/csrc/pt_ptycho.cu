@@ -15,8 +15,7 @@
 //    one block adds to a slab, and its frames' sums keep their order.
 //  Detector 128x128 has its own kernels (k_ptycho_fwd128, k_ptycho_adj128): 32
 //    values per thread, one 512-thread block per SM.  Few frames of 16x16 to
-//    64x64 take k_ptycho_fwd_few (few_frames), of 16x16 and 32x32 in the adjoint
-//    k_ptycho_adj_few (choose_split).
+//    64x64 take k_ptycho_fwd_few (few_frames) and k_ptycho_adj_few (choose_split).
 //  The adjoints also serve the residual-on-load and probe adjoints.
 //  Detector 8x8 uses a plain shared-memory Stockham path.
 #include <algorithm>
@@ -599,9 +598,10 @@ __global__ void __launch_bounds__(FR<DET>::BLOCK, PROBE ? FR<DET>::BPSP : FR<DET
 // instruction slots: the kernels above take 16 values per thread (16, 64 or 256
 // threads per frame), these 4 or 8 (64, 128 or 512 threads): row transforms, a
 // transpose through shared memory, column transforms.
-// Adjoint, det 16 and 32: choose_split compares the modelled times.  16 x 16 frames, adjoint: 9 x 74 scans 18.5 -> 14.4 us,
-// 65 x 14 scans on a 145 x 152 object 29 -> 20 us (more threads to clear its
-// slabs); but 224 x 146 scans take 94 us here and 66 us there.
+// Adjoint: choose_split compares the modelled times.  16 x 16 frames, adjoint:
+// 9 x 74 scans 18.5 -> 14.4 us, 65 x 14 scans on a 145 x 152 object 29 -> 20 us
+// (more threads to clear its slabs); but 224 x 146 scans take 94 us here and
+// 66 us there.
 template <int DET>
 struct PF {
     static constexpr int N2 = DET == 64 ? 8 : 4;           // threads per line
@@ -609,6 +609,8 @@ struct PF {
     static constexpr int KPT = N1 / N2;                    // k1 values per thread after the exchange
     static constexpr int NT = DET * N2;                    // threads per block
     static constexpr int P = DET + 8;                      // frame pitch (P = 8 mod 16)
+    // resident blocks of the adjoint per SM (80, 136 and 128 registers a thread)
+    static constexpr int BPS = DET == 16 ? 12 : DET == 32 ? 3 : 1;
     static constexpr size_t SMEM = (size_t)(DET * P + DET) * sizeof(float2);
 };
 
@@ -1264,8 +1266,16 @@ __global__ void k_fill_one(float2 *__restrict__ a, size_t n)
     if (e < n) a[e] = make_float2(1.f, 0.f);
 }
 
+// The object adjoint's split: blocks (and slabs) per angle, and whether they run
+// k_ptycho_adj_few (det 16 to 64).
+struct Split {
+    int parts = 1;
+    bool few = false;
+};
+
 struct pt_ptycho {
-    int ntheta = 0, nz = 0, n = 0, nscan = 0, det = 0, P = 0, parts = 1;
+    int ntheta = 0, nz = 0, n = 0, nscan = 0, det = 0, P = 0;
+    Split split[3];   // the object adjoint's, by residual (none, Poisson, Gaussian)
     int device = -1, nsm = 148;
     bool ready = false;
     float c = 0.f;
@@ -1277,7 +1287,6 @@ struct pt_ptycho {
     int *angles = nullptr;
     std::vector<int> order;
     bool ordered = false;       // that order is not 0, 1, 2, ...
-    bool few = false;           // det 16, 32: k_ptycho_adj_few
     bool parts_set = false;     // the split was chosen by the caller, the autotuner or the environment
     // slabs per angle that `partial` holds, and whether a launch has used them:
     // a captured graph may hold their address, so setobj leaves them where they are
@@ -1360,10 +1369,12 @@ template <int DET, int RESID, bool SUB>
 void launch_few(dim3 grid, pt_ptycho *h, const float2 *in, float2 *dst, float scale, const float *data, float dscale,
                 cudaStream_t st)
 {
-    if constexpr (DET <= 32)
+    // the order of the angles matters only where blocks wait for others to end
+    const bool queued = (size_t)grid.x * grid.y > (size_t)h->nsm * PF<DET>::BPS;
+    if constexpr (DET <= 64)
         k_ptycho_adj_few<DET, RESID, SUB><<<grid, PF<DET>::NT, PF<DET>::SMEM, st>>>(
             in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw, data, dscale,
-            h->ordered ? h->angles : nullptr, h->shift_ids());
+            h->ordered && queued ? h->angles : nullptr, h->shift_ids());
 }
 
 template <int DET, int RESID>
@@ -1377,9 +1388,10 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
         PT_LAUNCHED("k_ptycho_adj_small");
         return PT_OK;
     } else {
-        float2 *dst = h->parts > 1 ? h->partial : out;
-        h->slabs_used |= h->parts > 1;
-        const dim3 grid(h->parts, h->ntheta);
+        const Split split = h->split[RESID];
+        float2 *dst = split.parts > 1 ? h->partial : out;
+        h->slabs_used |= split.parts > 1;
+        const dim3 grid(split.parts, h->ntheta);
         // SUB: the sub-pixel model's per-frame probe tables (a separate
         // instantiation, so the reference model's kernels are unchanged)
         auto go = [&](auto full, auto sub) {
@@ -1388,7 +1400,7 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
                 k_ptycho_adj128<FU, RESID, S><<<grid, 512, P128_ASMEM, st>>>(
                     in, dst, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, h->P, scale, h->tw128,
                     h->tw, data, dscale, h->angles, h->shift_ids());
-            else if (DET <= 32 && h->few)
+            else if (DET <= 64 && split.few)
                 launch_few<DET, RESID, S>(grid, h, in, dst, scale, data, dscale, st);
             else
                 k_ptycho_adj<DET, FU, RESID, S>
@@ -1398,10 +1410,10 @@ int ptycho_adj_launch(pt_ptycho *h, float2 *out, const float2 *in, float scale, 
         };
         by_kind(h, go);
         PT_LAUNCHED("k_ptycho_adj");
-        if (h->parts > 1) {
+        if (split.parts > 1) {
             const size_t slab = (size_t)h->nz * h->n, total = slab * h->ntheta;
             const unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, 148 * 16);
-            k_ptycho_reduce<<<blocks, 256, 0, st>>>(h->partial, out, slab, h->parts, total);
+            k_ptycho_reduce<<<blocks, 256, 0, st>>>(h->partial, out, slab, split.parts, total);
             PT_LAUNCHED("k_ptycho_reduce");
         }
         return PT_OK;
@@ -1541,12 +1553,18 @@ int probe_adj_dispatch(pt_ptycho *h, void *gprb, bool fp64, const float2 *in, co
     return PT_ERR_UNSUPPORTED;
 }
 
-// Blocks of the probe adjoint that an SM holds, and the frames a block works on at a time.
-// Times of the adjoint's parts, per cell of an object slab where they scale
-// with it (a thread's and an SM's share of the clear, the sum of the parts).
+// Times of the object adjoint's steps in microseconds, but for det 128 in frames
+// of an SM (only one block runs there).
 struct SplitCost {
-    double lone, frame, clear, clear_sm, sum, sum_cell, fixed;
+    // one trip of a block alone on its SM, and an SM's time for a frame, by
+    // residual and whether the probe is as wide as the detector
+    double lone[3][2], frame[3][2];
+    double clear, fixed;          // a thread's clear of a slab cell; a call
+    double clear_sm = 9.5e-5;     // an SM's clear of a slab cell
+    double sum = 4.3, sum_part = 0.15, sum_cell = 2e-6;   // the sum of the parts: a launch, per part, per slab cell
 };
+// Resident blocks per SM (of the probe adjoint, of the object adjoint), frames
+// that a block works on at a time, and its threads.
 struct Residency {
     int probe_blocks, frames, blocks, threads;
     SplitCost cost;
@@ -1554,50 +1572,58 @@ struct Residency {
 Residency residency(int det)
 {
     switch (det) {
-    case 16: return {FR<16>::BPSP, FR<16>::FPB, FR<16>::BPS, FR<16>::BLOCK, {2.03, 0.081, 2.7e-3, 2.2e-4, 2.9, 1.7e-6, 2.9}};
-    case 32: return {FR<32>::BPSP, FR<32>::FPB, FR<32>::BPS, FR<32>::BLOCK, {2.21, 0.30, 5.3e-4, 1.9e-4, 5.9, 1.5e-6}};
-    case 64: return {FR<64>::BPSP, FR<64>::FPB, FR<64>::BPS, FR<64>::BLOCK, {3.05, 1.21, 2.0e-3, 1.15e-4, 5.5, 1.8e-6}};
-    // a unit is a frame; a block alone or with neighbours clears a slab's worth
-    // of frames at 0.375 of one, and once more for the sum
-    default: return {1, 1, 1, 512, {1, 1, 0, 0.375 / (128 * 128), 0, 0}};
+    case 16: return {FR<16>::BPSP, FR<16>::FPB, FR<16>::BPS, FR<16>::BLOCK,
+                     {{{3.57, 1.97}, {3.86, 2.64}, {5.80, 4.27}}, {{0.107, 0.100}, {0.165, 0.176}, {0.312, 0.335}}, 2.0e-3, 0.7}};
+    case 32: return {FR<32>::BPSP, FR<32>::FPB, FR<32>::BPS, FR<32>::BLOCK,
+                     {{{2.25, 1.69}, {2.87, 2.52}, {4.51, 2.64}}, {{0.384, 0.393}, {0.642, 0.594}, {1.05, 0.616}}, 6.5e-4, 0}};
+    case 64: return {FR<64>::BPSP, FR<64>::FPB, FR<64>::BPS, FR<64>::BLOCK,
+                     {{{2.75, 2.27}, {3.81, 2.98}, {5.12, 3.58}}, {{1.06, 1.47}, {1.56, 1.80}, {1.81, 2.09}}, 2.0e-3, 0}};
+    // a block clears a slab's worth of frames at 0.375 of one, and once more for the sum
+    default: return {1, 1, 1, 512, {{{1, 1}, {1, 1}, {1, 1}}, {}, 0, 0, 0.375 / (128 * 128), 0, 0, 0}};
     }
 }
 // k_ptycho_adj_few
 Residency residency_few(int det)
 {
-    if (det == 16) return {0, 1, 16, PF<16>::NT, {0.95, 0.262, 1.15e-3, 2.1e-4, 2.9, 1.6e-6, 0}};
-    return {0, 1, 4, PF<32>::NT, {0.83, 1.45, 1.4e-3, 3.5e-4, 2.5, 8.5e-7, 2.9}};
+    if (det == 16)
+        return {0, 1, PF<16>::BPS, PF<16>::NT,
+                {{{0.85, 0.94}, {1.52, 1.60}, {1.57, 1.65}}, {{0.200, 0.233}, {0.226, 0.251}, {0.229, 0.252}}, 2.0e-3, 0.7}};
+    if (det == 64)
+        return {0, 1, PF<64>::BPS, PF<64>::NT,
+                {{{2.85, 3.23}, {4.82, 4.95}, {4.97, 5.13}}, {{1.37, 1.72}, {2.06, 2.09}, {2.17, 2.20}}, 2.0e-3, 0}};
+    return {0, 1, PF<32>::BPS, PF<32>::NT,
+            {{{1.37, 1.50}, {2.86, 3.06}, {3.00, 3.19}}, {{0.733, 0.983}, {0.968, 1.27}, {0.965, 1.27}}, 1.4e-3, 0.1}};
 }
 
-// The adjoint's split of an angle's scans over blocks: the number of parts with
-// the earliest end, and for 16 and 32 pixels the kernel.  In microseconds, with R the blocks on an SM:
+// The adjoint's split of an angle's scans over blocks for one residual: the
+// number of parts with the earliest end, and up to 64 pixels the kernel.
+// With R the blocks on an SM:
 //   a block    clears its slab, at the SM's store rate, and takes trips of
-//              max(lone, R frames) each: a few blocks wait on latency, many on
-//              the SM;
+//              sqrt(lone^2 + (R frames)^2) each: a few blocks wait on latency,
+//              many on the SM;
 //   the sum    of more than one part reads every slab once, after a launch.
 // counts: the scans of each angle that are not skipped, in launch order, where
 // they differ: the blocks are then placed on the SMs one by one; else whole
 // waves of equal blocks and what is left.
-// More than 16 parts are tried only while all blocks run at once and their
-// slabs take at most 1 GiB; at most `most` parts.
-// The constants are the best over 116 calls of 16- to 64-pixel detectors timed at
-// every split (4 to 351 angles, 9 to 397 scans, objects of 33 to 254): the
-// choice is 3 to 7 % from the best one on average, over 64 further calls too.  16 x 16 frames run 24
-// blocks per SM and 32 x 32 frames 12; counting three as for 64 x 64 took 4 x
-// 325 scans from 39 to 51 us (33 us now) and 195 x 241 to 157 us (77 us now);
-// clears counted too low took 48 x 14 scans on a 251 x 254 object from 57 to
-// 96 us (45 us now).
-// Det 128, one block per SM, in units of a frame: 45 angles with 100 to 400 scans:
+// No more parts than an angle has scans, or than `most`; more than 16 only while
+// all blocks run at once and their slabs take at most 1 GiB.
+// The costs are least-squares fits, of the logarithm, to 335 calls of 16- and
+// 32-pixel and 70 of 64-pixel detectors, with each residual, timed at every
+// split (4 to 384 angles, 9 to 400 scans, objects of 19 to 256; rms 9 to 11 %).
+// Against the wave rule with k_ptycho_adj_few alone, 520 further calls with each
+// residual: mean time 0.80 / 0.73 / 0.77 of it (none, Poisson, Gaussian) at 16
+// pixels, 0.71 / 0.58 / 0.64 at 32 and 0.71 / 0.58 / 0.64 at 64; 61 of 1560 take
+// 3 % more or worse, at most one launch step of 2 us or 1.17 times.  One choice
+// for all residuals and probes had 207, up to 1.6 times.
+// Det 128, one block per SM: 45 angles with 100 to 400 scans:
 // 6 parts and the angles with most scans first instead of 3 parts in angle
 // order, Gaussian gradient 1.48 -> 1.09 ms, Poisson 1.43 -> 0.90 ms.
-struct Split {
-    int parts;
-    bool few;
-};
-Split choose_split(const pt_ptycho &h, const std::vector<int> *counts, size_t most)
+Split choose_split(const pt_ptycho &h, int resid, const std::vector<int> *counts, size_t most)
 {
     const double cells = (double)h.nz * h.n;
-    Split best_split = {1, false};
+    const bool full = h.P == h.det;
+    const int scans = counts ? std::max(counts->front(), 1) : h.nscan;   // of the angle that has most
+    Split best_split;
     double best = 1e300;
     auto time = [&](int p, const Residency &res) {
         const size_t slots = (size_t)h.nsm * res.blocks;
@@ -1607,10 +1633,10 @@ Split choose_split(const pt_ptycho &h, const std::vector<int> *counts, size_t mo
         auto block = [&](int scans, size_t sharing) {   // sharing: blocks on the SM
             const double trips = std::ceil((double)scans / (p * res.frames));
             return std::max(c.clear * cells / res.threads, passes * sharing * c.clear_sm * cells) +
-                   trips * std::max(c.lone, (double)sharing * res.frames * c.frame);
+                   trips * std::hypot(c.lone[resid][full], (double)sharing * res.frames * c.frame[resid][full]);
         };
         auto sharing = [&](size_t n) { return (std::min(n, slots) + h.nsm - 1) / h.nsm; };
-        const double sum = c.fixed + (p > 1 ? c.sum + c.sum_cell * cells * h.ntheta * (p + 1) : 0);
+        const double sum = c.fixed + (p > 1 ? c.sum + c.sum_part * p + c.sum_cell * cells * h.ntheta * (p + 1) : 0);
         double end = 0;
         if (!counts) {
             const size_t waves = blocks / slots, rest = blocks % slots;
@@ -1621,7 +1647,7 @@ Split choose_split(const pt_ptycho &h, const std::vector<int> *counts, size_t mo
             const size_t R = sharing(blocks);
             double all = 0;
             for (int n : *counts) all += p * block(n, R);
-            if (all / slots + sum >= best) return 1e300;   // no placement ends early enough
+            if (0.93 * (all / slots + sum) >= best) return 1e300;   // no placement ends early enough
             std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
             for (int n : *counts)
                 for (int k = 0; k < p; ++k) {
@@ -1637,18 +1663,35 @@ Split choose_split(const pt_ptycho &h, const std::vector<int> *counts, size_t mo
         return end + sum;
     };
     for (const bool few : {false, true}) {
-        if (few && h.det > 32) break;
+        if (few && h.det > 64) break;
         const Residency res = few ? residency_few(h.det) : residency(h.det);
         for (int p : {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 24, 32, 48, 64}) {
             const size_t blocks = (size_t)h.ntheta * p;
-            if (p > h.nscan || (size_t)p > most) break;
+            if (p > scans || (size_t)p > most) break;
             if (p > 16 && (h.det == 128 || blocks > (size_t)h.nsm * res.blocks || blocks * cells > (1u << 27))) break;
             const double end = time(p, res);
             if (end < best - 1e-9) {
                 best = end;
-                best_split = {p, few};
+                best_split.parts = p, best_split.few = few;
             }
         }
+    }
+    if (h.det <= 64) {
+        // a modelled gain of less than 7 % is within the model's error: then the
+        // split by whole waves of a block per SM, 3 % for each further part, in
+        // k_ptycho_adj_few
+        double least = 1e300;
+        int p0 = 1;
+        for (int p = 1; p <= std::min(scans, 16) && (size_t)p <= most; ++p) {
+            const double waves = std::ceil((double)h.ntheta * p / h.nsm);
+            const double cost = waves * std::ceil((double)scans / p) * (1.0 + 0.03 * (p - 1));
+            if (cost < least - 1e-9) {
+                least = cost;
+                p0 = p;
+            }
+        }
+        const double end = time(p0, residency_few(h.det));
+        if (best > 0.93 * end) best_split.parts = p0, best_split.few = true;
     }
     return best_split;
 }
@@ -1661,22 +1704,30 @@ void release_slabs(pt_ptycho *h)
     h->slabs_used = false;
 }
 
-// Uses `parts` parts from now on, with slabs for them; one part if they do not fit.
-bool set_parts(pt_ptycho *h, int parts)
+// Uses these splits from now on, with slabs for them; one part if they do not fit.
+bool use_splits(pt_ptycho *h, const Split (&split)[3])
 {
+    const int parts = std::max({split[0].parts, split[1].parts, split[2].parts});
+    std::copy(split, split + 3, h->split);
     if (parts > 1 && (size_t)parts > h->slabs) {
         release_slabs(h);
         if (cudaMalloc((void **)&h->partial, (size_t)parts * h->ntheta * h->nz * h->n * sizeof(float2)) !=
             cudaSuccess) {
             cudaGetLastError();
             h->partial = nullptr;
-            h->parts = 1;
+            for (Split &s : h->split) s.parts = 1;
             return false;
         }
         h->slabs = parts;
     }
-    h->parts = parts;
     return true;
+}
+// The same number of parts with every residual.
+bool set_parts(pt_ptycho *h, int parts)
+{
+    Split split[3];
+    for (int r = 0; r < 3; ++r) split[r] = {parts, h->split[r].few};
+    return use_splits(h, split);
 }
 
 void ptycho_free(pt_ptycho *h)
@@ -1843,14 +1894,13 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
     h->nsm = nsm;
     // PT_PTYCHO_ADJ_PARTS=<k> overrides the choice (tuning)
-    h->parts = 1;
     const char *env_parts = getenv("PT_PTYCHO_ADJ_PARTS");
     int parts = 1;
     if (env_parts && atoi(env_parts) >= 1) {
         parts = std::min<int>(atoi(env_parts), (int)nscan);
         h->parts_set = true;
     } else if (detx >= 16) {
-        h->parts = choose_split(*h, nullptr, SIZE_MAX).parts;   // setobj chooses again, for the scans that are there
+        h->split[0].parts = choose_split(*h, 0, nullptr, SIZE_MAX).parts;   // setobj chooses, for the scans that are there
     }
     // the small tables are cuts of one allocation, each on a 256-byte boundary
     const size_t P2 = nprb * nprb, nf = ntheta * nscan;
@@ -1967,9 +2017,10 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
         std::sort(counts.begin(), counts.end(), std::greater<int>());
         const bool even = counts.front() == h->nscan && counts.back() == h->nscan;
         auto choose = [&](size_t most) {
-            const Split split = choose_split(*h, even ? nullptr : &counts, most);
-            h->few = split.few;
-            return set_parts(h, split.parts);
+            Split split[3];
+            for (int r = 0; r < 3; ++r)
+                split[r] = r > 0 && h->det == 128 ? split[0] : choose_split(*h, r, even ? nullptr : &counts, most);
+            return use_splits(h, split);
         };
         // never more parts than slabs that a launch has used hold: those stay
         // (one part if new ones cannot be allocated)
@@ -2014,7 +2065,7 @@ extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int tria
     pt::clear_error();
     PT_CHECK_ARG(h && f && g && trials >= 1, "ptychofft.autotune: bad arguments");
     if (h->det < 16) {   // the small-detector kernel has no angle split
-        if (parts_out) *parts_out = h->parts;
+        if (parts_out) *parts_out = h->split[0].parts;
         return PT_OK;
     }
     cudaStream_t st = (cudaStream_t)stream;
@@ -2022,7 +2073,7 @@ extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int tria
     PT_CUDA(cudaEventCreate(&e0));
     PT_CUDA(cudaEventCreate(&e1));
     const int cands[] = {1, 2, 3, 4, 6, 8, 12, 16};
-    int best_p = h->parts;
+    int best_p = h->split[0].parts;
     float best_t = 1e30f;
     int rc = PT_OK;
     for (int p : cands) {
@@ -2055,7 +2106,7 @@ extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int tria
         pt::set_error("ptychofft.autotune: the chosen split's slabs could not be allocated");
         return PT_ERR_ALLOC;
     }
-    if (parts_out) *parts_out = h->parts;
+    if (parts_out) *parts_out = h->split[0].parts;
     return rc;
 }
 
@@ -2064,7 +2115,7 @@ extern "C" int pt_ptycho_set_parts(pt_ptycho *h, int parts)
     pt::clear_error();
     PT_CHECK_ARG(h && parts >= 1 && (size_t)parts <= h->nscan, "ptychofft.set_parts: parts must be in [1, nscan]");
     if (h->det < 16) {
-        PT_CHECK_ARG(parts == h->parts, "ptychofft.set_parts: the small-detector kernel has no angle split");
+        PT_CHECK_ARG(parts == h->split[0].parts, "ptychofft.set_parts: the small-detector kernel has no angle split");
         return PT_OK;
     }
     release_slabs(h);
@@ -2080,7 +2131,7 @@ extern "C" int pt_ptycho_get_parts(const pt_ptycho *h, int *parts)
 {
     pt::clear_error();
     PT_CHECK_ARG(h && parts, "ptychofft: null pointer");
-    *parts = h->parts;
+    *parts = h->split[0].parts;
     return PT_OK;
 }
 

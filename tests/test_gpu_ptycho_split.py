@@ -47,8 +47,7 @@ def test_setobj_leaves_the_slabs_of_a_captured_adjoint(nt, nz, n, ns, det, P, fe
     fresh.setobj(T(full), T(prb))
     op = ptychofft(nt, nz, n, nt, ns, det, det, P)
     op.setobj(T(part), T(prb))
-    before = op.parts
-    assert 1 < before < fresh.parts
+    assert 1 < op.parts <= few < fresh.parts     # at most a slab for each scan
     gd = T(g)
     f = torch.empty((nt, nz, n), dtype=torch.complex64, device="cuda")
     s = torch.cuda.Stream()
@@ -61,7 +60,7 @@ def test_setobj_leaves_the_slabs_of_a_captured_adjoint(nt, nz, n, ns, det, P, fe
         op.adj(f, gd)
     scan = T(full)
     op.setobj(scan, T(prb))
-    assert op.parts <= before
+    assert op.parts <= few
     orc = PtychoFFT(nt, nz, n, nt, ns, det, det, P)
     orc.setobj(full, prb)
     ref = orc.adj(g)
@@ -76,3 +75,32 @@ def test_setobj_leaves_the_slabs_of_a_captured_adjoint(nt, nz, n, ns, det, P, fe
     op.setobj(T(part), T(prb))
     op.setobj(scan, T(prb))
     assert op.parts == fresh.parts
+
+
+@pytest.mark.parametrize("nt,nz,n,ns,det,P", [
+    (2, 60, 61, 25, 16, 9), (150, 20, 22, 13, 16, 16),         # both kernels' sizes, with blocks that queue
+    (3, 50, 47, 31, 32, 25), (150, 37, 35, 7, 32, 32),
+    (5, 80, 79, 18, 64, 41), (150, 70, 66, 3, 64, 64), (6, 66, 70, 80, 64, 30)])
+@pytest.mark.parametrize("uneven", [False, True])
+def test_every_residual_has_a_split(nt, nz, n, ns, det, P, uneven):
+    """The plain adjoint and both gradients, each with its own split and kernel.
+    Gradients to 1e-5: the residual of counts within a factor of two of |f|^2 is
+    a quarter of f."""
+    from ptychotomo_b200 import ptychofft
+    rng = np.random.default_rng(det + 7 * ns)
+    scan = scans(rng, nt, nz, n, ns, P, ns)
+    if uneven:
+        for t in range(nt):
+            scan[:, t, rng.integers(0, ns + 1):] = -1
+    prb, h = crand(rng, (P, P)), crand(rng, (nt, ns, det, det))
+    op, orc = ptychofft(nt, nz, n, nt, ns, det, det, P), PtychoFFT(nt, nz, n, nt, ns, det, det, P)
+    op.setobj(T(scan), T(prb))
+    orc.setobj(scan, prb)
+    data = (np.abs(h) ** 2 * rng.uniform(0.25, 0.75, h.shape)).astype(np.float32)
+    f = torch.full((nt, nz, n), float("nan"), dtype=torch.complex64, device="cuda")
+    op.adj(f, T(h))
+    assert rel(f.cpu().numpy(), orc.adj(h)) <= 4e-6
+    for model, r in ((0, h - data * h / np.abs(h) ** 2), (1, h - np.sqrt(data) * np.exp(1j * np.angle(h)))):
+        f.fill_(float("nan"))
+        op.adj_resid(f, T(h), T(data), 1.0, model)
+        assert rel(f.cpu().numpy(), orc.adj(r)) <= 1e-5
