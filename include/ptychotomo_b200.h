@@ -175,10 +175,13 @@ int pt_ptycho_fwd_probe(pt_ptycho *h, void *g, const void *psi, const void *prb,
  * wave-count model).  f, g: caller buffers of the adjoint's shapes (f is
  * overwritten).  Allocates the slabs; blocks the host. */
 int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int trials, int *parts_out, void *stream);
-/* Sets the adjoint's split (1 <= parts <= Nscan; detectors below 16 keep
- * their one split) and allocates its slabs.  This call and the autotuner free
- * the slabs that were there: an adjoint captured in a graph before them must
- * not be replayed. */
+/* Sets the adjoint's split for every residual (1 <= parts <= Nscan; detectors
+ * below 16 keep their one split) and allocates its slabs; for detectors of 16
+ * to 64 the kernel is the one that suits this split, as it is where
+ * PT_PTYCHO_ADJ_PARTS in the environment of pt_ptycho_create sets it
+ * (PT_PTYCHO_ADJ_FEW=0 or 1 there: the kernel for many or for few frames).
+ * This call and the autotuner free the slabs that were there: an adjoint
+ * captured in a graph before them must not be replayed. */
 int pt_ptycho_set_parts(pt_ptycho *h, int parts);
 /* The adjoint's current split (the residual adjoints may have their own). */
 int pt_ptycho_get_parts(const pt_ptycho *h, int *parts);

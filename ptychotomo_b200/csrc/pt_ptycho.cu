@@ -1287,7 +1287,9 @@ struct pt_ptycho {
     int *angles = nullptr;
     std::vector<int> order;
     bool ordered = false;       // that order is not 0, 1, 2, ...
-    bool parts_set = false;     // the split was chosen by the caller, the autotuner or the environment
+    std::vector<int> counts;    // the scans of each angle that are not skipped, most first; empty: all
+    int parts_set = 0;          // the parts that the caller, the autotuner or the environment set; 0: chosen
+    int few_set = -1;           // k_ptycho_adj_few: 1 always, 0 never, -1 chosen
     // slabs per angle that `partial` holds, and whether a launch has used them:
     // a captured graph may hold their address, so setobj leaves them where they are
     size_t slabs = 0;
@@ -1602,11 +1604,11 @@ Residency residency_few(int det)
 //              sqrt(lone^2 + (R frames)^2) each: a few blocks wait on latency,
 //              many on the SM;
 //   the sum    of more than one part reads every slab once, after a launch.
-// counts: the scans of each angle that are not skipped, in launch order, where
-// they differ: the blocks are then placed on the SMs one by one; else whole
-// waves of equal blocks and what is left.
+// Where the angles have different numbers of scans (h.counts) the blocks are
+// placed on the SMs one by one; else whole waves of equal blocks and what is left.
 // No more parts than an angle has scans, or than `most`; more than 16 only while
-// all blocks run at once and their slabs take at most 1 GiB.
+// all blocks run at once and their slabs take at most 1 GiB.  only > 0: that
+// number of parts, and the kernel for it.
 // The costs are least-squares fits, of the logarithm, to 335 calls of 16- and
 // 32-pixel and 70 of 64-pixel detectors, with each residual, timed at every
 // split (4 to 384 angles, 9 to 400 scans, objects of 19 to 256; rms 9 to 11 %).
@@ -1618,11 +1620,12 @@ Residency residency_few(int det)
 // Det 128, one block per SM: 45 angles with 100 to 400 scans:
 // 6 parts and the angles with most scans first instead of 3 parts in angle
 // order, Gaussian gradient 1.48 -> 1.09 ms, Poisson 1.43 -> 0.90 ms.
-Split choose_split(const pt_ptycho &h, int resid, const std::vector<int> *counts, size_t most)
+Split choose_split(const pt_ptycho &h, int resid, size_t most, int only = 0)
 {
     const double cells = (double)h.nz * h.n;
     const bool full = h.P == h.det;
-    const int scans = counts ? std::max(counts->front(), 1) : h.nscan;   // of the angle that has most
+    const int scans = h.counts.empty() ? h.nscan : std::max(h.counts.front(), 1);   // of the angle that has most
+    const bool few_can = h.det >= 16 && h.det <= 64;
     Split best_split;
     double best = 1e300;
     auto time = [&](int p, const Residency &res) {
@@ -1638,18 +1641,18 @@ Split choose_split(const pt_ptycho &h, int resid, const std::vector<int> *counts
         auto sharing = [&](size_t n) { return (std::min(n, slots) + h.nsm - 1) / h.nsm; };
         const double sum = c.fixed + (p > 1 ? c.sum + c.sum_part * p + c.sum_cell * cells * h.ntheta * (p + 1) : 0);
         double end = 0;
-        if (!counts) {
+        if (h.counts.empty()) {
             const size_t waves = blocks / slots, rest = blocks % slots;
             end = waves * block(h.nscan, res.blocks) + (rest ? block(h.nscan, sharing(rest)) : 0);
         } else if (blocks <= slots) {   // all at once: the one with most scans ends last
-            end = block(counts->front(), sharing(blocks));
+            end = block(h.counts.front(), sharing(blocks));
         } else {
             const size_t R = sharing(blocks);
             double all = 0;
-            for (int n : *counts) all += p * block(n, R);
+            for (int n : h.counts) all += p * block(n, R);
             if (0.93 * (all / slots + sum) >= best) return 1e300;   // no placement ends early enough
             std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
-            for (int n : *counts)
+            for (int n : h.counts)
                 for (int k = 0; k < p; ++k) {
                     double start = 0;
                     if (ends.size() == slots) {
@@ -1663,26 +1666,31 @@ Split choose_split(const pt_ptycho &h, int resid, const std::vector<int> *counts
         return end + sum;
     };
     for (const bool few : {false, true}) {
-        if (few && h.det > 64) break;
+        if ((few && !few_can) || (few_can && h.few_set == !few)) continue;
         const Residency res = few ? residency_few(h.det) : residency(h.det);
         for (int p : {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 20, 24, 32, 48, 64}) {
             const size_t blocks = (size_t)h.ntheta * p;
-            if (p > scans || (size_t)p > most) break;
-            if (p > 16 && (h.det == 128 || blocks > (size_t)h.nsm * res.blocks || blocks * cells > (1u << 27))) break;
+            if (only)
+                p = only;
+            else if (p > scans || (size_t)p > most)
+                break;
+            else if (p > 16 && (h.det == 128 || blocks > (size_t)h.nsm * res.blocks || blocks * cells > (1u << 27)))
+                break;
             const double end = time(p, res);
             if (end < best - 1e-9) {
                 best = end;
                 best_split.parts = p, best_split.few = few;
             }
+            if (only) break;
         }
     }
-    if (h.det <= 64) {
+    if (few_can && h.few_set != 0) {
         // a modelled gain of less than 7 % is within the model's error: then the
         // split by whole waves of a block per SM, 3 % for each further part, in
         // k_ptycho_adj_few
         double least = 1e300;
-        int p0 = 1;
-        for (int p = 1; p <= std::min(scans, 16) && (size_t)p <= most; ++p) {
+        int p0 = only ? only : 1;
+        for (int p = 1; !only && p <= std::min(scans, 16) && (size_t)p <= most; ++p) {
             const double waves = std::ceil((double)h.ntheta * p / h.nsm);
             const double cost = waves * std::ceil((double)scans / p) * (1.0 + 0.03 * (p - 1));
             if (cost < least - 1e-9) {
@@ -1722,11 +1730,11 @@ bool use_splits(pt_ptycho *h, const Split (&split)[3])
     }
     return true;
 }
-// The same number of parts with every residual.
+// The same number of parts with every residual, in the kernel that suits it.
 bool set_parts(pt_ptycho *h, int parts)
 {
     Split split[3];
-    for (int r = 0; r < 3; ++r) split[r] = {parts, h->split[r].few};
+    for (int r = 0; r < 3; ++r) split[r] = choose_split(*h, r, SIZE_MAX, parts);
     return use_splits(h, split);
 }
 
@@ -1893,15 +1901,14 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
     h->nsm = nsm;
-    // PT_PTYCHO_ADJ_PARTS=<k> overrides the choice (tuning)
-    const char *env_parts = getenv("PT_PTYCHO_ADJ_PARTS");
-    int parts = 1;
-    if (env_parts && atoi(env_parts) >= 1) {
-        parts = std::min<int>(atoi(env_parts), (int)nscan);
-        h->parts_set = true;
-    } else if (detx >= 16) {
-        h->split[0].parts = choose_split(*h, 0, nullptr, SIZE_MAX).parts;   // setobj chooses, for the scans that are there
-    }
+    // PT_PTYCHO_ADJ_PARTS=<k> overrides the choice of the parts, PT_PTYCHO_ADJ_FEW=0
+    // or 1 that of the kernel (tuning and tests)
+    const char *env_parts = getenv("PT_PTYCHO_ADJ_PARTS"), *env_few = getenv("PT_PTYCHO_ADJ_FEW");
+    if (env_few) h->few_set = atoi(env_few) != 0;
+    if (env_parts && atoi(env_parts) >= 1)
+        h->parts_set = std::min<int>(atoi(env_parts), (int)nscan);
+    else if (detx >= 16)
+        h->split[0].parts = choose_split(*h, 0, SIZE_MAX).parts;   // setobj chooses, for the scans that are there
     // the small tables are cuts of one allocation, each on a 256-byte boundary
     const size_t P2 = nprb * nprb, nf = ntheta * nscan;
     size_t used = 0;
@@ -1922,7 +1929,7 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
         used += (count * sizeof(*p) + 255) / 256 * 256;
     };
     cuts(place);
-    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && (!h->parts_set || set_parts(h, parts));
+    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && (!h->parts_set || set_parts(h, h->parts_set));
     if (ok) cuts(place);
     // probe adjoint: one partial per frame in flight
     const Residency res = residency((int)detx);
@@ -2013,13 +2020,15 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
         PT_CUDA(cudaStreamSynchronize(st));
         h->order = order;
     }
-    if (!h->parts_set && h->det >= 16) {
-        std::sort(counts.begin(), counts.end(), std::greater<int>());
-        const bool even = counts.front() == h->nscan && counts.back() == h->nscan;
+    std::sort(counts.begin(), counts.end(), std::greater<int>());
+    if (counts.back() == h->nscan) counts.clear();
+    h->counts = counts;
+    if (h->parts_set > 0) {   // the kernels for it may change with the scans
+        for (int r = 0; r < 3; ++r) h->split[r].few = choose_split(*h, r, SIZE_MAX, h->split[r].parts).few;
+    } else if (h->parts_set == 0 && h->det >= 16) {
         auto choose = [&](size_t most) {
             Split split[3];
-            for (int r = 0; r < 3; ++r)
-                split[r] = r > 0 && h->det == 128 ? split[0] : choose_split(*h, r, even ? nullptr : &counts, most);
+            for (int r = 0; r < 3; ++r) split[r] = r > 0 && h->det == 128 ? split[0] : choose_split(*h, r, most);
             return use_splits(h, split);
         };
         // never more parts than slabs that a launch has used hold: those stay
@@ -2101,7 +2110,7 @@ extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int tria
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     release_slabs(h);   // the largest candidate's
-    h->parts_set = true;
+    h->parts_set = best_p;
     if (!set_parts(h, best_p)) {
         pt::set_error("ptychofft.autotune: the chosen split's slabs could not be allocated");
         return PT_ERR_ALLOC;
@@ -2119,7 +2128,7 @@ extern "C" int pt_ptycho_set_parts(pt_ptycho *h, int parts)
         return PT_OK;
     }
     release_slabs(h);
-    h->parts_set = true;
+    h->parts_set = parts;
     if (!set_parts(h, parts)) {
         pt::set_error("ptychofft.set_parts: the split's slabs could not be allocated");
         return PT_ERR_ALLOC;

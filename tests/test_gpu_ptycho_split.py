@@ -104,3 +104,76 @@ def test_every_residual_has_a_split(nt, nz, n, ns, det, P, uneven):
         f.fill_(float("nan"))
         op.adj_resid(f, T(h), T(data), 1.0, model)
         assert rel(f.cpu().numpy(), orc.adj(r)) <= 1e-5
+
+
+def adjoints(op, h, data, shape):
+    """The adjoint and both gradients."""
+    out = []
+    for run in (lambda f: op.adj(f, h), lambda f: op.adj_resid(f, h, data, 1.0, 0), lambda f: op.adj_resid(f, h, data, 1.0, 1)):
+        f = torch.full(shape, float("nan"), dtype=torch.complex64, device="cuda")
+        run(f)
+        out.append(f)
+    return out
+
+
+FORCED = [(1, 20, 19, 1, 16, 7, 1), (3, 40, 33, 3, 16, 16, 2), (2, 40, 37, 5, 32, 1, 5), (2, 41, 40, 4, 32, 31, 3),
+          (3, 50, 70, 7, 32, 32, 4), (1, 70, 66, 1, 64, 16, 1), (2, 66, 70, 6, 64, 33, 5), (2, 70, 71, 3, 64, 63, 1),
+          (2, 90, 64, 9, 64, 64, 2)]
+
+
+@pytest.mark.parametrize("nt,nz,n,ns,det,P,parts", FORCED)
+def test_both_kernels_at_forced_splits(nt, nz, n, ns, det, P, parts, monkeypatch):
+    """Gradients to 1e-5, as above.  The sub-pixel model's adjoint in one kernel
+    against the other."""
+    from ptychotomo_b200 import ptychofft
+    rng = np.random.default_rng(det + P)
+    scan = scans(rng, nt, nz, n, ns, P, ns)
+    if ns > 2:
+        scan[:, 0, 1] = -1
+    prb, h = crand(rng, (P, P)), crand(rng, (nt, ns, det, det))
+    data = (np.abs(h) ** 2 * rng.uniform(0.25, 0.75, h.shape)).astype(np.float32)
+    orc = PtychoFFT(nt, nz, n, nt, ns, det, det, P)
+    orc.setobj(scan, prb)
+    ref = [orc.adj(r) for r in (h, h - data * h / np.abs(h) ** 2, h - np.sqrt(data) * np.exp(1j * np.angle(h)))]
+    monkeypatch.setenv("PT_PTYCHO_ADJ_PARTS", str(parts))
+    sub = []
+    for few in ("0", "1"):
+        monkeypatch.setenv("PT_PTYCHO_ADJ_FEW", few)
+        op = ptychofft(nt, nz, n, nt, ns, det, det, P)
+        op.setobj(T(scan), T(prb))
+        assert op.parts == parts
+        for got, want, tol in zip(adjoints(op, T(h), T(data), (nt, nz, n)), ref, (4e-6, 1e-5, 1e-5)):
+            assert rel(got.cpu().numpy(), want) <= tol
+        op.set_subpixel(8)
+        sub.append(adjoints(op, T(h), T(data), (nt, nz, n)))
+    for a, b, tol in zip(*sub, (4e-6, 1e-5, 1e-5)):
+        assert rel(a.cpu().numpy(), b.cpu().numpy()) <= tol
+
+
+@pytest.mark.parametrize("nt,nz,n,ns,det,P", [(9, 36, 50, 36, 16, 16), (150, 30, 31, 40, 16, 9), (40, 40, 41, 20, 32, 29),
+                                              (30, 70, 66, 12, 64, 41), (3, 131, 130, 9, 128, 100)])
+@pytest.mark.parametrize("valid", [0.5, 1.0])
+def test_a_split_is_the_same_however_it_is_set(nt, nz, n, ns, det, P, valid, monkeypatch):
+    """By the environment, by the property before and after setobj: the same bits."""
+    from ptychotomo_b200 import ptychofft
+    rng = np.random.default_rng(nt + det)
+    scan = scans(rng, nt, nz, n, ns, P, int(valid * ns))
+    prb, h = crand(rng, (P, P)), T(crand(rng, (nt, ns, det, det)))
+    data = h.abs().square() * 0.5
+    for parts in (1, 3, ns):
+        ops = []
+        with monkeypatch.context() as m:
+            m.setenv("PT_PTYCHO_ADJ_PARTS", str(parts))
+            ops.append(ptychofft(nt, nz, n, nt, ns, det, det, P))
+            ops[0].setobj(T(scan), T(prb))
+        for before in (True, False):
+            ops.append(ptychofft(nt, nz, n, nt, ns, det, det, P))
+            if before:
+                ops[-1].parts = parts
+            ops[-1].setobj(T(scan), T(prb))
+            if not before:
+                ops[-1].parts = parts
+        assert [op.parts for op in ops] == [parts] * 3
+        a, b, c = (adjoints(op, h, data, (nt, nz, n)) for op in ops)
+        for x, y, z in zip(a, b, c):
+            assert torch.equal(x, y) and torch.equal(x, z)

@@ -45,11 +45,13 @@ def test_residual_over_the_range(model):
     check(out.cpu().numpy(), x, d, model)
 
 
-def one_value_frames(x, d, det, P, model, env, monkeypatch):
+def one_value_frames(x, d, det, P, model, parts, few, monkeypatch):
     """adj_resid of one frame per (x, d), over disjoint patches: [frame, P, P]."""
     from ptychotomo_b200 import ptychofft
-    if env:
-        monkeypatch.setenv("PT_PTYCHO_ADJ_PARTS", env)
+    if parts:
+        monkeypatch.setenv("PT_PTYCHO_ADJ_PARTS", parts)
+    if few:
+        monkeypatch.setenv("PT_PTYCHO_ADJ_FEW", few)
     side, k = 4, 12
     assert len(x) % k == 0
     nt, n, nz = len(x) // k, side * P, -(-k // side) * P
@@ -66,25 +68,26 @@ def one_value_frames(x, d, det, P, model, env, monkeypatch):
     return f.cpu().numpy().astype(np.complex128) * det
 
 
-FRAMES = [(16, 16, None), (16, 16, "1"), (16, 9, "1"), (32, 32, "2"), (32, 11, "1"), (64, 64, None), (64, 33, None),
-          (64, 32, "1"), (128, 128, None), (128, 100, "1")]
+# detector, probe, number of parts, kernel for few frames or not (None: chosen)
+FRAMES = [(16, 16, None, "1"), (16, 16, "1", "0"), (16, 9, "1", "0"), (32, 32, "2", "0"), (32, 11, "1", "0"), (32, 20, None, "1"),
+          (64, 64, None, "0"), (64, 33, None, "0"), (64, 32, "1", "1"), (128, 128, None, None), (128, 100, "1", None)]
 
 
-@pytest.mark.parametrize("det,P,env", FRAMES)
+@pytest.mark.parametrize("det,P,parts,few", FRAMES)
 @pytest.mark.parametrize("model", [0, 1])
-def test_gradient_residual_over_the_range(det, P, env, model, monkeypatch):
+def test_gradient_residual_over_the_range(det, P, parts, few, model, monkeypatch):
     x, d = np.repeat(X, len(D)), np.tile(D, len(X))
-    got = one_value_frames(x, d, det, P, model, env, monkeypatch)
+    got = one_value_frames(x, d, det, P, model, parts, few, monkeypatch)
     for i, j in ((0, 0), (P - 1, 0), (P // 2, P - 1)):
         check(got[:, i, j], x, d, model, floor=det * 2.0 ** -126)
 
 
-@pytest.mark.parametrize("det,P,env", FRAMES)
-def test_counts_that_are_not_numbers_stay_visible(det, P, env, monkeypatch):
+@pytest.mark.parametrize("det,P,parts,few", FRAMES)
+def test_counts_that_are_not_numbers_stay_visible(det, P, parts, few, monkeypatch):
     """A count that is NaN or infinite, or negative in the Gaussian model, makes
     its own patch not finite and no other."""
     for model, bad in ((0, [np.nan, np.inf]), (1, [np.nan, np.inf, -1.0])):
         x, d = np.full(24, 0.5 + 1j, np.complex64), np.ones(24, np.float32)
         d[5:5 + len(bad)] = bad
-        got = one_value_frames(x, d, det, P, model, env, monkeypatch)
+        got = one_value_frames(x, d, det, P, model, parts, few, monkeypatch)
         assert (~np.isfinite(got)).all(axis=(1, 2)).tolist() == [not (np.isfinite(v) and v >= 0) for v in d]
