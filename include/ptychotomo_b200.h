@@ -170,9 +170,10 @@ int pt_ptycho_adj_probe_resid64(pt_ptycho *h, void *gprb, const void *psi, const
 int pt_ptycho_fwd_probe(pt_ptycho *h, void *g, const void *psi, const void *prb, float scale, void *stream);
 /* Autotuner (no counterpart in the reference): the adjoint splits each
  * angle's scans over `parts` blocks (own slabs, then a fixed-order sum);
- * times the adjoint for parts in {1, 2, 3, 4, 6, 8, 12, 16} (<= Nscan),
- * `trials` runs each after a warm-up, and keeps the fastest (default: a
- * wave-count model).  f, g: caller buffers of the adjoint's shapes (f is
+ * times the plain adjoint at its present split and for parts in {1, 2, 3, 4,
+ * 6, 8, 12, 16} (<= Nscan), in both kernels for detectors of 16 to 64,
+ * `trials` runs each after a warm-up, and keeps the fastest (default: a time
+ * model); the residual adjoints keep their splits, and setobj this one.  f, g: caller buffers of the adjoint's shapes (f is
  * overwritten).  Allocates the slabs; blocks the host. */
 int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int trials, int *parts_out, void *stream);
 /* Sets the adjoint's split for every residual (1 <= parts <= Nscan; detectors

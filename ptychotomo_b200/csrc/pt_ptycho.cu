@@ -19,6 +19,7 @@
 //  The adjoints also serve the residual-on-load and probe adjoints.
 //  Detector 8x8 uses a plain shared-memory Stockham path.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdlib>
 #include <cstdint>
@@ -1288,7 +1289,7 @@ struct pt_ptycho {
     std::vector<int> order;
     bool ordered = false;       // that order is not 0, 1, 2, ...
     std::vector<int> counts;    // the scans of each angle that are not skipped, most first; empty: all
-    int parts_set = 0;          // the parts that the caller, the autotuner or the environment set; 0: chosen
+    int parts_set = 0;          // the parts that the caller or the environment set; 0: chosen, -1: autotuned
     int few_set = -1;           // k_ptycho_adj_few: 1 always, 0 never, -1 chosen
     // slabs per angle that `partial` holds, and whether a launch has used them:
     // a captured graph may hold their address, so setobj leaves them where they are
@@ -1713,10 +1714,10 @@ void release_slabs(pt_ptycho *h)
 }
 
 // Uses these splits from now on, with slabs for them; one part if they do not fit.
-bool use_splits(pt_ptycho *h, const Split (&split)[3])
+bool use_splits(pt_ptycho *h, std::array<Split, 3> split)
 {
     const int parts = std::max({split[0].parts, split[1].parts, split[2].parts});
-    std::copy(split, split + 3, h->split);
+    std::copy(split.begin(), split.end(), h->split);
     if (parts > 1 && (size_t)parts > h->slabs) {
         release_slabs(h);
         if (cudaMalloc((void **)&h->partial, (size_t)parts * h->ntheta * h->nz * h->n * sizeof(float2)) !=
@@ -1733,7 +1734,7 @@ bool use_splits(pt_ptycho *h, const Split (&split)[3])
 // The same number of parts with every residual, in the kernel that suits it.
 bool set_parts(pt_ptycho *h, int parts)
 {
-    Split split[3];
+    std::array<Split, 3> split;
     for (int r = 0; r < 3; ++r) split[r] = choose_split(*h, r, SIZE_MAX, parts);
     return use_splits(h, split);
 }
@@ -1929,7 +1930,7 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
         used += (count * sizeof(*p) + 255) / 256 * 256;
     };
     cuts(place);
-    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && (!h->parts_set || set_parts(h, h->parts_set));
+    bool ok = cudaMalloc((void **)&h->tables, used) == cudaSuccess && (h->parts_set == 0 || set_parts(h, h->parts_set));
     if (ok) cuts(place);
     // probe adjoint: one partial per frame in flight
     const Residency res = residency((int)detx);
@@ -2027,7 +2028,7 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
         for (int r = 0; r < 3; ++r) h->split[r].few = choose_split(*h, r, SIZE_MAX, h->split[r].parts).few;
     } else if (h->parts_set == 0 && h->det >= 16) {
         auto choose = [&](size_t most) {
-            Split split[3];
+            std::array<Split, 3> split;
             for (int r = 0; r < 3; ++r) split[r] = r > 0 && h->det == 128 ? split[0] : choose_split(*h, r, most);
             return use_splits(h, split);
         };
@@ -2066,9 +2067,10 @@ extern "C" int pt_ptycho_fwd(pt_ptycho *h, void *g, const void *f, void *stream)
     return ptycho_call(h, false, g, f, 1.0f, stream);
 }
 // ---- autotuner: the adjoint's angle split ---------------------------------
-// Times the object adjoint (the CG's dominant kernel) for each candidate
-// number of parts per angle and keeps the fastest.  Setup-time: allocates the
-// partial slabs of each candidate, blocks the host.
+// Times the plain object adjoint (the CG's dominant kernel) at the present split
+// and at others, in both kernels where there are two, and keeps the fastest; the
+// present one unless another is faster.  The residual adjoints keep their splits.
+// Setup-time: allocates the partial slabs of each candidate, blocks the host.
 extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int trials, int *parts_out, void *stream)
 {
     pt::clear_error();
@@ -2081,13 +2083,20 @@ extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int tria
     cudaEvent_t e0, e1;
     PT_CUDA(cudaEventCreate(&e0));
     PT_CUDA(cudaEventCreate(&e1));
-    const int cands[] = {1, 2, 3, 4, 6, 8, 12, 16};
-    int best_p = h->split[0].parts;
+    const Split resid[2] = {h->split[1], h->split[2]};
+    auto use = [&](const Split &plain) { return use_splits(h, {plain, resid[0], resid[1]}); };
+    std::vector<Split> cands = {h->split[0]};
+    const bool few_can = h->det <= 64;
+    for (const bool few : {false, true}) {
+        if ((few && !few_can) || (few_can && h->few_set == !few)) continue;
+        for (int p : {1, 2, 3, 4, 6, 8, 12, 16, h->split[0].parts})
+            if (p <= h->nscan) cands.push_back({p, few});
+    }
+    Split best = cands.front();
     float best_t = 1e30f;
     int rc = PT_OK;
-    for (int p : cands) {
-        if (p > h->nscan) break;
-        if (!set_parts(h, p)) continue;   // this split does not fit: skip it
+    for (const Split &c : cands) {
+        if (!use(c)) continue;   // this split does not fit: skip it
         std::vector<float> ts;
         for (int k = 0; k <= trials && rc == PT_OK; ++k) {   // the first run warms up
             cudaEventRecord(e0, st);
@@ -2099,19 +2108,19 @@ extern "C" int pt_ptycho_autotune(pt_ptycho *h, void *f, const void *g, int tria
                 ts.push_back(ms);
             }
         }
-        if (rc != PT_OK) break;
+        if (rc != PT_OK || ts.empty()) break;
         std::sort(ts.begin(), ts.end());
         const float med = ts[ts.size() / 2];
         if (med < best_t) {
             best_t = med;
-            best_p = p;
+            best = c;
         }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     release_slabs(h);   // the largest candidate's
-    h->parts_set = best_p;
-    if (!set_parts(h, best_p)) {
+    h->parts_set = -1;
+    if (!use(best)) {
         pt::set_error("ptychofft.autotune: the chosen split's slabs could not be allocated");
         return PT_ERR_ALLOC;
     }

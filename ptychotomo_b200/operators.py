@@ -134,9 +134,10 @@ class ptychofft:  # noqa: N801 - reference class name
                   "ptychofft.adj")
 
     def autotune(self, f, g, trials=3, stream=None):
-        """Time the adjoint for each split of an angle's scans over blocks and
-        keep the fastest.  f, g: buffers of adj's shapes (f is overwritten).
-        Returns the chosen number of parts."""
+        """Time the adjoint at its present split of an angle's scans over blocks
+        and at others and keep the fastest (adj_resid keeps its own).  f, g:
+        buffers of adj's shapes (f is overwritten).  Returns the chosen number
+        of parts."""
         out = ctypes.c_int()
         check(lib().pt_ptycho_autotune(self._h, as_ptr(f), as_ptr(g), int(trials), ctypes.byref(out), _s(stream)),
               "ptychofft.autotune")

@@ -177,3 +177,33 @@ def test_a_split_is_the_same_however_it_is_set(nt, nz, n, ns, det, P, valid, mon
         a, b, c = (adjoints(op, h, data, (nt, nz, n)) for op in ops)
         for x, y, z in zip(a, b, c):
             assert torch.equal(x, y) and torch.equal(x, z)
+
+
+@pytest.mark.parametrize("nt,nz,n,ns,det,P", [(4, 60, 61, 325, 16, 10), (60, 40, 41, 40, 32, 29), (6, 80, 79, 18, 64, 41),
+                                              (3, 131, 130, 9, 128, 100)])
+@pytest.mark.parametrize("few", [None, "0"])
+def test_autotuner_starts_from_the_present_split(nt, nz, n, ns, det, P, few, monkeypatch):
+    """The present split is among those timed, so the result is it or one that
+    was faster: never a split that was not offered.  The gradients keep theirs,
+    to the bit, and setobj keeps the tuned one."""
+    from ptychotomo_b200 import ptychofft
+    if few:
+        monkeypatch.setenv("PT_PTYCHO_ADJ_FEW", few)
+    rng = np.random.default_rng(nt + det)
+    scan = scans(rng, nt, nz, n, ns, P, ns)
+    prb, h = crand(rng, (P, P)), crand(rng, (nt, ns, det, det))
+    data = T(h).abs().square() * 0.5
+    op = ptychofft(nt, nz, n, nt, ns, det, det, P)
+    op.setobj(T(scan), T(prb))
+    before, default = adjoints(op, T(h), data, (nt, nz, n)), op.parts
+    f = torch.empty((nt, nz, n), dtype=torch.complex64, device="cuda")
+    tuned = op.autotune(f, T(h), trials=2)
+    assert tuned == op.parts and tuned in (1, 2, 3, 4, 6, 8, 12, 16, default)
+    op.setobj(T(scan[:, :, ::-1].copy()), T(prb))
+    assert op.parts == tuned
+    op.setobj(T(scan), T(prb))
+    after = adjoints(op, T(h), data, (nt, nz, n))
+    orc = PtychoFFT(nt, nz, n, nt, ns, det, det, P)
+    orc.setobj(scan, prb)
+    assert rel(after[0].cpu().numpy(), orc.adj(h)) <= 4e-6
+    assert torch.equal(after[1], before[1]) and torch.equal(after[2], before[2])
