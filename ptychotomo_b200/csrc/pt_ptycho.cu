@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <functional>
 #include <map>
+#include <numeric>
 #include <queue>
 #include <type_traits>
 #include <vector>
@@ -1288,7 +1289,8 @@ struct pt_ptycho {
     int *angles = nullptr;
     std::vector<int> order;
     bool ordered = false;       // that order is not 0, 1, 2, ...
-    std::vector<int> counts;    // the scans of each angle that are not skipped, most first; empty: all
+    std::vector<int> counts;    // the scans of each angle that are not skipped, most first
+    double scans_all = 0;       // their sum
     int parts_set = 0;          // the parts that the caller or the environment set; 0: chosen, -1: autotuned
     int few_set = -1;           // k_ptycho_adj_few: 1 always, 0 never, -1 chosen
     // slabs per angle that `partial` holds, and whether a launch has used them:
@@ -1605,8 +1607,11 @@ Residency residency_few(int det)
 //              sqrt(lone^2 + (R frames)^2) each: a few blocks wait on latency,
 //              many on the SM;
 //   the sum    of more than one part reads every slab once, after a launch.
-// Where the angles have different numbers of scans (h.counts) the blocks are
-// placed on the SMs one by one; else whole waves of equal blocks and what is left.
+// Angles with different numbers of scans: only det 128, whose SMs take few blocks
+// each, has the blocks placed one by one (45 angles: 0.3 ms of setobj; the bound
+// below it costs up to 12 %: 38 x 236 scans 442 -> 494 us).  The others have the
+// bound, which chooses as well as the placement on 119 calls, in constant time
+// (384 angles of 400 scans, 16 x 16: setobj 4.3 -> 1.0 ms).
 // No more parts than an angle has scans, or than `most`; more than 16 only while
 // all blocks run at once and their slabs take at most 1 GiB.  only > 0: that
 // number of parts, and the kernel for it.
@@ -1625,34 +1630,33 @@ Split choose_split(const pt_ptycho &h, int resid, size_t most, int only = 0)
 {
     const double cells = (double)h.nz * h.n;
     const bool full = h.P == h.det;
-    const int scans = h.counts.empty() ? h.nscan : std::max(h.counts.front(), 1);   // of the angle that has most
+    const int most_scans = h.counts.front(), least = h.counts.back(), scans = std::max(most_scans, 1);
     const bool few_can = h.det >= 16 && h.det <= 64;
     Split best_split;
     double best = 1e300;
     auto time = [&](int p, const Residency &res) {
-        const size_t slots = (size_t)h.nsm * res.blocks;
+        const size_t slots = (size_t)h.nsm * res.blocks, blocks = (size_t)h.ntheta * p;
         const SplitCost &c = res.cost;
-        const size_t blocks = (size_t)h.ntheta * p;
+        const double lone = c.lone[resid][full], frame = res.frames * c.frame[resid][full], q = (double)p * res.frames;
         const int passes = h.det == 128 && p > 1 ? 2 : 1;
-        auto block = [&](int scans, size_t sharing) {   // sharing: blocks on the SM
-            const double trips = std::ceil((double)scans / (p * res.frames));
-            return std::max(c.clear * cells / res.threads, passes * sharing * c.clear_sm * cells) +
-                   trips * std::hypot(c.lone[resid][full], (double)sharing * res.frames * c.frame[resid][full]);
-        };
-        auto sharing = [&](size_t n) { return (std::min(n, slots) + h.nsm - 1) / h.nsm; };
-        const double sum = c.fixed + (p > 1 ? c.sum + c.sum_part * p + c.sum_cell * cells * h.ntheta * (p + 1) : 0);
-        double end = 0;
-        if (h.counts.empty()) {
-            const size_t waves = blocks / slots, rest = blocks % slots;
-            end = waves * block(h.nscan, res.blocks) + (rest ? block(h.nscan, sharing(rest)) : 0);
-        } else if (blocks <= slots) {   // all at once: the one with most scans ends last
-            end = block(h.counts.front(), sharing(blocks));
-        } else {
-            const size_t R = sharing(blocks);
-            double all = 0;
-            for (int n : h.counts) all += p * block(n, R);
-            if (0.93 * (all / slots + sum) >= best) return 1e300;   // no placement ends early enough
+        auto clear = [&](size_t R) { return std::max(c.clear * cells / res.threads, passes * R * c.clear_sm * cells); };
+        auto block = [&](int n, size_t R) { return clear(R) + std::ceil(n / q) * std::hypot(lone, R * frame); };
+        auto sharing = [&](size_t n) { return (std::min(n, slots) + h.nsm - 1) / h.nsm; };   // blocks on an SM
+        const size_t R = sharing(blocks);
+        // trips of one block of each angle: every quotient rounded up, by a half on average
+        const double trips = (h.scans_all + h.ntheta * (q - 1) / 2) / q;
+        double end = c.fixed + (p > 1 ? c.sum + c.sum_part * p + c.sum_cell * cells * h.ntheta * (p + 1) : 0);
+        if (least == most_scans) {   // whole waves of equal blocks and what is left
+            const size_t rest = blocks % slots;
+            end += blocks / slots * block(most_scans, res.blocks) + (rest ? block(most_scans, sharing(rest)) : 0);
+        } else if (blocks <= slots) {   // all at once: the longest block, while the others end
+            end += clear(R) + std::hypot(std::ceil(most_scans / q) * lone, frame * trips * R / h.ntheta);
+        } else if (h.det < 128) {   // most scans first: the SMs end together, but for a part of the shortest block
+            const double all = p * (h.ntheta * clear(R) + trips * std::hypot(lone, R * frame));
+            end += std::max(block(most_scans, R), all / slots + 0.5 * block(least, R));
+        } else {   // one block after the other goes to the SM that is free first
             std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
+            double last = 0;
             for (int n : h.counts)
                 for (int k = 0; k < p; ++k) {
                     double start = 0;
@@ -1661,10 +1665,11 @@ Split choose_split(const pt_ptycho &h, int resid, size_t most, int only = 0)
                         ends.pop();
                     }
                     ends.push(start + block(n, R));
-                    end = std::max(end, start + block(n, R));
+                    last = std::max(last, start + block(n, R));
                 }
+            end += last;
         }
-        return end + sum;
+        return end;
     };
     for (const bool few : {false, true}) {
         if ((few && !few_can) || (few_can && h.few_set == !few)) continue;
@@ -1894,6 +1899,8 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
     h->det = (int)detx;
     h->P = (int)nprb;
     h->c = 1 / sqrtf(detx * dety);  // kernels.cuh:260
+    h->counts.assign(h->ntheta, h->nscan);
+    h->scans_all = (double)h->ntheta * h->nscan;
     if (cudaGetDevice(&h->device) != cudaSuccess) {
         delete h;
         pt::set_error("ptychofft: no CUDA device");
@@ -2022,8 +2029,8 @@ extern "C" int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb
         h->order = order;
     }
     std::sort(counts.begin(), counts.end(), std::greater<int>());
-    if (counts.back() == h->nscan) counts.clear();
     h->counts = counts;
+    h->scans_all = std::accumulate(counts.begin(), counts.end(), 0.0);
     if (h->parts_set > 0) {   // the kernels for it may change with the scans
         for (int r = 0; r < 3; ++r) h->split[r].few = choose_split(*h, r, SIZE_MAX, h->split[r].parts).few;
     } else if (h->parts_set == 0 && h->det >= 16) {
