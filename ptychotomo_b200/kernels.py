@@ -108,7 +108,7 @@ class Reducer:
     def _steps(self, gammas):
         """Device address of the step lengths: inside the table of halvings, or a copy."""
         J = len(gammas)
-        if gammas[0] > 0 and math.frexp(gammas[0])[0] == 0.5 and all(b == 0.5 * a for a, b in zip(gammas, gammas[1:])):
+        if J and gammas[0] > 0 and math.frexp(gammas[0])[0] == 0.5 and all(b == 0.5 * a for a, b in zip(gammas, gammas[1:])):
             k = 2 - math.frexp(gammas[0])[1]          # gammas[0] = 2^(1 - k)
             if 0 <= k and k + J <= len(self.halvings):
                 return self.halvings.data_ptr() + 8 * k
