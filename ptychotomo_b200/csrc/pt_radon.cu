@@ -369,9 +369,9 @@ __global__ void __launch_bounds__(GPB *ZC, 4)
 // once, and gathers from there.  Weights, loads and the order of the sums are
 // those of k_fwd_gather_pts, so the results are bit-identical.
 // points per block of the tiled gather: up to 128 wide there are too few blocks
-// of 128 points to fill the GPU evenly (64^3 forward 64 -> 53 us, 128^3 208 ->
-// 204); at 256 wide half-empty blocks cost more than they balance (1.42 and
-// 1.45 ms)
+// of 128 points to fill the GPU evenly (64 wide, 64 slices, 96 angles 56 -> 50
+// us; 128^3, 128 angles 177 -> 171); at 256 wide half-empty blocks cost more than
+// they balance (256^3, 384 angles 1.36 and 1.39 ms)
 template <int N>
 constexpr int tile_points() { return N <= 192 ? 64 : 128; }
 template <int W>
@@ -538,10 +538,15 @@ __global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
 // K3a and K3b in one launch for short lines: a block gathers the N points of
 // one angle through L1 into shared memory and transforms them (the same sums
 // and rounds as k_fwd_gather_pts and k_fwd_lines).  rec is in point order.
-// One launch and one pass over the lines buffer less: 32 wide, 9 slices 24.8 ->
-// 20.9 us (bound by the launches), 64^3 61 -> 58 us.  From 128 wide the tiles in
-// shared memory win.
-constexpr int FUSED_N = 96;   // longest line (64 wide)
+// One launch and one pass over the lines buffer less, but the grid is read
+// through L1.  32 wide, against the tiles in shared memory (us): 8 slices, 96
+// angles 16.4 and 18.4; 256 slices, 96 angles 151 and 164; where all the blocks
+// of the pipelines are more than FUSED_BLOCKS the tiles win: 32 slices, 192
+// angles 27.9 and 23.6; 16 slices, 384 angles 26.7 and 22.6 (8 slices, 384
+// angles: 18.5 and 20.5).  64 wide the tiles win at every size (8 slices, 24
+// angles 21.3 and 18.5; 64 slices, 96 angles 59 and 50).
+constexpr int FUSED_N = 48;   // longest line (32 wide)
+constexpr int FUSED_BLOCKS = 384;
 template <int N, int W>
 __global__ void __launch_bounds__(GPB *ZC, 4)
     k_fwd_gather_lines(const float2 *__restrict__ fg, size_t set, const float4 *__restrict__ rec,
@@ -977,7 +982,7 @@ float radon_pre(const pt_radon *h)
     return s / (float)h->N;
 }
 
-// Tensor maps of the two haloed grid buffers for k_fwd_gather_tma: float32,
+// Tensor maps of the haloed grid buffers (RSETS) for k_fwd_gather_tma: float32,
 // dims (innermost first) {ZC * 4 floats = one column pair of the chunk's
 // slices, G/2 + GH_PAIRS pairs, G + GH_ROWS rows}, row-major strides
 // {ZC * 16, (G/2 + GH_PAIRS) * ZC * 16} bytes, box {ZC * 4, TILE_PAIRS, tile_rows}: the
@@ -1085,7 +1090,7 @@ int run_fwd(pt_radon *h, float2 *g, const float2 *f, float scale, cudaStream_t s
             k_fwd_gather_tile<N, W><<<dim3(h->nchunks, cnt), GPB * ZC, tile_smem<N, W>(), s>>>(fg, stride, ln, h->rec,
                                                                                            h->chunks, npts);
             PT_LAUNCHED("k_fwd_gather_tile");
-        } else {
+        } else if constexpr (N > FUSED_N) {
             k_fwd_gather_pts<N, W><<<dim3((npts + GPB - 1) / GPB, cnt), GPB * ZC, 0, s>>>(fg, stride, ln, h->rec, npts);
             PT_LAUNCHED("k_fwd_gather_pts");
         }
@@ -1351,12 +1356,14 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
     if (rc == PT_OK && cudaMemset(h->tma_err, 0, sizeof(int)) == cudaSuccess)
         h->tma_ok = encode_grid_maps(h);   // gather 2 is offered only if every map encodes
     // default variant: two pipelines of two chunks per launch, TMA-staged tiles
-    // (up to 64 wide the gather and the lines in one launch).
-    // Against four pipelines of one (us): 32 wide, 9 slices 25 and 42; 64^3 55
-    // and 123; 128 x 84 slices 140 and 144; 128^3 231 and 215; 256^3 1437 and
-    // 1443.  One pipeline of four is slower from 64^3 up (60, 148, 237, 1598)
+    // (or the gather and the lines in one launch, see FUSED_N).
+    // Against four pipelines of one (us): 64 wide, 64 slices, 96 angles 50 and 57;
+    // 128 x 84 slices, 128 angles 123 and 124; 128^3, 128 angles 171 and 172, 192
+    // angles 202 to 214 and 205; 256^3, 384 angles 1359 and 1355.  One pipeline of
+    // four is slower from 64 slices up (55, 144, 205, 230, 1497)
     h->streams = 2;
-    h->gather = N <= FUSED_N ? 0 : h->tma_ok ? 2 : 1;
+    const size_t inflight = ntheta * std::min<size_t>((nz + ZC - 1) / ZC, RSETS);
+    h->gather = N <= FUSED_N && inflight <= FUSED_BLOCKS ? 0 : h->tma_ok ? 2 : 1;
     if (rc == PT_OK && cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess) rc = PT_ERR_CUDA;
     for (int k = 0; k < RSETS - 1 && rc == PT_OK; ++k)
         if (cudaStreamCreateWithFlags(&h->side[k], cudaStreamNonBlocking) != cudaSuccess ||
