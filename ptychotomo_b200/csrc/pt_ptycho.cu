@@ -1070,7 +1070,6 @@ __global__ void __launch_bounds__(512, 1)
     float2 *tab = ex + 128 * 128;
     const int part = blockIdx.x, parts = gridDim.x, th0 = PROBE ? 0 : angles[blockIdx.y];
     float2 *slab = PROBE ? dst + (size_t)part * P * P : dst + ((size_t)th0 * parts + part) * nz * n;
-    for (int e = threadIdx.x; e < (PROBE ? P * P : nz * n); e += 512) slab[e] = czero();
     const int grp = threadIdx.x >> 7, q0 = threadIdx.x >> 7 << 5 | (threadIdx.x & 31), rt0 = (threadIdx.x >> 5) & 3;
     const int off0 = FULL ? 0 : (128 - P) / 2;
     constexpr bool TAB = !SUB && !PROBE;
