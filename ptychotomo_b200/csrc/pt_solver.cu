@@ -416,25 +416,29 @@ __global__ void __launch_bounds__(256) k_cmul(float2 *out, const float2 *a, cons
     };
     auto at = [](const float2 *p, size_t i) { return reinterpret_cast<const Pack *>(p)[i]; };
     const size_t stride = (size_t)gridDim.x * blockDim.x, np = n / V;
+    auto load = [&](size_t i, Pack &x, Pack &y, Pack &z) {
+        x = at(a, i);
+        y = at(b, i);
+        if (MODE == 1) z = at(c, i);
+    };
+    auto store = [&](size_t i, const Pack &x, const Pack &y, const Pack &z) {
+        Pack r;
+#pragma unroll
+        for (int k = 0; k < V; ++k) r.v[k] = product(x.v[k], y.v[k], MODE == 1 ? z.v[k] : czero());
+        reinterpret_cast<Pack *>(out)[i] = r;
+    };
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (; i < np; i += U * stride) {
+    for (; i + (U - 1) * stride < np; i += U * stride) {
         Pack x[U], y[U], z[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const size_t e = i + u * stride;
-            if (e >= np) break;
-            x[u] = at(a, e);
-            y[u] = at(b, e);
-            if (MODE == 1) z[u] = at(c, e);
-        }
+        for (int u = 0; u < U; ++u) load(i + u * stride, x[u], y[u], z[u]);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (i + u * stride >= np) break;
-            Pack r;
-#pragma unroll
-            for (int k = 0; k < V; ++k) r.v[k] = product(x[u].v[k], y[u].v[k], MODE == 1 ? z[u].v[k] : czero());
-            reinterpret_cast<Pack *>(out)[i + u * stride] = r;
-        }
+        for (int u = 0; u < U; ++u) store(i + u * stride, x[u], y[u], z[u]);
+    }
+    for (; i < np; i += stride) {
+        Pack x, y, z;
+        load(i, x, y, z);
+        store(i, x, y, z);
     }
     if (V > 1 && blockIdx.x == 0 && threadIdx.x < n % V) {   // the elements past the last whole access
         const size_t e = np * V + threadIdx.x;
@@ -742,7 +746,10 @@ extern "C" int pt_cmul_c64(void *out, const void *a, const void *b, const void *
 {
     pt::clear_error();
     PT_CHECK_ARG(out && a && b && (mode != 1 || c) && mode >= 0 && mode <= 2, "cmul: bad arguments");
-    const bool wide = (((uintptr_t)out | (uintptr_t)a | (uintptr_t)b | (mode == 1 ? (uintptr_t)c : 0)) & 15) == 0;
+    // 16-byte accesses from 2^22 elements: a product of 1000, 1 M, 4 M and 16 M
+    // takes 2.9, 6.2, 14.5 and 63.4 us with them and 2.1, 4.2, 14.4 and 66.5 without
+    const bool aligned = (((uintptr_t)out | (uintptr_t)a | (uintptr_t)b | (mode == 1 ? (uintptr_t)c : 0)) & 15) == 0;
+    const bool wide = aligned && n >= ((size_t)1 << 22);
     const unsigned blocks = ew_blocks(wide ? (n + 1) / 2 : n);
     cudaStream_t st = (cudaStream_t)stream;
     float2 *o = (float2 *)out;

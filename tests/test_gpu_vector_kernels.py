@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 U = 2.0 ** -24
 TRIP = 148 * 16 * 256                      # threads of the elementwise grid
-SIZES = [1, 2, 3, 255, 513, TRIP * 2 - 1, TRIP * 4 + 2, TRIP * 4 + 3]
+SIZES = [1, 2, 3, 255, 513, TRIP * 2 - 1, TRIP * 4 + 2, TRIP * 4 + 3, (1 << 22) - 1, (1 << 22) + 1, (1 << 22) + TRIP * 4 + 2]
 
 
 def crand(n, seed, shift=0):
