@@ -1457,7 +1457,7 @@ int ptycho_run(pt_ptycho *h, bool adj, float2 *out, const float2 *in, float scal
         auto go = [&](auto full, auto sub) {
             constexpr bool FU = decltype(full)::value, S = decltype(sub)::value;
             if constexpr (DET == 128) {
-                k_ptycho_fwd128<FU, S><<<std::min(nframes, h->nsm), 512, P128_FSMEM, st>>>(
+                k_ptycho_fwd128<FU, S><<<std::min(nframes, h->nsm), 512, S ? P128_EX : P128_FSMEM, st>>>(
                     in, out, h->corner, h->phase_tab(), h->probe_tab(), h->nz, h->n, h->nscan, nframes, h->P, scale,
                     h->tw128, h->tw, h->shift_ids());
             } else {
