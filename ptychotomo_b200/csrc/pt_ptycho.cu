@@ -93,13 +93,14 @@ __device__ __forceinline__ void resid_line(float2 (&v)[M], float (&d)[M], float 
     if constexpr (RESID != 0) {
         unsigned rare = 0;
 #pragma unroll
+        float top = 0.f;   // Poisson: one maximum per value, and one test per line
         for (int m = 0; m < M; ++m) {
             const float D = d[m] * dscale;
             const float a2 = v[m].x * v[m].x + v[m].y * v[m].y;
             if constexpr (RESID == 1) {
                 const float b = a2 + 1e-32f, y = rcp_normal(b);
                 d[m] = D * fmaf(fmaf(-b, y, 1.f), y, y);
-                if (!(b <= 1e37f && fabsf(d[m]) <= 1e38f)) rare |= 1u << m;
+                top = fmaxf(top, fmaxf(b, fabsf(d[m])));   // a NaN makes its value NaN without further care
                 continue;
             }
             const float z = rsqrt_normal(D), s0 = D * z;
@@ -109,6 +110,11 @@ __device__ __forceinline__ void resid_line(float2 (&v)[M], float (&d)[M], float 
             d[m] = s * rsqrt_normal(a2);
         }
         if (rare) {
+        if (RESID == 1 && top > 1e37f) {
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+                if (fmaxf(v[m].x * v[m].x + v[m].y * v[m].y, fabsf(d[m])) > 1e37f) rare |= 1u << m;
+        }
 #pragma unroll
             for (int m = 0; m < M; ++m)
                 if (rare >> m & 1) {
