@@ -1196,20 +1196,20 @@ __global__ void k_probe_t(const float2 *__restrict__ prb, float2 *__restrict__ p
 // fixed order.  The kernels are the object adjoints in their PROBE mode.
 
 // gprb[px P + py] = c sum_b part[b][py P + px].  A block takes 32 elements; its
-// eight warps sum the partials b = warp, warp + 8, ..., then the eight sums are
-// added in warp order, in FP64: the order then shows in the last bit at most.
+// warps sum the partials b = warp, warp + warps, ..., then their sums are added
+// in warp order, in FP64: the order then shows in the last bit at most.
 // T double2: the sum as it is, for a caller that adds several.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
     k_probe_reduce(const float2 *__restrict__ part, T *__restrict__ gprb, int nblk, int P, float c)
 {
-    __shared__ double2 sums[8][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ double2 sums[32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     double2 s = make_double2(0.0, 0.0);
     if (i < P * P)
 #pragma unroll 4
-        for (int b = warp; b < nblk; b += 8) {
+        for (int b = warp; b < nblk; b += warps) {
             const float2 v = part[(size_t)b * P * P + i];
             s.x += v.x;
             s.y += v.y;
@@ -1217,7 +1217,7 @@ __global__ void __launch_bounds__(256)
     sums[warp][lane] = s;
     __syncthreads();
     if (warp || i >= P * P) return;
-    for (int k = 1; k < 8; ++k) {
+    for (int k = 1; k < warps; ++k) {
         s.x += sums[k][lane].x;
         s.y += sums[k][lane].y;
     }
@@ -1552,11 +1552,14 @@ int probe_adj_launch(pt_ptycho *h, void *gprb, bool fp64, const float2 *in, cons
         else
             go(std::false_type{});
         PT_LAUNCHED("k_ptycho_adj_probe");
-        const unsigned blocks = (unsigned)((h->P * h->P + 31) / 32);
+        // many partials: 32 warps (with eight, the few blocks of a small probe waited on
+        // 4736 / 8 partials a warp: 16 x 16 frames of 100 x 150 scans 156 us, now 35; 64 x
+        // 64 frames of 40 x 60, 296 partials, 45 and 39); det 128 has at most 148
+        const unsigned blocks = (unsigned)((h->P * h->P + 31) / 32), threads = h->prb_blocks > 256 ? 1024 : 256;
         if (fp64)
-            k_probe_reduce<<<blocks, 256, 0, st>>>(h->prb_part, (double2 *)gprb, h->prb_blocks, h->P, h->c);
+            k_probe_reduce<<<blocks, threads, 0, st>>>(h->prb_part, (double2 *)gprb, h->prb_blocks, h->P, h->c);
         else
-            k_probe_reduce<<<blocks, 256, 0, st>>>(h->prb_part, (float2 *)gprb, h->prb_blocks, h->P, h->c);
+            k_probe_reduce<<<blocks, threads, 0, st>>>(h->prb_part, (float2 *)gprb, h->prb_blocks, h->P, h->c);
         PT_LAUNCHED("k_probe_reduce");
         return PT_OK;
     }
