@@ -540,13 +540,15 @@ __global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
 // and rounds as k_fwd_gather_pts and k_fwd_lines).  rec is in point order.
 // One launch and one pass over the lines buffer less, but the grid is read
 // through L1.  32 wide, against the tiles in shared memory (us): 8 slices, 96
-// angles 16.4 and 18.4; 256 slices, 96 angles 151 and 164; where all the blocks
-// of the pipelines are more than FUSED_BLOCKS the tiles win: 32 slices, 192
-// angles 27.9 and 23.6; 16 slices, 384 angles 26.7 and 22.6 (8 slices, 384
-// angles: 18.5 and 20.5).  64 wide the tiles win at every size (8 slices, 24
-// angles 21.3 and 18.5; 64 slices, 96 angles 59 and 50).
+// angles 16.4 and 18.4; 256 slices, 96 angles 151 and 164.  With more than
+// FUSED_POINTS polar points in the chunks that the pipelines work on at once
+// (angles x N x chunks) the tiles win.  32 wide: 384 angles, 8 slices (18432
+// points) 18.5 and 20.5, 16 slices 26.7 and 22.6; 16 wide: 192 angles, 32 slices
+// (18432) 20.5 and 20.6, 288 angles 22.4 and 20.6; 8 wide: 288 angles, 32 slices
+// (13824) 18.4 and 19.6, 768 angles 26.7 and 22.6.  64 wide the tiles win at every
+// size (8 slices, 24 angles 21.3 and 18.5; 64 slices, 96 angles 59 and 50).
 constexpr int FUSED_N = 48;   // longest line (32 wide)
-constexpr int FUSED_BLOCKS = 384;
+constexpr int FUSED_POINTS = 18432;
 template <int N, int W>
 __global__ void __launch_bounds__(GPB *ZC, 4)
     k_fwd_gather_lines(const float2 *__restrict__ fg, size_t set, const float4 *__restrict__ rec,
@@ -1362,8 +1364,8 @@ extern "C" int pt_radon_create_ex(size_t ntheta, size_t nz, size_t n, int m_over
     // angles 202 to 214 and 205; 256^3, 384 angles 1359 and 1355.  One pipeline of
     // four is slower from 64 slices up (55, 144, 205, 230, 1497)
     h->streams = 2;
-    const size_t inflight = ntheta * std::min<size_t>((nz + ZC - 1) / ZC, RSETS);
-    h->gather = N <= FUSED_N && inflight <= FUSED_BLOCKS ? 0 : h->tma_ok ? 2 : 1;
+    const size_t inflight = npts * std::min<size_t>((nz + ZC - 1) / ZC, RSETS);
+    h->gather = N <= FUSED_N && inflight <= FUSED_POINTS ? 0 : h->tma_ok ? 2 : 1;
     if (rc == PT_OK && cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess) rc = PT_ERR_CUDA;
     for (int k = 0; k < RSETS - 1 && rc == PT_OK; ++k)
         if (cudaStreamCreateWithFlags(&h->side[k], cudaStreamNonBlocking) != cudaSuccess ||

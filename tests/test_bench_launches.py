@@ -13,6 +13,7 @@ import bench
     (64, 40, 96, {"radon_fwd_streams": 2, "radon_gather": "L1"}, 1, 4 * 3 + 5),
     (32, 32, 96, None, 1, 3 * 2 + 5),                                                   # gather and lines in one launch
     (32, 32, 97, None, 1, 4 * 2 + 5),
+    (16, 32, 192, None, 1, 3 * 2 + 5), (16, 32, 193, None, 1, 4 * 2 + 5), (8, 8, 1536, None, 1, 3 * 1 + 5),
     (32, 32, 97, {"radon_fwd_streams": 1, "radon_gather": "L1"}, 1, 3 * 1 + 5)])
 def test_launches_per_step(n, nz, ntheta, tuned, parts, launches):
     ops = SimpleNamespace(c=dict(n=n, nz=nz, ntheta=ntheta), tuned=tuned, ptycho=SimpleNamespace(parts=parts))

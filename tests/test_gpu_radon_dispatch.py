@@ -8,7 +8,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,nz,nt", [(8, 3, 5), (16, 33, 96), (32, 32, 96), (32, 32, 97), (32, 8, 384), (32, 9, 193),
+@pytest.mark.parametrize("n,nz,nt", [(8, 3, 5), (8, 32, 384), (8, 32, 385), (16, 33, 96), (16, 25, 192), (16, 25, 193), (32, 32, 96), (32, 32, 97), (32, 8, 384), (32, 9, 193),
                                      (64, 3, 12), (64, 40, 97)])
 def test_default_forward_has_the_bits_of_every_variant(n, nz, nt):
     from ptychotomo_b200 import radonusfft
