@@ -1080,9 +1080,9 @@ __global__ void __launch_bounds__(512, 1)
     const int off0 = FULL ? 0 : (128 - P) / 2;
     constexpr bool TAB = !SUB && !PROBE;
     const int rows = !TAB ? 0 : FULL ? P128_ATAB / 1024 : min(P, P128_ATAB / (P * (int)sizeof(float2)));
-    f128_probe_rows(tab, prbT, rows, P);
+    if constexpr (TAB) f128_probe_rows(tab, prbT, rows, P);
     for (int e = threadIdx.x; e < (PROBE ? P * P : nz * n); e += 512) slab[e] = czero();
-    f128_probe_wait();
+    if constexpr (TAB) f128_probe_wait();
     __syncthreads();
     const int count = PROBE ? nframes : nscan;
     for (int s = part; s < count; s += parts) {
