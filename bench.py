@@ -281,7 +281,7 @@ class Ops:
 
     def launches_per_step(self):
         """Kernel launches of one step: radon fwd 4 per 4 / streams chunks of 8
-        slices (2 streams by default; up to 32 wide the gather through L1, the
+        slices (2 streams by default; up to 64 wide the gather through L1, the
         default while at most 18432 polar points are in flight, includes the
         line transforms: 3), radon adj 3, ptycho
         fwd 1, ptycho adj 1 plus the slab reduction when the angles are split
@@ -290,8 +290,8 @@ class Ops:
         batch = 4 // tuned.get("radon_fwd_streams", 2)
         zc = -(-self.c["nz"] // (8 * batch))
         inflight = self.c["ntheta"] * self.c["n"] * 3 // 2 * min(-(-self.c["nz"] // 8), 4)
-        gather = tuned.get("radon_gather", GATHER_NAMES[0 if self.c["n"] <= 32 and inflight <= 18432 else 2])
-        fused = self.c["n"] <= 32 and gather == GATHER_NAMES[0]
+        gather = tuned.get("radon_gather", GATHER_NAMES[0 if self.c["n"] <= 64 and inflight <= 18432 else 2])
+        fused = self.c["n"] <= 64 and gather == GATHER_NAMES[0]
         return (3 if fused else 4) * zc + 3 + 1 + 1 + (self.ptycho.parts > 1)
 
 

@@ -545,9 +545,11 @@ __global__ void __launch_bounds__(ptfft::Exchange<N, ZC>::NT, N > 384 ? 2 : 4)
 // (angles x N x chunks) the tiles win.  32 wide: 384 angles, 8 slices (18432
 // points) 18.5 and 20.5, 16 slices 26.7 and 22.6; 16 wide: 192 angles, 32 slices
 // (18432) 20.5 and 20.6, 288 angles 22.4 and 20.6; 8 wide: 288 angles, 32 slices
-// (13824) 18.4 and 19.6, 768 angles 26.7 and 22.6.  64 wide the tiles win at every
-// size (8 slices, 24 angles 21.3 and 18.5; 64 slices, 96 angles 59 and 50).
-constexpr int FUSED_N = 48;   // longest line (32 wide)
+// (13824) 18.4 and 19.6, 768 angles 26.7 and 22.6.  64 wide the tiles take less
+// time on the device at every size (25 slices, 28 angles 22 against 25 us; 64
+// slices, 96 angles 50 and 59), but with few angles a caller who launches each
+// call waits for their fourth launch (25 slices, 28 angles 27.5 against 25.4).
+constexpr int FUSED_N = 96;   // longest line (64 wide)
 constexpr int FUSED_POINTS = 18432;
 template <int N, int W>
 __global__ void __launch_bounds__(GPB *ZC, 4)
