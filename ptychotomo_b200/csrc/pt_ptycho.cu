@@ -1308,8 +1308,9 @@ struct pt_ptycho {
     int *angles = nullptr;
     std::vector<int> order;
     bool ordered = false;       // that order is not 0, 1, 2, ...
-    std::vector<int> counts;    // the scans of each angle that are not skipped, most first
-    double scans_all = 0;       // their sum
+    // the scans of each angle that are not skipped, most first (none before setobj: as if all), and their sum
+    std::vector<int> counts;
+    double scans_all = 0;
     int parts_set = 0;          // the parts that the caller or the environment set; 0: chosen, -1: autotuned
     int few_set = -1;           // k_ptycho_adj_few: 1 always, 0 never, -1 chosen
     // slabs per angle that `partial` holds, and whether a launch has used them:
@@ -1652,7 +1653,8 @@ Split choose_split(const pt_ptycho &h, int resid, size_t most, int only = 0)
 {
     const double cells = (double)h.nz * h.n;
     const bool full = h.P == h.det;
-    const int most_scans = h.counts.front(), least = h.counts.back(), scans = std::max(most_scans, 1);
+    const int most_scans = h.counts.empty() ? h.nscan : h.counts.front(), least = h.counts.empty() ? h.nscan : h.counts.back();
+    const int scans = std::max(most_scans, 1);
     const bool few_can = h.det >= 16 && h.det <= 64;
     Split best_split;
     double best = 1e300;
@@ -1921,7 +1923,6 @@ extern "C" int pt_ptycho_create(size_t ntheta, size_t nz, size_t n, size_t nthet
     h->det = (int)detx;
     h->P = (int)nprb;
     h->c = 1 / sqrtf(detx * dety);  // kernels.cuh:260
-    h->counts.assign(h->ntheta, h->nscan);
     h->scans_all = (double)h->ntheta * h->nscan;
     if (cudaGetDevice(&h->device) != cudaSuccess) {
         delete h;
