@@ -135,7 +135,9 @@ int pt_ptycho_destroy(pt_ptycho *h);
 int pt_ptycho_setobj(pt_ptycho *h, const float *scan, const void *prb, void *stream);
 /* ptychofft::fwd(g, f) — src/cuda/ptychofft.cu:58-76.  g = F Q f. */
 int pt_ptycho_fwd(pt_ptycho *h, void *g, const void *f, void *stream);
-/* ptychofft::adj(f, g) — src/cuda/ptychofft.cu:78-93.  f = Q* F* g. */
+/* ptychofft::adj(f, g) — src/cuda/ptychofft.cu:78-93.  f = Q* F* g.
+ * Deterministic.  For detectors of 16 to 128 what is below 2^-126 may be taken
+ * as zero in the sums over the scans (here and in the gradients below). */
 int pt_ptycho_adj(pt_ptycho *h, void *f, const void *g, void *stream);
 /* fwd/adj with the output multiplied by `scale` (Solver.fwd_ptycho /
  * adj_ptycho apply coefptycho this way, solver.py:100-125). */

@@ -79,8 +79,9 @@ __device__ __forceinline__ float rcp_normal(float x)
 // x - D x / b, b = |x|^2 + 1e-32: 1 / b is one Newton step from the hardware's
 // approximation; Gaussian x (1 - sqrt(D) / |x|): sqrt(D) is one Heron step from
 // D / sqrt(D), and 1 / |x| the approximation that pt_residual_gaussian takes.
-// Either step leaves the correctly rounded value but for rare last bits.  A
-// value out of range (|x|^2 above 1e37; Poisson also D / b above 1e38; Gaussian
+// Either step gives the correctly rounded value: no difference from __frcp_rn
+// for any b in [1e-32, 1e37] nor from __fsqrt_rn for any D in [1e-30, 1e37].  A
+// value out of range (|x|^2 above 1e37; Poisson also D / b above 1e37; Gaussian
 // also |x|^2 below 1e-30, or D not zero and outside these bounds, negative or
 // not finite) makes the thread take pt_residual_* for it afterwards.  With a test and a call site per value
 // and the rounded reciprocal or square root of the library, the det-128
@@ -92,8 +93,8 @@ __device__ __forceinline__ void resid_line(float2 (&v)[M], float (&d)[M], float 
 {
     if constexpr (RESID != 0) {
         unsigned rare = 0;
-#pragma unroll
         float top = 0.f;   // Poisson: one maximum per value, and one test per line
+#pragma unroll
         for (int m = 0; m < M; ++m) {
             const float D = d[m] * dscale;
             const float a2 = v[m].x * v[m].x + v[m].y * v[m].y;
@@ -109,12 +110,12 @@ __device__ __forceinline__ void resid_line(float2 (&v)[M], float (&d)[M], float 
             if (!(a2 >= 1e-30f && a2 <= 1e37f && (D == 0.f || (D >= 1e-30f && D <= 1e37f)))) rare |= 1u << m;
             d[m] = s * rsqrt_normal(a2);
         }
-        if (rare) {
         if (RESID == 1 && top > 1e37f) {
 #pragma unroll
             for (int m = 0; m < M; ++m)
                 if (fmaxf(v[m].x * v[m].x + v[m].y * v[m].y, fabsf(d[m])) > 1e37f) rare |= 1u << m;
         }
+        if (rare) {
 #pragma unroll
             for (int m = 0; m < M; ++m)
                 if (rare >> m & 1) {
@@ -256,8 +257,8 @@ __global__ void __launch_bounds__(ptycho_block<DET>(), 1)
 // on the probe's columns only, packed onto the first threads, and R2 skips
 // the slots outside it.
 // 192 angles x 225 scans, 64 x 64 detector, 16-pixel probe, forward: 1.04 ->
-// 0.38 ms; Poisson gradient of 128 x 49 scans of a 64-pixel probe: 0.31 ->
-// 0.13 ms.
+// 0.41 ms; Poisson gradient of 128 x 49 scans of a 64-pixel probe: 0.31 ->
+// 0.14 ms.
 template <int DET>
 struct FR {
     static constexpr int QA = DET / 16, RT = DET / 16, J = QA * RT;
@@ -371,10 +372,11 @@ __device__ __forceinline__ int fresh(int t)
     return t;
 }
 
-// *p += v in L2, without waiting for the sum (one FP32 addition per component,
-// as a load, an add and a store round it).  Each frame adds to a pixel at most
-// once and the frames of a block are separated by its barriers, so the order of
-// the sums, and the result, is that of the frames.
+// *p += v in L2, without waiting for the sum: one FP32 addition per component,
+// rounded as an add rounds it, but for subnormal inputs and results, which red
+// flushes to zero on global memory (k_ptycho_adj_few keeps them).  Each frame
+// adds to a pixel at most once and the frames of a block are separated by its
+// barriers, so the order of the sums, and the result, is that of the frames.
 __device__ __forceinline__ void add_l2(float2 *p, float2 v)
 {
     asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(v.x), "f"(v.y) : "memory");
@@ -827,11 +829,12 @@ __global__ void __launch_bounds__(PF<DET>::NT, 1)
 // The probe table (128 KB) does not stay in the 100 KB of L1 that the exchange
 // buffer leaves: rereading it cyclically hit 10 % (forward).  Its first 96 KB
 // sit in shared memory instead, the rest is read through L2.
-// 256^3, 384 angles x 169 scans: forward 3.75 -> 3.34 ms (a table of 64 KB
-// costs 0.05, later patch loads 0.17 more), adjoint 4.26 -> 3.70 ms.  The
-// adjoint keeps 32 KB only: with 96 KB in the table the L1 left for loads in
-// flight is too small (4.00 ms; 16 KB 3.83, 48 KB 3.75).  The arithmetic and
-// the exchange alone take 2.1 ms of the forward, the exchange 1.1 ms.
+// 256^3, 384 angles x 169 scans on one raster: forward 3.75 -> 3.34 ms (a table
+// of 64 KB costs 0.05, later patch loads 0.17 more), adjoint 4.26 -> 3.70 ms
+// (jittered scans 4.4 -> 3.75 to 3.95).  The adjoint keeps 32 KB only: with 96
+// KB in the table the L1 left for loads in flight is too small (4.00 ms; 16 KB
+// 3.83, 48 KB 3.75).  The arithmetic and the exchange alone take 2.1 ms of the
+// forward, the exchange 1.1 ms.
 constexpr int P128_EX = 128 * 128 * 8;          // exchange buffer
 constexpr int P128_FTAB = 96 * 1024, P128_ATAB = 32 * 1024;   // probe rows kept in shared memory: forward, adjoint
 constexpr int P128_FSMEM = P128_EX + P128_FTAB, P128_ASMEM = P128_EX + P128_ATAB;
