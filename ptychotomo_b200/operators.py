@@ -145,6 +145,8 @@ class ptychofft:  # noqa: N801 - reference class name
 
     @property
     def parts(self):
+        """The adjoint's split: blocks (and slabs) per angle.  Setting it sets
+        the residual adjoints' too, each in the kernel that suits it."""
         out = ctypes.c_int()
         check(lib().pt_ptycho_get_parts(self._h, ctypes.byref(out)), "ptychofft.parts")
         return out.value
